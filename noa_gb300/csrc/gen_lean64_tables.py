@@ -17,6 +17,7 @@ LOG_BITS = 8        # 256 bins over the top 8 mantissa bits
 LOG_SPLIT = 106     # bins t >= 106 (m >= 1 + 106/256 > sqrt 2) are halved: m in [0.707, 1)
 C_BITS = 10         # c_t = C_t / 2^10: m * c_t is exact in 64-bit integers
 EXP_N = 128         # 2^(j/128)
+MAGIC = 0x4B400000  # bits of 1.5 2^23: a float there carries a 22-bit signed integer in its low bits
 
 
 def f32(x):
@@ -30,16 +31,13 @@ def ff(x):
 
 
 def log_tables():
-    """Per bin t: (C_t, F_t, L_t).
+    """Per bin t: (c_t 2^11 / 2^h, L_t).
 
-    c_t = C_t / 2^10 is 1 / (bin centre) rounded to 10 fractional bits, so
-    that r = m c_t - 1 is an exact 64-bit integer multiple of 2^-(62+h);
-    |r| < 2^-8.7.  F_t is the number of fractional bits of the bin's
-    fixed-point sum L_t + r + d = log m: the largest |log m| of the bin times
-    2^F_t is at most 2^62.  L_t = -log(c_t) in units of 2^-F_t, rounded.
-    The two bins that touch 1 use c_t = 1, L_t = 0 and F_t = 0 (a marker:
-    their scale follows the size of r, so that log m = r + d keeps full
-    relative accuracy down to m = 1 +- 2^-53).
+    c_t = C_t / 2^10 is 1 / (bin centre) rounded to 10 fractional bits and
+    m = M 2^-(52+h), so that r = m c_t - 1 is an exact 64-bit integer multiple
+    of 2^-63; |r| < 2^-8.7.  L_t is -log(c_t) in units of 2^-63, less the
+    offsets MAGIC 2^23 + MAGIC 2 that the two integer parts of the sum carry,
+    modulo 2^64.
     """
     rows = []
     one = 1 << C_BITS
@@ -47,31 +45,33 @@ def log_tables():
         h = 1 if t >= LOG_SPLIT else 0
         lo = (1 + mpmath.mpf(t) / (1 << LOG_BITS)) / 2 ** h
         hi = (1 + mpmath.mpf(t + 1) / (1 << LOG_BITS)) / 2 ** h
-        if t in (0, (1 << LOG_BITS) - 1):
-            rows.append((one, 0, 0))
-            continue
         C = int(mpmath.nint(one / ((lo + hi) / 2)))
-        big = max(abs(mpmath.log(lo)), abs(mpmath.log(hi)))
-        F = 62 - int(mpmath.ceil(mpmath.log(big, 2)))
-        assert big * mpmath.mpf(2) ** F <= mpmath.mpf(2) ** 62
-        assert F >= 62 + h  # the shift of r into the sum is never negative
         for m in (lo, hi):  # |r| stays below 2^-8.7 over the bin
             assert abs(m * C / one - 1) < mpmath.mpf(2) ** -8.7
-        L = int(mpmath.nint(-mpmath.log(mpmath.mpf(C) / one) * mpmath.mpf(2) ** F))
-        rows.append((C, F, L))
+        L = int(mpmath.nint(-mpmath.log(mpmath.mpf(C) / one) * mpmath.mpf(2) ** 63))
+        L = (L - (MAGIC << 23) - (MAGIC << 1)) % (1 << 64)
+        rows.append((C << (1 - h), L - (1 << 64) if L >> 63 else L))
     return rows
+
+
+def signed_words(v, n):
+    """v (an integer) as n words of 32 bits, each in [-2^31, 2^31), lowest first."""
+    w = []
+    for _ in range(n):
+        d = v & 0xFFFFFFFF
+        d -= (1 << 32) if d >> 31 else 0
+        w.append(d)
+        v = (v - d) >> 32
+    assert v == 0
+    return w
 
 
 def main():
     rows = log_tables()
-    T = [float(mpmath.power(2, mpmath.mpf(j) / EXP_N)) for j in range(EXP_N)]
     ln2 = mpmath.log(2)
-    ln2n = ln2 / EXP_N
-    # hi part with 32 significant bits: k * hi is exact for |k| < 2^21
-    e = int(mpmath.floor(mpmath.log(ln2n, 2)))
-    hi = mpmath.floor(ln2n / mpmath.power(2, e - 31)) * mpmath.power(2, e - 31)
-    lo = ln2n - hi
-    lo_h, lo_l = ff(lo)
+    ln2_l, ln2_h = signed_words(int(mpmath.nint(ln2 * mpmath.mpf(2) ** 63)), 2)
+    k_l, k_m, k_h = signed_words(int(mpmath.nint(ln2 / EXP_N * mpmath.mpf(2) ** 95)), 3)
+    T = [int(mpmath.nint(mpmath.power(2, mpmath.mpf(j) / EXP_N) * mpmath.mpf(2) ** 61)) for j in range(EXP_N)]
     third_h, third_l = ff(mpmath.mpf(1) / 3)
     sixth_h, sixth_l = ff(mpmath.mpf(1) / 6)
     out = []
@@ -80,27 +80,29 @@ def main():
     out.append(f"#define LEAN64_LOG_BITS {LOG_BITS}")
     out.append(f"#define LEAN64_LOG_SPLIT {LOG_SPLIT}")
     out.append(f"#define LEAN64_EXP_N {EXP_N}")
-    out.append(f"#define LEAN64_LN2 {float(ln2)!r}")
     out.append(f"#define LEAN64_INV_LN2N {float(EXP_N / ln2)!r}")
-    out.append(f"#define LEAN64_LN2N_HI {float(hi)!r}")
-    out.append(f"#define LEAN64_LN2N_LO {float(lo)!r}")
-    out.append(f"#define LEAN64_LN2N_LO_H {lo_h!r}f")
-    out.append(f"#define LEAN64_LN2N_LO_L {lo_l!r}f")
+    out.append("/* ln 2 = LN2_H 2^-31 + LN2_L 2^-63 */")
+    out.append(f"#define LEAN64_LN2_H {ln2_h}")
+    out.append(f"#define LEAN64_LN2_L {ln2_l}")
+    out.append("/* ln 2 / 128 = K_H 2^-31 + K_M 2^-63 + K_L 2^-95 */")
+    out.append(f"#define LEAN64_K_H {k_h}")
+    out.append(f"#define LEAN64_K_M {k_m}")
+    out.append(f"#define LEAN64_K_L {k_l}")
     out.append(f"#define LEAN64_THIRD_H {third_h!r}f")
     out.append(f"#define LEAN64_THIRD_L {third_l!r}f")
     out.append(f"#define LEAN64_SIXTH_H {sixth_h!r}f")
     out.append(f"#define LEAN64_SIXTH_L {sixth_l!r}f")
-    out.append("/* Per bin t, one 16-byte entry {C_t | F_t << 32, L_t}: the 10-bit")
-    out.append("   reciprocal C_t / 2^10 of the bin centre, the number F_t of fractional")
-    out.append("   bits of the bin's fixed-point sum (0: the two bins at 1, scaled by")
-    out.append("   the size of r) and -log(C_t / 2^10) in units of 2^-F_t. */")
+    out.append("/* Per bin t, one 16-byte entry {c_t, L_t}: the reciprocal c_t of the bin")
+    out.append("   centre in units of 2^-11 (2^-10 for the halved bins t >= LOG_SPLIT; 10")
+    out.append("   fractional bits) and -log(c_t) in units of 2^-63, less the offsets of the")
+    out.append("   two float-carried integers that are added to it (MAGIC 2^23 + MAGIC 2). */")
     out.append("#define LEAN64_LOG_TAB_DATA {\\")
-    out.append(",\\\n".join("    {%dLL, %dLL}" % (C | (F << 32), L) for C, F, L in rows) + "}")
+    out.append(",\\\n".join("    {%dLL, %dLL}" % r for r in rows) + "}")
     out.append("static __device__ const longlong2 lean64_log_tab[%d] = LEAN64_LOG_TAB_DATA;" % len(rows))
-    out.append("/* 2^(j/128) rounded to double. */")
+    out.append("/* 2^(j/128) in units of 2^-61, rounded. */")
     out.append("#define LEAN64_EXP_TAB_DATA {\\")
-    out.append(",\\\n".join("    %s" % repr(v) for v in T) + "}")
-    out.append("static __device__ const double lean64_exp_t[%d] = LEAN64_EXP_TAB_DATA;" % len(T))
+    out.append(",\\\n".join("    %dLL" % v for v in T) + "}")
+    out.append("static __device__ const long long lean64_exp_t[%d] = LEAN64_EXP_TAB_DATA;" % len(T))
     print("\n".join(out))
 
 

@@ -8,26 +8,32 @@
  * FP64 instruction count with issue ~80% idle (ncu: FP64 pipe 86%, issue
  * 12%), and replacing one FP64 instruction by up to ~30 integer or FP32
  * instructions still shortens it.  The functions here keep double accuracy
- * (about 1 ulp; tests compare them with CUDA's functions and numpy) and do
+ * (0.5 - 0.9 ulp; tests compare them with CUDA's functions and numpy) and do
  * their work in exact 64-bit integer arithmetic (range reduction, products
  * with short table constants, fixed-point sums rounded once to double) and
  * in float-float arithmetic (the small correction terms, which need 2^-47
- * relative), leaving FP64 only where a double is the natural operand:
+ * relative).  What they spend is ALU issue (64 lanes: shifts, selects, 64-bit
+ * adds), so values cross between float and integer through the FMA pipe
+ * (integers carried in the low bits of a float, products by powers of two
+ * instead of shifts) or as the two 32-bit words of a fixed-point number,
+ * never by normalising.  Four processes x 3e7 pairs: 42.2 ms with the same
+ * methods at 1 / 2 / 0 FP64 instructions and normalised conversions (about
+ * twice the ALU instructions), 35.3 ms as they are:
  *
- *   lean_log   1 FP64 op.  Tang's table method (P. T. P. Tang, ACM TOMS
- *              16(4), 1990): x = 2^e m, c_t = C_t / 2^10 ~ 1/m from the top
- *              8 mantissa bits; r = m c_t - 1 exact in 64-bit integers;
- *              log x = e ln2 + [-log c_t + r + (log1p(r) - r)], the bracket
- *              a fixed-point sum at the bin's scale, the final e ln2 one
- *              FMA.  The two bins next to 1 use c_t = 1 with a scale that
- *              follows r: full relative accuracy near 1.
- *   lean_exp   2 FP64 ops.  Tang's table method (ACM TOMS 15(2), 1989):
- *              k = round(x 128 / ln2), r = x - k hi (one exact FMA), the
- *              rest of exp(r) - 1 in float-float and a fixed-point sum;
- *              exp x = 2^k' fma(T_j, p, T_j), 2^k' added to the exponent.
- *   lean_rcp   0 FP64 ops.  MUFU seed, exact float-float residual 1 - m y0
- *              on the mantissa split into three floats, y0 (1 + e + e^2)
- *              summed in fixed point and rounded once.
+ *   lean_log   0 FP64 ops.  Tang's table method (P. T. P. Tang, ACM TOMS
+ *              16(4), 1990): x = 2^e m, c_t ~ 1/m with 10 fractional bits from
+ *              the top 8 mantissa bits; r = m c_t - 1 exact in 64-bit integers;
+ *              log x = e ln2 - log c_t + r + (log1p(r) - r), summed in 64-bit
+ *              fixed point at a scale that follows |e| and rounded once.
+ *              Within 2^-8 of 1 c = 1 and the scale follows r: full
+ *              relative accuracy near 1.
+ *   lean_exp   0 FP64 ops.  Tang's table method (ACM TOMS 15(2), 1989): x as a
+ *              64-bit fixed-point number, k = round(x 128 / ln2),
+ *              r = x - k ln2 / 128 modulo 2^64, expm1(r) - r in float-float,
+ *              2^k' T_j (1 + expm1 r) by integer products, rounded once.
+ *   lean_rcp   0 FP64 ops.  MUFU seed y0 as an integer, the exact residual
+ *              1 - m y0 by one 64-bit integer product, y0 (1 + e + e^2) in
+ *              fixed point, rounded once.
  *   lean_div   1 FP64 op: a * lean_rcp(b).
  *   lean_sqrt  6 FP64 ops.  MUFU rsqrt, then two Newton steps on s = x y.
  *
@@ -89,7 +95,7 @@ __device__ __forceinline__ bool bits_ge(double x, double c) {
 
 #if defined(LEAN64_HOST_TABLES) && !defined(__CUDA_ARCH__)
 static const longlong2 lean64_log_tab_host[1 << LEAN64_LOG_BITS] = LEAN64_LOG_TAB_DATA;
-static const double lean64_exp_t_host[LEAN64_EXP_N] = LEAN64_EXP_TAB_DATA;
+static const long long lean64_exp_t_host[LEAN64_EXP_N] = LEAN64_EXP_TAB_DATA;
 #endif
 
 namespace detail {
@@ -102,9 +108,11 @@ __device__ __forceinline__ float u2f(unsigned b) { return __uint_as_float(b); }
 __device__ __forceinline__ int clz64(unsigned long long x) { return __clzll((long long)x); }
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ int f2i_rn(float x) { return __float2int_rn(x); }
+__device__ __forceinline__ int clz32(unsigned x) { return __clz((int)x); }
+__device__ __forceinline__ float i2f(int i) { return __int2float_rn(i); }
+__device__ __forceinline__ unsigned mulhi_s(int a, int b) { return (unsigned)__mulhi(a, b); }
 __device__ __forceinline__ longlong2 log_entry(int t) { return __ldg(&lean64_log_tab[t]); }
-__device__ __forceinline__ double exp_entry(int j) { return __ldg(&lean64_exp_t[j]); }
+__device__ __forceinline__ long long exp_entry(int j) { return __ldg(&lean64_exp_t[j]); }
 #elif defined(LEAN64_HOST_TABLES)
 inline long long d2ll(double x) { long long b; memcpy(&b, &x, 8); return b; }
 inline double ll2d(long long b) { double x; memcpy(&x, &b, 8); return x; }
@@ -113,9 +121,11 @@ inline float u2f(unsigned b) { float x; memcpy(&x, &b, 4); return x; }
 inline int clz64(unsigned long long x) { return __builtin_clzll(x); }
 inline float fadd(float a, float b) { return a + b; }  // host code is built with -ffp-contract=off
 inline float fmul(float a, float b) { return a * b; }
-inline int f2i_rn(float x) { return (int)nearbyintf(x); }
+inline int clz32(unsigned x) { return __builtin_clz(x); }
+inline float i2f(int i) { return (float)i; }
+inline unsigned mulhi_s(int a, int b) { return (unsigned)(((long long)a * b) >> 32); }
 inline longlong2 log_entry(int t) { return lean64_log_tab_host[t]; }
-inline double exp_entry(int j) { return lean64_exp_t_host[j]; }
+inline long long exp_entry(int j) { return lean64_exp_t_host[j]; }
 #endif
 
 // f 2^F as a signed 64-bit integer, truncated toward zero; 0 for zero and
@@ -145,43 +155,58 @@ LEAN64_FN double fix_to_double(long long S, int F) {
     return ll2d((long long)(sign | (((unsigned long long)(1085 - lz - F) << 52) + m)));
 }
 
+// Z 2^-F as a double, rounded half up in the last place, for |Z| >= 2^32: the
+// leading bit is then in the high word (one 32-bit count).
+LEAN64_FN double fix_wide_to_double(long long Z, int F) {
+    const unsigned long long U = Z < 0 ? 0ull - (unsigned long long)Z : (unsigned long long)Z;
+    const int lz = clz32((unsigned)(U >> 32)) - 1;  // the caller keeps |Z| < 2^63
+    const unsigned long long m = ((U << lz) + 0x200ull) >> 10;  // leading bit at 52
+    return ll2d((long long)((((unsigned long long)(1084 - lz - F) << 52) + m) |
+                            ((unsigned long long)Z & 0x8000000000000000ull)));
+}
+
+// The pair dh + dl as an integer in units of 2^-(S + 22), in two parts of 22
+// bits that float adds round: i1 = round(d 2^S), i2 = round((d 2^S - i1) 2^22).
+// Returns their float carriers (bits MAGIC + i; MAGIC = 0x4B400000), whose
+// offsets the caller's constants take off.  Requires |d| 2^S < 2^22.
+LEAN64_FN void fix_parts(float dh, float dl, float scale, unsigned &b1, unsigned &b2) {
+    const float t1 = fmaf(fadd(dh, dl), scale, 12582912.f);
+    const float g = fmaf(dl, scale, fmaf(dh, scale, -fadd(t1, -12582912.f)));
+    b1 = f2u(t1);
+    b2 = f2u(fmaf(g, 4194304.f, 12582912.f));
+}
+
 } // namespace detail
 
-// log x with one FP64 instruction.  x = 2^e m, m in [0.707, 1.414) (bin t of
-// the top 8 mantissa bits, halved above sqrt 2), c = C_t / 2^10 ~ 1/m:
-//   r = m c - 1 = R 2^-(62+h)      exact, one 64-bit integer multiply
-//   d = log1p(r) - r               float-float, ~2^-47 relative
-//   T = -log c + r + d             64-bit fixed point at the bin's scale
-//                                  2^-F_t, rounded once to double
-//   log x = fma(e, ln2, T)         the one FP64 instruction
-// |T| <= 0.347 < ln2 / 2, so the fma never cancels; in the two bins next to
-// 1 the scale follows r (log x = r + d there), so log x keeps full relative
-// accuracy at x = 1 +- 2^-53.
+// log x with no FP64 instruction.  x = 2^e m, m in [0.707, 1.414) (bin t of
+// the top 8 mantissa bits, halved above sqrt 2), c_t ~ 1/m:
+//   r = m c - 1 = R 2^-63          exact, one 64-bit integer multiply
+//   d = log1p(r) - r               float-float, ~2^-47 relative; r enters as
+//                                  rh + rl, the two words of R
+//   log x = e ln2 - log c + r + d  64-bit fixed point: 2^-63 for e = 0, 2^-58
+//                                  for |e| <= 15, 2^-51 beyond (|log x| >= 0.34,
+//                                  0.34 and 10.7: at least 2^-57 relative)
+// rounded once to double.  Within 2^-8 of 1 (e = 0) c = 1 and the scale
+// follows r (log x = r + d), so log x keeps full relative accuracy at
+// x = 1 +- 2^-53.
 LEAN64_FN double lean_log(double x) {
     using namespace detail;
     const long long b = d2ll(x);
+    const unsigned hi = (unsigned)((unsigned long long)b >> 32);
     // positive, normal and finite?
-    if ((unsigned long long)(b - 0x0010000000000000LL) >= 0x7FE0000000000000ULL)
+    if (hi - 0x00100000u >= 0x7FE00000u)
         return log(x);
-    const int hi = (int)(b >> 32);
-    const int t = (hi >> 12) & 0xFF;
-    const int h = t >= LEAN64_LOG_SPLIT ? 1 : 0;
-    const int e = (hi >> 20) - 1023 + h;
-    const unsigned long long M = ((unsigned long long)b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
-    const longlong2 ent = log_entry(t);  // {C_t | F_t << 32, L_t}, one 16-byte load
-    const unsigned long long C = (unsigned long long)ent.x & 0xFFFFull;
-    const int Ft = (int)(ent.x >> 32);
-    const long long R = (long long)(M * C - (1ull << (62 + h)));
-    if (R == 0)  // m = 1: x = 2^e
-        return fpconv::f64i(e) * LEAN64_LN2;
-    const unsigned long long A = R < 0 ? 0ull - (unsigned long long)R : (unsigned long long)R;
-    const int lz = clz64(A);              // 8 <= lz <= 63
-    const unsigned long long N = A << lz;  // |r| = N 2^-(62+h+lz), N in [2^63, 2^64)
-    // r = rh + rl: the top 24 bits of N exactly, then the next 23
-    const unsigned sgn = R < 0 ? 0x80000000u : 0u;
-    const float rh = u2f(sgn | ((unsigned)(128 - h - lz) << 23) | ((unsigned)(N >> 40) & 0x7FFFFFu));
-    const float v = fadd(u2f(0x4B000000u | ((unsigned)(N >> 17) & 0x7FFFFFu)), -8388608.f);  // exact
-    const float rl = fmul(u2f(sgn | ((unsigned)(82 - h - lz) << 23)), v);                   // +- v 2^(-45-h-lz)
+    const int e = (int)(hi + ((256u - LEAN64_LOG_SPLIT) << 12) - 0x3FF00000u) >> 20;  // bins above the split carry
+    const bool near1 = hi - 0x3FEFF000u < 0x2000u;
+    const longlong2 ent = log_entry((hi >> 12) & 0xFFu);  // {c_t, L_t}, one 16-byte load
+    const unsigned C = near1 ? (hi < 0x3FF00000u ? 1024u : 2048u) : (unsigned)ent.x;
+    const unsigned long long M = ((unsigned long long)((hi & 0x000FFFFFu) | 0x00100000u) << 32) | (unsigned)b;
+    const long long R = (long long)(M * C + 0x8000000000000000ull);
+    // r = rh + rl: the high word rounded and the signed low word, renormalised
+    const float rw = fmul(i2f((int)((R + 0x80000000ll) >> 32)), 0x1p-31f);
+    const float rv = fmul(i2f((int)(unsigned)R), 0x1p-63f);
+    const float rh = fadd(rw, rv);
+    const float rl = fadd(rv, -fadd(rh, -rw));
     // d = -r^2/2 + r^3 w,  w = 1/3 - r/4 + r^2 (1/5 - r/6 + r^2/7)
     const float sh = fmul(rh, rh);
     const float sl = fmaf(fmul(2.f, rh), rl, fmaf(rh, rh, -sh));
@@ -198,108 +223,104 @@ LEAN64_FN double lean_log(double x) {
     const float hs = fmul(-0.5f, sh);
     const float dh = fadd(hs, uh);
     const float dl = fadd(fadd(uh, -fadd(dh, -hs)), fmaf(-0.5f, sl, ul));
-    // T = L_t + r + d in units of 2^-F
-    const int F = Ft != 0 ? Ft : 60 + h + lz;
-    const long long Sr = (long long)(A << (F - 62 - h));  // shift 1..7, or lz - 2 at 1
-    const long long S = ent.y + (R < 0 ? -Sr : Sr) + fix_from_float(dh, F) + fix_from_float(dl, F);
-    return fma(fpconv::f64i(e), LEAN64_LN2, fix_to_double(S, F));
+    if (near1) {
+        if (R == 0)
+            return 0.0;
+        const unsigned long long A = R < 0 ? 0ull - (unsigned long long)R : (unsigned long long)R;
+        const int lz = clz64(A);  // |r| < 2^-8: lz >= 8
+        const int F = 61 + lz;
+        const long long Sr = (long long)(A << (lz - 2));
+        return fix_to_double((R < 0 ? -Sr : Sr) + fix_from_float(dh, F) + fix_from_float(dl, F), F);
+    }
+    unsigned b1, b2;
+    fix_parts(dh, dl, 0x1p40f, b1, b2);
+    const long long T = R + (long long)((unsigned long long)ent.y + (unsigned long long)b1 * 0x800000ull +
+                                        (unsigned long long)b2 * 2ull);
+    const int s = e == 0 ? 0 : ((unsigned)(e + 15) <= 30u ? 5 : 12);
+    const long long Q = T + (long long)e * LEAN64_LN2_L;
+    const long long Z = (long long)(int)((unsigned)e << ((32 - s) & 31)) * LEAN64_LN2_H + (Q >> s);
+    return fix_wide_to_double(Z, 63 - s);
 }
 
-// exp x with two FP64 instructions.  k = round(x 128 / ln2), 2^(k/128) =
-// 2^k' T_j:
-//   r = x - k hi                   exact (hi has 32 bits), the first FMA
-//   rt = r - k lo                  float-float (the reduced argument)
-//   d = expm1(rt) - rt             float-float, ~2^-47 relative
-//   p = r + (d - k lo)             64-bit fixed point, 2^-70, rounded once
-//   exp x = 2^k' fma(T_j, p, T_j)  the second FMA; 2^k' on the exponent bits
+// exp x with no FP64 instruction.  k = round(x 128 / ln2) from a float,
+// 2^(k/128) = 2^k' T_j:
+//   r = x - k ln2 / 128            64-bit fixed point, 2^-63, modulo 2^64
+//   d = expm1(r) - r               float-float, ~2^-47 relative
+//   exp x = 2^k' T_j (1 + r + d)   integer products, rounded once
 LEAN64_FN double lean_exp(double x) {
     using namespace detail;
-    if ((d2ll(x) & 0x7FFFFFFFFFFFFFFFLL) >= 0x4085E00000000000LL)  // |x| >= 700, inf, NaN
+    const long long b = d2ll(x);
+    const unsigned hi = (unsigned)((unsigned long long)b >> 32), a = hi & 0x7FFFFFFFu;
+    if (a >= 0x4085E000u)  // |x| >= 700, inf, NaN
         return exp(x);
-    const int k = f2i_rn(fmul(fpconv::f32(x), (float)LEAN64_INV_LN2N));
-    const double r = fma(-fpconv::f64i(k), LEAN64_LN2N_HI, x);
-    const unsigned long long br = (unsigned long long)d2ll(r);
-    const unsigned er = (unsigned)(br >> 52) & 0x7FFu;
-    const unsigned rs = (unsigned)(br >> 32) & 0x80000000u;
-    // r = rh + rl to 2^-47 (the top 24 bits, then 23); zero below 2^-80,
-    // where r only enters linearly
-    const bool big = er >= 943u;
-    const float rh = big ? u2f(rs | ((er - 896u) << 23) | ((unsigned)(br >> 29) & 0x7FFFFFu)) : 0.f;
-    const float rv = fadd(u2f(0x4B000000u | ((unsigned)(br >> 6) & 0x7FFFFFu)), -8388608.f);
-    const float rl = big ? fmul(u2f(rs | ((er - 942u) << 23)), rv) : 0.f;
-    // k lo and rt = r - k lo
-    const float kf = fadd(u2f(0x4B400000u + (unsigned)k), -12582912.f);  // exact, |k| < 2^22
-    const float kh = fmul(kf, LEAN64_LN2N_LO_H);
-    const float kl = fmaf(kf, LEAN64_LN2N_LO_L, fmaf(kf, LEAN64_LN2N_LO_H, -kh));
-    const float th = fadd(rh, -kh);
-    const float tb = fadd(th, -rh);
-    const float te = fadd(fadd(rh, -fadd(th, -tb)), fadd(-kh, -tb));
-    const float tl = fadd(te, fadd(rl, -kl));
-    // d = rt^2 (1/2 + rt w),  w = 1/6 + rt (1/24 + rt (1/120 + rt/720))
-    const float sh = fmul(th, th);
-    const float sl = fmaf(fmul(2.f, th), tl, fmaf(th, th, -sh));
-    const float g = fmul(th, fmaf(th, fmaf(th, 1.f / 720.f, 1.f / 120.f), 1.f / 24.f));
+    // |x| as a float, cut to 24 bits (2^-126 for what is smaller), with x's sign
+    const unsigned am = a > 0x38100000u ? a : 0x38100000u;
+    const float xf = u2f((((am << 3) | ((unsigned)b >> 29)) - (896u << 23)) | (hi & 0x80000000u));
+    const int k = (int)(f2u(fmaf(xf, (float)LEAN64_INV_LN2N, 12582912.f)) - 0x4B400000u);
+    // x in units of 2^-63 modulo 2^64 (the high bits cancel in r; below 2^-11 cut at 2^-63)
+    const unsigned long long M = (((unsigned long long)b) & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
+    const int n = (int)(a >> 20) - 1012;  // -1012 .. 20
+    const unsigned long long X = n >= 0 ? M << n : M >> (n < -63 ? 63 : -n);
+    const long long sx = (long long)(int)hi >> 63;
+    const long long r = (((long long)X ^ sx) - sx) -
+                        ((long long)k * LEAN64_K_M + (long long)((unsigned long long)(long long)(k * LEAN64_K_H) << 32) +
+                         (int)mulhi_s(k, LEAN64_K_L));
+    // r = rh + rl: the high word rounded and the signed low word
+    const float rh = fmul(i2f((int)((r + 0x80000000ll) >> 32)), 0x1p-31f);
+    const float rl = fmul(i2f((int)(unsigned)r), 0x1p-63f);
+    // d = r^2 (1/2 + r w),  w = 1/6 + r (1/24 + r (1/120 + r/720))
+    const float sh = fmul(rh, rh);
+    const float sl = fmaf(fmul(2.f, rh), rl, fmaf(rh, rh, -sh));
+    const float g = fmul(rh, fmaf(rh, fmaf(rh, 1.f / 720.f, 1.f / 120.f), 1.f / 24.f));
     const float wh = fadd(LEAN64_SIXTH_H, g);
     const float wl = fadd(fadd(g, -fadd(wh, -LEAN64_SIXTH_H)), LEAN64_SIXTH_L);
-    const float vh = fmul(th, wh);
-    const float vl = fmaf(th, wl, fmaf(tl, wh, fmaf(th, wh, -vh)));
+    const float vh = fmul(rh, wh);
+    const float vl = fmaf(rh, wl, fmaf(rl, wh, fmaf(rh, wh, -vh)));
     const float qh = fadd(0.5f, vh);
     const float ql = fadd(fadd(vh, -fadd(qh, -0.5f)), vl);
     const float dh = fmul(sh, qh);
     const float dl = fmaf(sh, ql, fmaf(sl, qh, fmaf(sh, qh, -dh)));
-    // p = r + d - k lo in units of 2^-70
-    const unsigned long long Mr = (br & 0x000FFFFFFFFFFFFFull) | (er ? 0x0010000000000000ull : 0ull);
-    const int shr = 1005 - (int)(er ? er : 1u);  // the weight of bit 0 of Mr is 2^(er - 1075)
-    const long long Pr = (long long)(shr <= 0 ? Mr << (-shr < 10 ? -shr : 10) : Mr >> (shr > 63 ? 63 : shr));
-    // d - k lo as one float pair (two-sum), then into the fixed-point sum
-    const float xs = fadd(dh, -kh);
-    const float xb = fadd(xs, -dh);
-    const float xl = fadd(fadd(fadd(dh, -fadd(xs, -xb)), fadd(-kh, -xb)), fadd(dl, -kl));
-    const long long S = (rs ? -Pr : Pr) + fix_from_float(xs, 70) + fix_from_float(xl, 70);
-    const double p = S == 0 ? 0.0 : fix_to_double(S, 70);
-    const double tj = exp_entry(k & (LEAN64_EXP_N - 1));
-    const double y = fma(tj, p, tj);
-    return ll2d((long long)((unsigned long long)d2ll(y) + ((unsigned long long)(long long)(k >> 7) << 52)));
+    // p = r + d in units of 2^-63
+    unsigned b1, b2;
+    fix_parts(dh, dl, 0x1p39f, b1, b2);
+    const long long p = (long long)((unsigned long long)r - (0x4B400000ull << 24) - (0x4B400000ull << 2) +
+                                    (unsigned long long)b1 * 0x1000000ull + (unsigned long long)b2 * 4ull);
+    // T (1 + p) in units of 2^-61: T = Th 2^31 + Tl, p = ph 2^32 + pl; the
+    // product of the low parts starts at 2^56 so that its sum is not negative
+    const long long T = exp_entry(k & (LEAN64_EXP_N - 1));
+    const int Th = (int)(T >> 31), Tl = (int)(T & 0x7FFFFFFFll), ph = (int)(p >> 32);
+    const unsigned long long V = (unsigned long long)(unsigned)Th * (unsigned)p + 0x0100000000000000ull +
+                                 (unsigned long long)((long long)Tl * (ph * 2));
+    const long long U = T + (long long)Th * ph + (long long)(V >> 32) - 0x01000000ll;
+    // T_0 (1 + p) may lie below 1
+    const int low = (int)(U >> 32) < 0x20000000 ? 1 : 0;
+    const unsigned long long m = (((unsigned long long)U << low) + 0x100ull) >> 9;  // leading bit at 52
+    return ll2d((long long)(((unsigned long long)((k >> 7) - low + 1022) << 52) + m));
 }
 
-// 1/b with no FP64 instruction.  b = +-2^E m, m in [1, 2) split exactly into
-// floats m1 + m2 + m3 (24 + 23 + 6 bits); y0 = MUFU rcp(m1) ~ 1/m to 2^-22;
-// the residual e = 1 - m y0 in float-float (exact products by FMA, 1 - m1 y0
-// exact by Sterbenz); 1/m = y0 (1 + e + e^2) to ~2^-64, summed in 64-bit fixed
-// point (2^-62) and rounded once; 2^-E and the sign go on the bits.  Zero,
-// subnormal, |b| >= 2^1022 (a subnormal result), inf and NaN take IEEE 1/b.
-// a / b is a * lean_rcp(b): one FP64 multiply.
+// 1/b with no FP64 instruction.  b = +-2^E m, m = M 2^-52 in [1, 2);
+// y0 = Y 2^-23 ~ 1/m from the MUFU reciprocal; 1 - m y0 = e = -N 2^-75 exactly
+// (the product M Y modulo 2^64; |e| < 2^-21); 1/m = y0 (1 + e + e^2) to 2^-62,
+// with e and e^2 in units of 2^-60, rounded once; 2^-E and the sign go on the
+// bits.  Zero, subnormal, |b| >= 2^1022 (a subnormal result), inf and NaN take
+// IEEE 1/b.  a / b is a * lean_rcp(b): one FP64 multiply.
 LEAN64_FN double lean_rcp(double b) {
     using namespace detail;
     const unsigned long long bb = (unsigned long long)d2ll(b);
-    const unsigned eb = (unsigned)(bb >> 52) & 0x7FFu;
-    if (eb - 1u >= 2044u)
+    const unsigned hi = (unsigned)(bb >> 32);
+    if ((hi & 0x7FFFFFFFu) - 0x00100000u >= 0x7FC00000u)
         return 1.0 / b;
-    const unsigned long long M = bb & 0x000FFFFFFFFFFFFFull;
-    const float m1 = u2f((127u << 23) | (unsigned)(M >> 29));                                     // [1, 2)
-    const float m2 = fmul(fadd(u2f(0x4B000000u | ((unsigned)(M >> 6) & 0x7FFFFFu)), -8388608.f), 0x1p-46f);
-    const float m3 = fmul(fadd(u2f(0x4B000000u | ((unsigned)M & 0x3Fu)), -8388608.f), 0x1p-52f);
-    const float y0 = rcp_approx(m1);
-    const float p1 = fmul(m1, y0);
-    const float p1e = fmaf(m1, y0, -p1);
-    const float a = fadd(1.f, -p1);  // exact
-    const float p2 = fmul(m2, y0);
-    const float p2e = fmaf(m2, y0, -p2);
-    // e = a - p1e - p2 - (p2e + m3 y0), |e| < 2^-21
-    const float s1 = fadd(a, -p1e);
-    const float s1b = fadd(s1, -a);
-    const float s1e = fadd(fadd(a, -fadd(s1, -s1b)), fadd(-p1e, -s1b));
-    const float eh = fadd(s1, -p2);
-    const float eb2 = fadd(eh, -s1);
-    const float e1 = fadd(fadd(s1, -fadd(eh, -eb2)), fadd(-p2, -eb2));
-    const float el = fadd(fadd(e1, s1e), -fmaf(m3, y0, p2e));
-    // y0 (e + e^2) as a float pair
-    const float ch = fmul(y0, eh);
-    const float cl = fmaf(y0, fmaf(eh, eh, el), fmaf(y0, eh, -ch));
-    const long long S = fix_from_float(y0, 62) + fix_from_float(ch, 62) + fix_from_float(cl, 62);
-    const double ym = fix_to_double(S, 62);  // 1/m in (0.5, 1]
-    return ll2d((long long)(((unsigned long long)d2ll(ym) - ((unsigned long long)(long long)((int)eb - 1023) << 52)) |
-                            (bb & 0x8000000000000000ull)));
+    const float m1 = u2f((((hi << 3) | ((unsigned)bb >> 29)) & 0x007FFFFFu) | 0x3F800000u);
+    const unsigned Y = f2u(fadd(rcp_approx(m1), 1.f)) - 0x3F800000u;  // in (2^22, 2^23]
+    const unsigned long long M = ((unsigned long long)((hi & 0x000FFFFFu) | 0x00100000u) << 32) | (unsigned)bb;
+    const long long N = (long long)(M * Y);
+    const int nh = (int)(N >> 32);
+    // -(e + e^2) in units of 2^-60, rounded
+    const long long c = (N - (long long)((unsigned long long)((long long)nh * nh) >> 11) + 0x4000ll) >> 15;
+    const long long C = (1ll << 29) - c * (long long)Y;  // units of 2^-83, half of 2^-53 added
+    const unsigned long long m = (unsigned long long)((C >> 30) + ((long long)Y << 30));  // 1/m in units of 2^-53
+    const unsigned mh = (unsigned)(m >> 32) + 0x7FC00000u - (hi & 0xFFF00000u);
+    return ll2d((long long)(((unsigned long long)mh << 32) | (unsigned)m));
 }
 
 LEAN64_FN double lean_div(double a, double b) { return a * lean_rcp(b); }
