@@ -50,6 +50,10 @@ typedef struct noa_dcs_consts {
     double br_half_m2;      /* 0.5 mass mass */
     double br_Dn_sqrte_m2;  /* D_n sqrte - 2 */
     double br_BZe_mass;     /* BZ_e mass */
+    double br_n0, br_n1;    /* Phi_n's numerator    BZ_n (mass + delta (D_n sqrte - 2)) = n0 + delta n1 */
+    double br_d0, br_d1;    /* Phi_n's denominator  D_n (me + delta sqrte BZ_n)        = d0 + delta d1 */
+    double br_e0, br_e1;    /* Phi_e's first factor over BZ_e mass, (1 + delta phie) / (BZ_e mass) = e0 + delta e1 */
+    double br_f1;           /* Phi_e's second factor me + delta sqrte BZ_e = me + delta f1 */
 
     /* pair production, dcs.hh:148-170 */
     double pp_Z13;          /* Z^(1/3) */
@@ -66,6 +70,14 @@ typedef struct noa_dcs_consts {
     double pp_cZ;           /* 1.794664e-34 Z */
     double pp_gamma1;       /* form-factor constants, dcs.hh:235-241 */
     double pp_gamma2;
+    double pp_g1;           /* gamma1 Z13 Z13 */
+    double pp_g2;           /* gamma2 Z13 */
+    double pp_6m2;          /* 6 mass mass: x1 = 6 m^2 / (E (E - q)) */
+    double pp_inv_AZ13;     /* 1 / AZ13 */
+    double pp_2sm;          /* 2 sqrte me = cL / AZ13 */
+    double pp_kappa;        /* 1.5 Z13 / r */
+    double pp_2_inv_r2;     /* 2 / (r r) */
+    double pp_cZs;          /* cZ scale_A */
 
     /* photonuclear, dcs.hh:310-319, 370-375 */
     double ph_logA;         /* log(A) */
@@ -74,11 +86,16 @@ typedef struct noa_dcs_consts {
     double ph_log_q02;      /* log(Q02 / Lambda2), ALLM */
     double ph_inv_log_q02;  /* 1 / log(Q02 / Lambda2) */
     double ph_scale;        /* 0.5 cf 1e3 N_A / A, cf = 2.603096e-35 (FP32C final scaling) */
+    double ph_scale_A;      /* ph_scale A */
+    double ph_k1, ph_k0;    /* DRSS exponent (0.069 log10 x + 0.097) log A = k1 log x + k0 */
+    double ph_m2;           /* mass mass */
 
     /* ionisation, dcs.hh:408-443 */
     double io_Wmin;         /* 0.62 I */
     double io_k_rad;        /* 0.5 m1 m1 / me, radiative-correction threshold */
     double io_cZA;          /* 1.535336e-5 Z / A */
+    double io_cW;           /* (mass mass + me me) / (2 me): 1 / W_max = (E + cW) / P2 */
+    double io_4_inv_m2;     /* 4 / (mass mass) */
 
     /* float pairs (hi + lo to ~2^-48) for float-float arithmetic */
     float inv_mass_h, inv_mass_l;  /* 1 / mass */
@@ -124,6 +141,13 @@ static inline void noa_dcs_fill_consts(noa_dcs_consts *c, double A, double I, in
         c->br_half_m2 = 0.5 * mass * mass;
         c->br_Dn_sqrte_m2 = c->br_D_n * sqrte - 2.;
         c->br_BZe_mass = c->br_BZ_e * mass;
+        c->br_n0 = c->br_BZ_n * mass;
+        c->br_n1 = c->br_BZ_n * c->br_Dn_sqrte_m2;
+        c->br_d0 = c->br_D_n * me;
+        c->br_d1 = c->br_D_n * sqrte * c->br_BZ_n;
+        c->br_e0 = 1. / c->br_BZe_mass;
+        c->br_e1 = c->br_phie_factor / c->br_BZe_mass;
+        c->br_f1 = sqrte * c->br_BZ_e;
     }
     { // dcs.hh:153-166, 235-241
         const double sqrte = 1.6487212707;
@@ -145,6 +169,14 @@ static inline void noa_dcs_fill_consts(noa_dcs_consts *c, double A, double I, in
         c->pp_cZ = 1.794664E-34 * (double)Z;
         c->pp_gamma1 = (Z == 1) ? 4.4E-05 : 1.95E-05;
         c->pp_gamma2 = (Z == 1) ? 4.8E-05 : 5.30E-05;
+        c->pp_g1 = c->pp_gamma1 * Z13 * Z13;
+        c->pp_g2 = c->pp_gamma2 * Z13;
+        c->pp_6m2 = 6. * mass * mass;
+        c->pp_inv_AZ13 = Z13 / A_;
+        c->pp_2sm = 2. * sqrte * me;
+        c->pp_kappa = 1.5 * Z13 / r;
+        c->pp_2_inv_r2 = 2. / (r * r);
+        c->pp_cZs = c->pp_cZ * c->scale_A;
     }
     { // dcs.hh:290, 313-315, 370-374
         const double M = 0.931494, mpi = 0.134977;
@@ -155,12 +187,18 @@ static inline void noa_dcs_fill_consts(noa_dcs_consts *c, double A, double I, in
         c->ph_log_q02 = log(0.52544 / 0.06527);
         c->ph_inv_log_q02 = 1. / c->ph_log_q02;
         c->ph_scale = 0.5 * 2.603096E-35 * c->scale_A;
+        c->ph_scale_A = 0.5 * 2.603096E-35 * 1E+03 * NOA_AVOGADRO_NUMBER;
+        c->ph_k1 = 0.069 * 0.43429448190325182765 * c->ph_logA;
+        c->ph_k0 = 0.097 * c->ph_logA;
+        c->ph_m2 = mass * mass;
     }
     { // dcs.hh:422, 435-436
         c->io_Wmin = 0.62 * I;
         const double m1 = mass - me;
         c->io_k_rad = 0.5 * m1 * m1 / me;
         c->io_cZA = 1.535336E-05 * (double)Z / A;
+        c->io_cW = 0.5 * (mass * mass + me * me) / me;
+        c->io_4_inv_m2 = 4. / (mass * mass);
     }
 }
 

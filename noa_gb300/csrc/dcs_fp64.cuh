@@ -72,35 +72,63 @@ static __device__ __noinline__ double ol_exp(double x) { return lean_exp(x); }
 static __device__ __noinline__ double ol_rcp(double x) { return lean_rcp(x); }
 static __device__ __noinline__ double ol_div(double a, double b) { return lean_div(a, b); }
 
-// ---------------------------------------------------------------- bremsstrahlung
-// q < qe_max decides whether the electron term exists (physics.hh:142):
-// against a lean qe_max, and in IEEE arithmetic like the reference when q is
-// within 64 ulp of it.
-__device__ __forceinline__ bool brems_below(double E, double q, const noa_dcs_consts &c) {
-    const double qe_lean = E * lean_rcp(1. + c.br_half_m2 * lean_rcp(ME * E));
-    const long long dist = __double_as_longlong(q) - __double_as_longlong(qe_lean);
-    if (dist < 64 && dist > -64)
-        return brems_below_qe(E, q, c);
-    return q < qe_lean;
+// Whether E (or K) exceeds q by more than a part in 2^10 - 2^11, both of
+// ordinary size (2^-62 to 2^97, and q above 2^-94; NaN and negative values
+// fail).  There 1 - q / E and K - q keep 42 bits or more whatever the rounding
+// of q / E, so that the quotients may be taken lean.  Nearer the edge the
+// reference's own rounding shows in the result (by 1 / (1 - q / E) ulp), and
+// its IEEE operations are kept.  High words only.
+__device__ __forceinline__ bool clear_of_edge(double E, double q) {
+    const int he = __double2hiint(E), hq = __double2hiint(q);
+    return he >= 0x3C000000 && he < 0x46000000 && hq >= 0x3A000000 && he - hq >= 0x400;
 }
 
-__device__ __forceinline__ double brems_fp64(double K, double q, const noa_dcs_consts &c) {
+// ---------------------------------------------------------------- bremsstrahlung
+// q < qe_max decides whether the electron term exists (physics.hh:142):
+// cross-multiplied, q (me E + m^2 / 2) < me E^2, and in IEEE arithmetic like
+// the reference when the two sides are within 64 ulp.
+__device__ __forceinline__ bool brems_below(double E, double q, const noa_dcs_consts &c) {
+    const double t = ME * E;
+    const long long dist = __double_as_longlong(q * (t + c.br_half_m2)) - __double_as_longlong(t * E);
+    if (!(dist >= 64 || dist <= -64) || !clear_of_edge(E, q))
+        return brems_below_qe(E, q, c);
+    return dist < 0;
+}
+
+// The reference's form for pairs near the kinematic edge (nu -> 1, where its
+// rounded nu = q / E shows in 1 - nu) and inputs of unusual size.
+static __device__ __noinline__ double brems_edge(double K, double q, const noa_dcs_consts &c) {
     const double mass = c.mass;
     const double sqrte = 1.648721271;
     const double E = K + mass;
-    const double invE = lean_rcp(E);
-    const double delta_factor = c.br_half_m2 * invE;
-    const bool below = brems_below(E, q, c);
-    const double nu = __ddiv_rn(q, E);  // as the reference: 1 - nu cancels as q -> E
-    const double delta = delta_factor * nu * lean_rcp(1. - nu);
+    const double nu = __ddiv_rn(q, E);
+    const double delta = c.br_half_m2 * lean_rcp(E) * nu * lean_rcp(1. - nu);
     const double Phi_n = clamp0(lean_log(c.br_BZ_n * (mass + delta * c.br_Dn_sqrte_m2) *
                                          lean_rcp(c.br_D_n * (ME + delta * sqrte * c.br_BZ_n))));
     double Phi_e = 0.;
-    if (below)
+    if (brems_below_qe(E, q, c))
         Phi_e = clamp0(lean_log(c.br_BZe_mass *
                                 lean_rcp((1. + delta * c.br_phie_factor) * (ME + delta * sqrte * c.br_BZ_e))));
     const double dcs = c.br_dcs_factor * (c.Zd * Phi_n + Phi_e) * (4. / 3. * (lean_rcp(nu) - 1.) + nu);
     return (dcs < 0.) ? 0. : dcs * c.scale_A;
+}
+
+// 25 FP64 instructions (42 in the reference's form): the element's factors
+// are folded into the two linear forms of each logarithm, Phi_e is taken as
+// the logarithm of the inverse, and the scales are one constant.
+__device__ __forceinline__ double brems_fp64(double K, double q, const noa_dcs_consts &c) {
+    const double E = K + c.mass;
+    if (!clear_of_edge(E, q))
+        return brems_edge(K, q, c);
+    const double invE = lean_rcp(E);
+    const double nu = q * invE;
+    const double delta = c.br_half_m2 * invE * nu * lean_rcp(1. - nu);
+    const double Phi_n = clamp0(lean_log(fma(delta, c.br_n1, c.br_n0) * lean_rcp(fma(delta, c.br_d1, c.br_d0))));
+    double Phi_e = 0.;
+    if (brems_below(E, q, c))
+        Phi_e = clamp0(-lean_log(fma(delta, c.br_e1, c.br_e0) * fma(delta, c.br_f1, ME)));
+    const double shape = fma(4. / 3., E * lean_rcp(q), nu - 4. / 3.);
+    return clamp0(c.br_scale * fma(c.Zd, Phi_n, Phi_e) * shape);
 }
 
 // ---------------------------------------------------------------- pair production
@@ -174,79 +202,147 @@ __device__ __forceinline__ bool pprod_live(double K, double q, const noa_dcs_con
     return pprod_live_tail(K, q, c.mass, c.inv_mass_h, c.inv_mass_l, x0);
 }
 
-__device__ __forceinline__ double pprod_fp64(double K, double q, const noa_dcs_consts &c) {
-    if (q <= 4. * ME)
-        return 0.;
-    if (q >= K + c.pp_kmax_shift)
-        return 0.;
-    const double argmin = pprod_argmin_exact(K, q, c);
-    if ((argmin >= 1.) || (argmin <= 0.))
-        return 0.;
-    const double mass = c.mass;
-    const double E = K + mass;
-    const double nu = __ddiv_rn(q, E);
-    const double beta = 0.5 * nu * nu * ol_rcp(1. - nu);
-    const double xi_factor = c.pp_half_r2 * beta;
-    const double tmin = ol_log(argmin);
-    // Le's two logs share one: log(AZ13 sqrt(xe) q / D1) - log(D2)/2 = log(AZ13^2 q^2 xe / (D1^2 D2)) / 2
-    const double aq2 = (c.pp_AZ13 * q) * (c.pp_AZ13 * q);
-    const double b2 = 2. * beta, b15 = 1.5 * beta, b3 = 3. * beta, b4 = 4. * beta;
+// beta = nu^2 / (2 (1 - nu)) and argmin with the reference's own rounding
+// (nu = q / E rounded, argmin in IEEE order), for pairs near an edge: 1 - nu
+// and log(argmin) amplify the last bit there.
+static __device__ __noinline__ double2 pprod_edge(double K, double q, double mass) {
+    noa_dcs_consts c;  // pprod_argmin_exact reads only the mass
+    c.mass = mass;
+    const double nu = __ddiv_rn(q, K + mass);
+    return make_double2(0.5 * nu * nu * ol_rcp(1. - nu), pprod_argmin_exact(K, q, c));
+}
 
-    double I = 0.;
-#pragma unroll 1  // rolled: 1% faster than unrolled on GB300 (smaller code, same FP64 work)
-    for (int j = 0; j < 8; j++) {
-        const double eps = ol_exp(kGL8X[j] * tmin);
-        const double rho = 1. - eps;
-        const double rho2 = rho * rho;
-        const double rho21 = eps * (2. - eps);
-        const double xi = xi_factor * rho21;
-        const double xi_i = ol_rcp(xi);
-        const double opxi = 1. + xi;
-        const double inv_opxi = ol_rcp(opxi);
+// What one open pair's nodes share.  With s = 1 - rho^2 = eps (2 - eps) every
+// factor of the reference's integrand that does not take a logarithm is linear
+// in s (dcs.hh:188-216), so that it costs one FMA per node:
+//   (2 + rho^2)(1 + beta) + xi (3 + rho^2) = a0 + s (a1 - s xf),  xi = xf s
+//   5 - rho^2 + 4 beta (1 + rho^2)         = n0 + s n1
+//   rho^2 + 2 beta (2 - rho^2)             = -(dc + s ds)
+//   (1 + rho^2)(1 + 1.5 beta) - (1 + 2 beta) s / xi = m0 + s m1
+//   4 + rho^2 + 3 beta (1 + rho^2)         = q0 + s q1
+//   (1 + rho^2)(1.5 + 2 beta)              = e0 + s e1
+// c1 = cL / (AZ13 q) scales the screening lengths, which are taken over q.
+struct PprodPair {
+    double tmin, xf, beta, a0, a1, n0, n1, d1, dc, ds, c1, m0, m1, e0, e1, q0, q1;
+};
 
-        double Be;
-        if (bits_ge(xi, 1E+03))
-            Be = 0.5 * xi_i * ((3. - rho2) + b2 * (1. + rho2));
-        else
-            Be = ((2. + rho2) * (1. + beta) + xi * (3. + rho2)) * ol_log(1. + xi_i) + (rho21 - beta) * inv_opxi -
-                 3. - rho2;
-        const double Ye = ol_div(5. - rho2 + b4 * (1. + rho2),
-                                   2. * (1. + b3) * ol_log(3. + xi_i) - rho2 - b2 * (2. - rho2));
-        const double xe = opxi * (1. + Ye);
-        const double cLi = c.pp_cL * ol_rcp(rho21);
-        const double d1 = q + cLi * xe;
-        const double Le = 0.5 * ol_log(aq2 * xe * ol_rcp(d1 * d1 * (1. + c.pp_cLe * xe)));
-        const double Phi_e = clamp0(Be * Le);
-
-        double Bmu;
-        if (!bits_ge(xi, 1.0000000000000002E-03))  // xi <= 1e-3
-            Bmu = 0.5 * xi * (5. - rho2 + beta * (3. + rho2));
-        else
-            Bmu = ((1. + rho2) * (1. + b15) - xi_i * (1. + b2) * rho21) * ol_log(opxi) +
-                  xi * (rho21 - beta) * inv_opxi + (1. + b2) * rho21;
-        const double Ymu = ol_div(4. + rho2 + b3 * (1. + rho2),
-                                    (1. + rho2) * (1.5 + b2) * ol_log(3. + xi) + 1. - 1.5 * rho2);
-        const double xmu = opxi * (1. + Ymu);
-        const double Lmu = ol_log(c.pp_r_AZ13 * q * ol_rcp(c.pp_15_Z13 * (q + cLi * xmu)));
-        const double Phi_mu = clamp0(Bmu * Lmu);
-        const double f = -(Phi_e + Phi_mu * c.pp_inv_r2) * (1. - rho) * tmin;
-        I = fma(f, kGL8W[j], I);
+__device__ __forceinline__ void pprod_setup(double K, double q, const noa_dcs_consts &c, PprodPair &p) {
+    const double E = K + c.mass;
+    const double rq = ol_rcp(q);
+    double beta, argmin;
+    bool edge = !clear_of_edge(K, q);
+    if (!edge) {
+        // gamma = E / m and gamma - q / m = (E - q) / m
+        const double rEE = ol_rcp(E * (E - q));
+        beta = (0.5 * q) * q * rEE;
+        const double x0 = 4. * ME * rq, x1 = c.pp_6m2 * rEE;
+        const double omx0 = 1. - x0;
+        argmin = fma(2., omx0 * x1, x0) * ol_rcp(fma(1. - x1, lean64::lean_sqrt(omx0), 1.));
+        edge = __double2hiint(argmin) >= 0x3FEFF800;  // argmin >= 1 - 2^-10
     }
+    if (edge) {
+        const double2 e = pprod_edge(K, q, c.mass);
+        beta = e.x;
+        argmin = e.y;
+    }
+    p.tmin = ol_log(argmin);
+    p.beta = beta;
+    p.xf = c.pp_half_r2 * beta;
+    p.a0 = fma(3., beta, 3.);
+    p.a1 = fma(4., p.xf, -1. - beta);
+    p.n0 = fma(8., beta, 4.);
+    p.n1 = fma(-4., beta, 1.);
+    p.d1 = fma(6., beta, 2.);
+    p.dc = fma(-2., beta, -1.);
+    p.ds = fma(-2., beta, 1.);
+    p.c1 = c.pp_2sm * rq;
+    p.m0 = fma(p.dc, ol_rcp(p.xf), fma(3., beta, 2.));
+    p.m1 = fma(-1.5, beta, -1.);
+    p.e0 = fma(4., beta, 3.);
+    p.e1 = fma(-2., beta, -1.5);
+    p.q0 = fma(6., beta, 5.);
+    p.q1 = fma(-3., beta, -1.);
+}
 
-    const double gamma = __dadd_rn(1., __ddiv_rn(K, mass));
+// Clamp of the reference's `if (Phi < 0.) Phi = 0.;` for -Phi; keeps NaN.
+__device__ __forceinline__ double clamp0_neg(double v) {
+    return (unsigned long long)(__double_as_longlong(v) - 1) < 0x7FF0000000000000ULL ? 0. : v;
+}
+
+// Node j: w_j (1 - rho) (-2) (Phi_e + Phi_mu / r^2), 51 FP64 instructions (about 75
+// in the reference's form) beside 6 logarithms, an exponential and 6
+// reciprocals.  The screening logarithms are those of the inverse arguments,
+//   Le  = -log(d^2 (1 / xe + cLe)) / 2,   d = 1 / AZ13 + c1 xe / s
+//   Lmu = -log(kappa (1 / AZ13 + c1 xmu / s)),
+// which spares their products with 1 / d and the square root.
+__device__ __forceinline__ double pprod_node(const PprodPair &p, int j, const noa_dcs_consts &c) {
+    const double eps = ol_exp(kGL8X[j] * p.tmin);
+    const double s = eps * (2. - eps);
+    const double xi = p.xf * s;
+    const double xi_i = ol_rcp(xi);
+    const double opxi = 1. + xi;
+    const double inv_opxi = ol_rcp(opxi);
+    const double sb = s - p.beta;
+    const double crs = p.c1 * ol_rcp(s);
+
+    double Be;
+    if (bits_ge(xi, 1E+03))
+        Be = xi_i * fma(0.5 * s, p.ds, -p.dc);
+    else
+        Be = fma(fma(s, fma(-s, p.xf, p.a1), p.a0), ol_log(1. + xi_i), fma(sb, inv_opxi, s - 4.));
+    const double Ye = fma(s, p.n1, p.n0) * ol_rcp(fma(p.d1, ol_log(3. + xi_i), fma(s, p.ds, p.dc)));
+    const double xe = fma(opxi, Ye, opxi);
+    const double de = fma(crs, xe, c.pp_inv_AZ13);
+    const double Pe = clamp0_neg(Be * ol_log(de * de * (ol_rcp(xe) + c.pp_cLe)));
+
+    double Bmu;
+    if (!bits_ge(xi, 1.0000000000000002E-03))  // xi <= 1e-3
+        Bmu = 0.5 * xi * fma(p.beta, 4. - s, 4. + s);
+    else
+        Bmu = fma(fma(s, p.m1, p.m0), ol_log(opxi), fma(sb, xi * inv_opxi, -p.dc * s));
+    const double Ymu = fma(s, p.q1, p.q0) *
+                       ol_rcp(fma(fma(s, p.e1, p.e0), ol_log(3. + xi), fma(1.5, s, -0.5)));
+    const double xmu = fma(opxi, Ymu, opxi);
+    const double Pmu = clamp0_neg(Bmu * ol_log(c.pp_kappa * fma(crs, xmu, c.pp_inv_AZ13)));
+    // 1 - rho as the reference rounds it: for small eps its last bit (2^-54 / eps) shows in the result
+    return fma(Pmu, c.pp_2_inv_r2, Pe) * (1. - (1. - eps)) * kGL8W[j];
+}
+
+// From the sum of the nodes: the atomic-electron form factor zeta and the
+// scales.  (mass + K) / E of the reference's two factors cancels.
+__device__ __forceinline__ double pprod_finish(double K, double q, double tmin, double sum, const noa_dcs_consts &c) {
+    const double E = K + c.mass;
+    const double gamma = E * c.inv_mass;
     double zeta = 0.;
     if (!(gamma <= 35.)) {
-        zeta = 0.073 * ol_log(gamma * ol_rcp(1. + c.pp_gamma1 * gamma * c.pp_Z13 * c.pp_Z13)) - 0.26;
+        zeta = 0.073 * ol_log(gamma * ol_rcp(fma(c.pp_g1, gamma, 1.))) - 0.26;
         if (zeta <= 0.)
             zeta = 0.;
         else
-            zeta = ol_div(zeta, 0.058 * ol_log(gamma * ol_rcp(1. + c.pp_gamma2 * gamma * c.pp_Z13)) - 0.14);
+            zeta = zeta * ol_rcp(0.058 * ol_log(gamma * ol_rcp(fma(c.pp_g2, gamma, 1.))) - 0.14);
     }
-    const double dcs = ol_div(c.pp_cZ * (c.Zd + zeta) * (E - q) * I, q * E);
-    return (dcs < 0.) ? 0. : dcs * (mass + K) * c.scale_A;
+    return clamp0(c.pp_cZs * (c.Zd + zeta) * (E - q) * (0.5 * tmin * sum) * ol_rcp(q));
+}
+
+// An open pair (pprod_live), its nodes one after the other.
+__device__ __forceinline__ double pprod_fp64(double K, double q, const noa_dcs_consts &c) {
+    PprodPair p;
+    pprod_setup(K, q, c, p);
+    double sum = 0.;
+#pragma unroll 1  // rolled: smaller code, same FP64 work
+    for (int j = 0; j < 8; j++)
+        sum += pprod_node(p, j, c);
+    return pprod_finish(K, q, p.tmin, sum, c);
 }
 
 // ---------------------------------------------------------------- photonuclear
+// Q2min and Q2max with the reference's own rounding, for pairs near an edge.
+static __device__ __noinline__ double2 photo_edge(double K, double q, double mass) {
+    const double y = __ddiv_rn(q, K + mass);
+    return make_double2(__ddiv_rn(x_mul(x_mul(x_mul(mass, mass), y), y), x_sub(1., y)),
+                        x_sub(x_mul(2.0 * PH_M, q - PH_MPI), PH_MPI * PH_MPI));
+}
+
 // photo_window's open / closed decision (dcs.hh:357-381), float first: in
 // float every bound is decided with a relative margin of 1e-5 (1e-4 of the
 // terms for Q2max >= Q2min, whose float difference cancels near q_min; with
@@ -279,18 +375,51 @@ __device__ __forceinline__ bool photo_live(double K, double q, const noa_dcs_con
     return photo_window(K, q, c, a, b);
 }
 
-__device__ __forceinline__ double photo_fp64(double K, double q, const noa_dcs_consts &c) {
-    double Q2min, Q2max;
-    if (!photo_window(K, q, c, Q2min, Q2max))
-        return 0.;
-    const double mass = c.mass;
-    const double E = K + mass;
-    const double y = __ddiv_rn(q, E);
-    const double pQ2min = ol_log(Q2min);
-    const double pQ2max = ol_log(Q2max);
-    const double dpQ2 = pQ2max - pQ2min;
-    const double pQ2c = 0.5 * (pQ2max + pQ2min);
+// What one open pair's nodes share.
+struct PhotoPair {
+    double pc, hd;          // log Q2 = pc + hd x_j
+    double h;               // x = h Q2
+    double inv_dP, inv_dR;  // 1 / (mP2 + 2 M q), 1 / (mR2 + 2 M q)
+    double k2;              // DRSS exponent k1 log Q2 + k2
+    double omy, yy, invEE;  // 1 - y, y^2, 1 / E^2
+};
 
+__device__ __forceinline__ void photo_setup(double K, double q, const noa_dcs_consts &c, PhotoPair &p) {
+    const double E = K + c.mass;
+    const double invE = ol_rcp(E);
+    double Q2min = 0., Q2max = 0.;
+    bool edge = !clear_of_edge(K, q);
+    if (!edge) {
+        const double mq = c.mass * q;
+        Q2min = mq * mq * ol_rcp(E * (E - q));
+        Q2max = fma(2.0 * PH_M, q, -(2.0 * PH_M * PH_MPI + PH_MPI * PH_MPI));
+        edge = __double2hiint(Q2max) - __double2hiint(Q2min) < 0x400;  // a nearly closed window
+    }
+    if (edge) {
+        const double2 e = photo_edge(K, q, c.mass);
+        Q2min = e.x;
+        Q2max = e.y;
+    }
+    const double half_min = 0.5 * ol_log(Q2min), log_max = ol_log(Q2max);
+    p.pc = fma(0.5, log_max, half_min);
+    p.hd = fma(0.5, log_max, -half_min);
+    p.h = (0.5 / PH_M) * ol_rcp(q);
+    p.inv_dP = ol_rcp(fma(2.0 * PH_M, q, 49.457));
+    p.inv_dR = ol_rcp(fma(2.0 * PH_M, q, 0.15052));
+    p.k2 = fma(c.ph_k1, ol_log(p.h), c.ph_k0);
+    const double y = q * invE;
+    p.omy = (E - q) * invE;
+    p.yy = y * y;
+    p.invEE = invE * invE;
+}
+
+// Node j: w_j (F2A / (A / 2)) Q2 dds of dcs.hh:289-354, 62 FP64 instructions
+// (about 90 in the reference's form) beside 6 logarithms, 10 exponentials and
+// 8 reciprocals.  W2 - M2 = Q2 (1/x - 1) = 2 M q - Q2, which makes the
+// denominators of xP and xR constants of the pair; log x and log(Q2 / 0.04)
+// follow from log Q2 = pc + hd x_j; c1 + (c1 - c2) (1 / (1 + e) - 1) is
+// c2 + (c1 - c2) / (1 + e); Q2 / Q2^2 is taken together.
+__device__ __forceinline__ double photo_node(const PhotoPair &p, int j, const noa_dcs_consts &c) {
     // ALLM parameters, dcs.hh:262-288.
     const double m02 = 0.31985, mP2 = 49.457, mR2 = 0.15052, Q02 = 0.52544;
     const double cP1 = 0.28067, cP2 = 0.22291, cP3 = 2.1979;
@@ -299,62 +428,57 @@ __device__ __forceinline__ double photo_fp64(double K, double q, const noa_dcs_c
     const double cR1 = 0.80107, cR2 = 0.97307, cR3 = 3.4942;
     const double aR1 = 0.58400, aR2 = 0.37888, aR3 = 2.6063;
     const double bR1 = 0.01147, bR2 = 3.7582, bR3 = 0.49338;
-    const double M2 = 0.8803505929;
     const double inv_lambda2 = 1. / 0.06527;
-    const double inv_ln10 = 0.43429448190325182765;
 
-    const double cf = 2.603096E-35;
-    const double invEE = ol_rcp(E * E);
-    const double inv_q = ol_rcp(q);
-    const double Mq = PH_M * q;
-    const double inv_Mq = ol_rcp(Mq);
-    const double two_Mq = 2. * Mq;
-    const double two_m2 = 2 * mass * mass;
-    const double yy = y * y;
-    double ds = 0.;
+    const double lq = fma(p.hd, kGL9X[j], p.pc);
+    const double Q2 = ol_exp(lq);
+    const double invQ2 = ol_rcp(Q2);
+    const double x = p.h * Q2;
+    // ALLM F2, dcs.hh:289-306
+    const double lnt = ol_log(ol_log(ol_log((Q2 + Q02) * inv_lambda2) * c.ph_inv_log_q02));
+    const double cP = fma(cP1 - cP2, ol_rcp(1.0 + ol_exp(cP3 * lnt)), cP2);
+    const double aP = fma(aP1 - aP2, ol_rcp(1.0 + ol_exp(aP3 * lnt)), aP2);
+    const double bP = fma(bP2, ol_exp(bP3 * lnt), bP1);
+    const double l1x = ol_log(1. - x);
+    double F2 = cP * ol_exp(fma(aP, ol_log((Q2 + mP2) * p.inv_dP), bP * l1x));
+    const double cR = fma(cR2, ol_exp(cR3 * lnt), cR1);
+    const double aR = fma(aR2, ol_exp(aR3 * lnt), aR1);
+    const double bR = fma(bR2, ol_exp(bR3 * lnt), bR1);
+    F2 = fma(cR, ol_exp(fma(aR, ol_log((Q2 + mR2) * p.inv_dR), bR * l1x)), F2);
+    F2 = Q2 * ol_rcp(Q2 + m02) * F2;
+    // DRSS shadowing, dcs.hh:310-319
+    if (!bits_ge(x, 0.0014))
+        F2 *= c.ph_a_low;
+    else if (!bits_ge(x, 0.04))
+        F2 *= ol_exp(fma(c.ph_k1, lq, p.k2));
+    F2 *= fma(x, fma(x, fma(x, x - 2.35, 2.45), -1.85), 2.0);
+    // 1 + R, Whitlow, dcs.hh:322-332
+    const bool low = !bits_ge(Q2, 0.3);
+    const double q2 = low ? 0.3 : Q2;
+    const double inv_q2 = low ? 1. / 0.3 : invQ2;
+    const double lg = low ? 2.0149030205422647 : lq + 3.2188758248682006;  // log(25 q2)
+    const double theta = fma(12.0 * 0.015625 * q2, ol_rcp((1.0 + q2) * fma(x, x, 0.015625)), 1.);
+    const double R1 = fma(-0.3534, ol_rcp(fma(q2, q2, 0.09)),
+                          fma(0.5747, inv_q2, fma(0.635 * theta, ol_rcp(lg), 1.)));
+    // dcs.hh:348-354, times Q2
+    const double t = fma(-c.ph_m2, invQ2, 0.5) * fma(Q2, p.invEE, p.yy);
+    const double dds = fma(fma(t, ol_rcp(R1), p.omy), invQ2, -0.25 * p.invEE);
+    return F2 * dds * kGL9W[j];
+}
+
+__device__ __forceinline__ double photo_finish(double K, double q, double hd, double sum, const noa_dcs_consts &c) {
+    return clamp0(c.ph_scale_A * sum * hd * (K + c.mass) * ol_rcp(q));
+}
+
+// An open pair (photo_live), its nodes one after the other.
+__device__ __forceinline__ double photo_fp64(double K, double q, const noa_dcs_consts &c) {
+    PhotoPair p;
+    photo_setup(K, q, c, p);
+    double sum = 0.;
 #pragma unroll 1
-    for (int j = 0; j < 9; j++) {
-        const double Q2 = ol_exp(pQ2c + 0.5 * dpQ2 * kGL9X[j]);
-        const double invQ2 = ol_rcp(Q2);
-        const double x = 0.5 * Q2 * inv_Mq;
-        // ALLM F2, dcs.hh:289-306
-        const double W2 = M2 + Q2 * (two_Mq * invQ2 - 1.0);
-        const double t = ol_log(ol_log((Q2 + Q02) * inv_lambda2) * c.ph_inv_log_q02);
-        const double xP = (Q2 + mP2) * ol_rcp(Q2 + mP2 + W2 - M2);
-        const double xR = (Q2 + mR2) * ol_rcp(Q2 + mR2 + W2 - M2);
-        const double lnt = ol_log(t);
-        const double cP = cP1 + (cP1 - cP2) * (ol_rcp(1.0 + ol_exp(cP3 * lnt)) - 1.0);
-        const double aP = aP1 + (aP1 - aP2) * (ol_rcp(1.0 + ol_exp(aP3 * lnt)) - 1.0);
-        const double bP = bP1 + bP2 * ol_exp(bP3 * lnt);
-        const double cR = cR1 + cR2 * ol_exp(cR3 * lnt);
-        const double aR = aR1 + aR2 * ol_exp(aR3 * lnt);
-        const double bR = bR1 + bR2 * ol_exp(bR3 * lnt);
-        const double l1x = ol_log(1 - x);
-        const double F2P = cP * ol_exp(aP * ol_log(xP) + bP * l1x);
-        const double F2R = cR * ol_exp(aR * ol_log(xR) + bR * l1x);
-        const double F2p = Q2 * ol_rcp(Q2 + m02) * (F2P + F2R);
-        // DRSS shadowing, dcs.hh:310-319
-        double a = 1.0;
-        if (x < 0.0014)
-            a = c.ph_a_low;
-        else if (x < 0.04)
-            a = ol_exp((0.069 * (ol_log(x) * inv_ln10) + 0.097) * c.ph_logA);
-        const double F2A = 0.5 * c.A * a * (2.0 + x * (-1.85 + x * (2.45 + x * (-2.35 + x)))) * F2p;
-        // Whitlow R, dcs.hh:322-332
-        const bool low = !bits_ge(Q2, 0.3);
-        const double q2 = low ? 0.3 : Q2;
-        const double inv_q2 = low ? 1. / 0.3 : invQ2;
-        const double theta = 1 + 12.0 * q2 * 0.015625 * ol_rcp((1.0 + q2) * (0.015625 + x * x));
-        const double R = 0.635 * theta * ol_rcp(ol_log(q2 * 25.)) + 0.5747 * inv_q2 -
-                         0.3534 * ol_rcp(0.09 + q2 * q2);
-        // dcs.hh:348-354
-        const double dds = (1 - y + 0.5 * (1 - two_m2 * invQ2) * (yy + Q2 * invEE) * ol_rcp(1 + R)) *
-                               (invQ2 * invQ2) -
-                           0.25 * invEE * invQ2;
-        const double d2 = cf * F2A * dds * inv_q;
-        ds = fma(d2 * Q2, kGL9W[j], ds);
-    }
-    return (ds < 0.) ? 0. : 0.5 * ds * dpQ2 * (mass + K) * c.scale_A;
+    for (int j = 0; j < 9; j++)
+        sum += photo_node(p, j, c);
+    return photo_finish(K, q, p.hd, sum, c);
 }
 
 // Out-of-line entries of the two quadrature bodies for the FP32C redo paths
@@ -389,37 +513,36 @@ __device__ __forceinline__ int ion_first_exit(double K, double q, const noa_dcs_
     return (W > cut * hi && qf < W * lo) ? 1 : -1;
 }
 
+// 22 FP64 instructions on the open path (about 35 in the reference's form):
+// 1 / W_max = (E + cW) / P2, and 1 / P2 is taken out of the close-collision
+// bracket; the comparisons are of bit patterns where K and q are positive and
+// normal (first > 0).
 __device__ __forceinline__ double ion_fp64(double K, double q, const noa_dcs_consts &c) {
-    const double mass = c.mass;
-    const double P2 = K * (K + 2. * mass);
-    const double E = K + mass;
+    const double E = K + c.mass;
+    const double P2 = K * (E + c.mass);
     const int first = ion_first_exit(K, q, c);
-    double inv_Wmax;
+    if (first == 0)
+        return 0.;
+    double EcW = E + c.io_cW;  // P2 / W_max
+    bool radiative;
     if (first < 0) {
-        const double Wmax = ion_wmax(P2, E, c);
-        if ((Wmax < NOA_X_FRACTION * K) || (q > Wmax))
+        const double P2_ref = K * (K + 2. * c.mass);
+        const double Wmax = ion_wmax(P2_ref, E, c);
+        if ((Wmax < NOA_X_FRACTION * K) || (q > Wmax) || (q <= c.io_Wmin))
             return 0.;
-        inv_Wmax = lean_rcp(Wmax);
-    } else if (first == 0) {
-        return 0.;
+        EcW = P2 * lean_rcp(Wmax);
+        radiative = K >= c.io_k_rad;
     } else {
-        // 1 / W_max = (mass^2 + me (me + 2 E)) / (2 me P2), lean
-        inv_Wmax = (mass * mass + ME * (ME + 2. * E)) * lean_rcp(2. * ME * P2);
+        if (bits_ge(c.io_Wmin, q))
+            return 0.;
+        radiative = bits_ge(K, c.io_k_rad);
     }
-    if (q <= c.io_Wmin)
-        return 0.;
-    const double inv_P2 = lean_rcp(P2);
     const double inv_q = lean_rcp(q);
-    const double a0 = 0.5 * inv_P2;
-    const double a1 = -inv_Wmax;
-    const double a2 = E * E * inv_P2;
-    const double cs = c.io_cZA * E * (a0 + inv_q * (a1 + a2 * inv_q));
-    double Delta = 0.;
-    if (K >= c.io_k_rad) {
-        const double L1 = lean_log(1. + q * (2. / ME));
-        Delta = 1.16141E-03 * L1 * (lean_log(4. * E * (E - q) * c.inv_m2) - L1);
-    }
-    return cs * (1. + Delta);
+    const double cs = c.io_cZA * E * lean_rcp(P2) * fma(inv_q, fma(E * E, inv_q, -EcW), 0.5);
+    if (!radiative)
+        return cs;
+    const double L1 = lean_log(fma(q, 2. / ME, 1.));
+    return cs * fma(1.16141E-03 * L1, lean_log(c.io_4_inv_m2 * E * (E - q)) - L1, 1.);
 }
 
 } // namespace noa_dcs
