@@ -4,19 +4,17 @@
  * Two launch shapes:
  *
  *  - map kernel (bremsstrahlung, ionisation): every pair is live or nearly so
- *    and the body is short, so each thread evaluates ITEMS pairs of a
- *    block-contiguous tile with coalesced loads and stores.
+ *    and the body is short: one pair a thread and step.
  *
  *  - compacting kernel (pair production, photonuclear): ~46% / ~80% of the
  *    pairs of the seeded workload are closed kinematically and the live ones
  *    run an 8- or 9-node quadrature.  A CTA classifies a tile with the cheap
  *    bound checks (the reference's early returns), writes the zeros straight
  *    away, and appends the live pairs (K, q, index) to a queue in shared
- *    memory.  Whenever the queue holds a full CTA's worth of work, every
- *    thread pops one pair and runs the quadrature, so all 32 lanes of a warp
- *    take the same trip through the node loop.  The remainder is drained after
- *    the last tile.  This is the warp-uniform regime grouping of the hot path;
- *    it needs no global scratch.
+ *    memory.  Whenever the queue holds a full batch, and at the end for the
+ *    remainder, the CTA evaluates it together (quad_batch).  The tile follows
+ *    the size of the call, so that a short list spreads over the SMs.  No
+ *    global scratch.
  *
  * Each kernel calls the evaluation from exactly one place.  nvcc inlines
  * every call site separately and may contract a * b + c into an FMA
@@ -30,38 +28,37 @@
  * (physics.hh:126-128); it has no GPU pair-production, photonuclear or
  * ionisation kernel.
  */
-#include "dcs_fp64.cuh"
-#include "dcs_launch.h"
+#include "dcs_quad.cuh"
 
 #include <cuda_runtime.h>
 
 namespace noa_dcs {
 
-constexpr int MAP_THREADS = 256;
-constexpr int MAP_ITEMS = 4;
-constexpr int CMP_THREADS = 256;
-constexpr int CMP_ITEMS = 4;
-constexpr int CMP_TILE = CMP_THREADS * CMP_ITEMS;
+constexpr int MAP_THREADS = 128;
+constexpr int MAP_MIN_CTAS = 10;
+// One pair a thread up to 1000 CTAs an SM (19e6 pairs), grid-stride beyond:
+// the hardware's own distribution of short CTAs balances the SMs better than
+// a resident grid (1e7 pairs 516 / 360 us against 525 / 368 us at 10 CTAs an
+// SM, 1e6 pairs 69 / 52 against 72 / 53).
+constexpr int MAP_GRID_CTAS = 1000;
+constexpr int CMP_THREADS = 128;
+constexpr int CMP_ITEMS = 2;
+constexpr int CMP_TILE = CMP_THREADS * CMP_ITEMS;  // largest tile
 constexpr int CMP_QCAP = CMP_TILE + CMP_THREADS;
 
 // Resident CTAs per SM that the compacting kernels are compiled for (the
-// register budget per thread follows).  Measured on 1e8 pairs: pair
-// production 82.1 ms at 2 (108 registers) against 89.4 ms at 3 and 82.1 ms
-// at 1; photonuclear 45.0 ms at 4 (64 registers) against 47.6 ms at 3,
-// 45.2 ms at 5 and 46.0 ms at 2.
-#define NOA_DCS_PPROD_MIN_CTAS 2
-#define NOA_DCS_PHOTO_MIN_CTAS 4
-
+// register budget per thread follows) and their grid is made of.  Measured at
+// 1e7 pairs: pair production 5.13 / 5.06 / 5.07 ms at 4 / 5 / 6; photonuclear
+// 2.56 / 2.49 / 2.45 / 2.48 ms at 5 / 6 / 7 / 8.
+#ifndef NOA_DCS_PPROD_MIN_CTAS
+#define NOA_DCS_PPROD_MIN_CTAS 5
+#endif
+#ifndef NOA_DCS_PHOTO_MIN_CTAS
+#define NOA_DCS_PHOTO_MIN_CTAS 7
+#endif
 template <int PROC>
-__device__ __forceinline__ double eval_fp64(double K, double q, const noa_dcs_consts &c) {
-    if (PROC == NOA_DCS_PROC_BREMS)
-        return brems_fp64(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PPROD)
-        return pprod_fp64(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PHOTO)
-        return photo_fp64(K, q, c);
-    else
-        return ion_fp64(K, q, c);
+constexpr int cmp_min_ctas() {
+    return PROC == NOA_DCS_PROC_PHOTO ? NOA_DCS_PHOTO_MIN_CTAS : NOA_DCS_PPROD_MIN_CTAS;
 }
 
 template <int PROC>
@@ -73,63 +70,26 @@ __device__ __forceinline__ bool live_fp64(double K, double q, const noa_dcs_cons
 }
 
 template <int PROC>
-__global__ void __launch_bounds__(MAP_THREADS) dcs_fp64_map_kernel(const double *__restrict__ K,
+__global__ void __launch_bounds__(MAP_THREADS, MAP_MIN_CTAS) dcs_fp64_map_kernel(const double *__restrict__ K,
                                                                    const double *__restrict__ q, double *out,
                                                                    int64_t n, const noa_dcs_consts c) {
-    const int64_t tile = (int64_t)MAP_THREADS * MAP_ITEMS;
-    for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
 #pragma unroll 1  // one inlined copy of the evaluation
-        for (int j = 0; j < MAP_ITEMS; j++) {
-            const int64_t i = base + j * MAP_THREADS + threadIdx.x;
-            const double v = eval_fp64<PROC>(i < n ? K[i] : 1., i < n ? q[i] : 1., c);
-            if (i < n)
-                out[i] = v;
-        }
-    }
-}
-
-// Block-wide exclusive scan of one small count per thread.
-__device__ __forceinline__ int block_exclusive_scan(int v, int *warp_tot, int *total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o)
-            x += y;
-    }
-    if (lane == 31)
-        warp_tot[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        int w = lane < (int)(blockDim.x >> 5) ? warp_tot[lane] : 0;
-        int s = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o)
-                s += y;
-        }
-        if (lane < (int)(blockDim.x >> 5))
-            warp_tot[lane] = s - w;
-        if (lane == 31)
-            *total = s;
-    }
-    __syncthreads();
-    return warp_tot[warp] + x - v;
+    for (int64_t i = (int64_t)blockIdx.x * MAP_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * MAP_THREADS)
+        out[i] = PROC == NOA_DCS_PROC_BREMS ? brems_fp64(K[i], q[i], c) : ion_fp64(K[i], q[i], c);
 }
 
 template <int PROC>
-__global__ void __launch_bounds__(CMP_THREADS, PROC == NOA_DCS_PROC_PHOTO ? NOA_DCS_PHOTO_MIN_CTAS : NOA_DCS_PPROD_MIN_CTAS) dcs_fp64_compact_kernel(const double *__restrict__ K,
-                                                                       const double *__restrict__ q, double *out,
-                                                                       int64_t n, const noa_dcs_consts c) {
+__global__ void __launch_bounds__(CMP_THREADS, cmp_min_ctas<PROC>())
+    dcs_fp64_compact_kernel(const double *__restrict__ K, const double *__restrict__ q, double *out, int64_t n, int tile,
+                            const noa_dcs_consts c) {
     __shared__ double qK[CMP_QCAP];
     __shared__ double qQ[CMP_QCAP];
     __shared__ int64_t qI[CMP_QCAP];
+    __shared__ QuadSmem<PROC, CMP_THREADS> quad;
     __shared__ int warp_tot[CMP_THREADS / 32];
     __shared__ int tile_live;
     int qn = 0; // queue length, identical in every thread
-    int64_t base = (int64_t)blockIdx.x * CMP_TILE;
+    int64_t base = (int64_t)blockIdx.x * tile;
     for (;;) {
         const bool more = base < n;  // block-uniform
         if (more) {
@@ -137,8 +97,9 @@ __global__ void __launch_bounds__(CMP_THREADS, PROC == NOA_DCS_PROC_PHOTO ? NOA_
             unsigned live = 0;
 #pragma unroll
             for (int j = 0; j < CMP_ITEMS; j++) {
-                const int64_t i = base + j * CMP_THREADS + threadIdx.x;
-                if (i < n) {
+                const int o = j * CMP_THREADS + threadIdx.x;
+                const int64_t i = base + o;
+                if (o < tile && i < n) {
                     k[j] = K[i];
                     r[j] = q[i];
                     if (live_fp64<PROC>(k[j], r[j], c))
@@ -147,8 +108,7 @@ __global__ void __launch_bounds__(CMP_THREADS, PROC == NOA_DCS_PROC_PHOTO ? NOA_
                         out[i] = 0.;
                 }
             }
-            const int mine = __popc(live);
-            int pos = qn + block_exclusive_scan(mine, warp_tot, &tile_live);
+            int pos = qn + block_scan<CMP_THREADS>(__popc(live), warp_tot, &tile_live);
 #pragma unroll
             for (int j = 0; j < CMP_ITEMS; j++) {
                 if (live & (1u << j)) {
@@ -160,15 +120,19 @@ __global__ void __launch_bounds__(CMP_THREADS, PROC == NOA_DCS_PROC_PHOTO ? NOA_
             }
             __syncthreads();
             qn += tile_live;
-            base += (int64_t)gridDim.x * CMP_TILE;
+            base += (int64_t)gridDim.x * tile;
         }
         // full batches while tiles remain, then the remainder: one call site
         while (qn >= CMP_THREADS || (!more && qn > 0)) {
             const int take = qn < CMP_THREADS ? qn : CMP_THREADS;
-            if ((int)threadIdx.x < take) {
-                const int e = qn - take + threadIdx.x;
-                out[qI[e]] = eval_fp64<PROC>(qK[e], qQ[e], c);
-            }
+            const int first = qn - take;
+            quad_batch<PROC, CMP_THREADS>(
+                quad, take, c,
+                [&](int e, double &k, double &r) {
+                    k = qK[first + e];
+                    r = qQ[first + e];
+                },
+                [&](int e, double v) { out[qI[first + e]] = v; });
             qn -= take;
             __syncthreads();
         }
@@ -184,24 +148,28 @@ static int sm_count() {
     return sms > 0 ? sms : 1;
 }
 
+static int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
 template <int PROC>
 static cudaError_t launch_map(const double *K, const double *q, double *out, int64_t n, const noa_dcs_consts &c,
                               cudaStream_t s) {
-    const int64_t tile = (int64_t)MAP_THREADS * MAP_ITEMS;
-    const int64_t tiles = (n + tile - 1) / tile;
-    const int64_t cap = (int64_t)sm_count() * 8;
-    const int grid = (int)(tiles < cap ? tiles : cap);
-    dcs_fp64_map_kernel<PROC><<<grid, MAP_THREADS, 0, s>>>(K, q, out, n, c);
+    const int64_t blocks = ceil_div(n, MAP_THREADS);
+    const int64_t cap = (int64_t)sm_count() * MAP_GRID_CTAS;
+    dcs_fp64_map_kernel<PROC><<<(int)(blocks < cap ? blocks : cap), MAP_THREADS, 0, s>>>(K, q, out, n, c);
     return cudaGetLastError();
 }
 
+// One resident wave at most, in equal tiles: the largest tile while the call
+// fills it, else n spread over all resident CTAs, so that a short list reaches
+// every SM; not below 8 pairs (two warps of nodes).
 template <int PROC>
 static cudaError_t launch_compact(const double *K, const double *q, double *out, int64_t n,
                                   const noa_dcs_consts &c, cudaStream_t s) {
-    const int64_t tiles = (n + CMP_TILE - 1) / CMP_TILE;
-    const int64_t cap = (int64_t)sm_count() * 4;
-    const int grid = (int)(tiles < cap ? tiles : cap);
-    dcs_fp64_compact_kernel<PROC><<<grid, CMP_THREADS, 0, s>>>(K, q, out, n, c);
+    const int64_t cap = (int64_t)sm_count() * cmp_min_ctas<PROC>();
+    const int64_t steps = ceil_div(n, cap * CMP_TILE);
+    int64_t tile = ceil_div(n, cap * steps);
+    tile = tile < 8 ? 8 : tile;
+    dcs_fp64_compact_kernel<PROC><<<(int)ceil_div(n, tile * steps), CMP_THREADS, 0, s>>>(K, q, out, n, (int)tile, c);
     return cudaGetLastError();
 }
 

@@ -14,22 +14,29 @@
  * Kernel: a CTA takes a tile of kpt kinetic energies and all their nodes
  * (kpt * nodes pairs, at most 1536).  Each pair (K, q_i) is classified with the
  * process's exact bounds; closed pairs contribute 0, open ones go to the
- * shared-memory work queue and are evaluated 256 at a time with every lane
- * busy.  Each weighted node value lands in a shared array indexed by
- * (K, node), and one thread per K then sums its nodes in node order -- the
- * reference's own order -- so the result does not depend on scheduling.
+ * shared-memory work queue and are evaluated in batches with every lane busy,
+ * the two quadrature processes a (pair, node) a thread (quad_batch).  Each
+ * weighted node value lands in a shared array indexed by (K, node), and one
+ * warp per K then sums its nodes in a fixed order, so the result does not
+ * depend on scheduling.
+ *
+ * kpt and the CTA's width follow the number of energies: a table of 146
+ * energies has one energy a CTA and 512 threads on it (a 9-node photonuclear
+ * batch of 8 energies in 256 threads kept 19 of 152 SMs busy for 740 us); a
+ * fine grid has 8 energies a CTA of 128 threads, five or six CTAs an SM.
  */
-#include "dcs_fp64.cuh"
-#include "dcs_launch.h"
+#include "dcs_quad.cuh"
 
 #include <cuda_runtime.h>
 
 namespace noa_dcs {
 
-constexpr int I_THREADS = 256;
 constexpr int I_PAIRS = 1536;  // pairs per tile (kpt * nodes <= I_PAIRS)
-constexpr int I_QCAP = I_PAIRS + I_THREADS;
 constexpr int I_KMAX = 128;    // kinetic energies per tile at most
+
+constexpr int I_BATCH = 128;   // pairs per batch of the quadrature processes
+constexpr int I_NARROW = 128;  // CTA widths: many energies / at most one per SM
+constexpr int I_WIDE = 512;
 
 __constant__ double kGL6X[6] = {0.03376524, 0.16939531, 0.38069041, 0.61930959, 0.83060469, 0.96623476};
 __constant__ double kGL6W[6] = {0.08566225, 0.18038079, 0.23395697, 0.23395697, 0.18038079, 0.08566225};
@@ -46,18 +53,6 @@ struct IntegralParams {
 };
 
 template <int PROC>
-__device__ __forceinline__ double i_eval(double K, double q, const noa_dcs_consts &c) {
-    if (PROC == NOA_DCS_PROC_BREMS)
-        return brems_fp64(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PPROD)
-        return pprod_fp64(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PHOTO)
-        return photo_fp64(K, q, c);
-    else
-        return ion_fp64(K, q, c);
-}
-
-template <int PROC>
 __device__ __forceinline__ bool i_open(double K, double q, const noa_dcs_consts &c) {
     if (PROC == NOA_DCS_PROC_PPROD)
         return pprod_live(K, q, c);
@@ -65,6 +60,9 @@ __device__ __forceinline__ bool i_open(double K, double q, const noa_dcs_consts 
         return photo_live(K, q, c);
     else if (PROC == NOA_DCS_PROC_ION) {
         // ionisation's early returns, dcs.hh:415-424
+        const int first = ion_first_exit(K, q, c);
+        if (first >= 0)
+            return first && !bits_ge(c.io_Wmin, q);
         const double P2 = K * (K + 2. * c.mass);
         const double Wmax = ion_wmax(P2, K + c.mass, c);
         return !((Wmax < NOA_X_FRACTION * K) || (q > Wmax) || (q <= c.io_Wmin));
@@ -97,56 +95,42 @@ __device__ __forceinline__ double ion_analytic(double K, double xlow, int moment
     return x_mul(x_div(x_mul(1.535336E-05, c.Zd), c.A), term);
 }
 
-__device__ __forceinline__ int i_scan(int v, int *warp_tot, int *total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o)
-            x += y;
-    }
-    if (lane == 31)
-        warp_tot[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        const int w = lane < (I_THREADS >> 5) ? warp_tot[lane] : 0;
-        int s = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o)
-                s += y;
-        }
-        if (lane < (I_THREADS >> 5))
-            warp_tot[lane] = s - w;
-        if (lane == 31)
-            *total = s;
-    }
-    __syncthreads();
-    return warp_tot[warp] + x - v;
-}
-
-// Weighted value of node slot (f h w of numerics.hh:86, f = dcs q or dcs q^2).
-template <int PROC>
-__device__ __forceinline__ double i_node_value(double K, double q, double h, int node, int moment,
-                                               const noa_dcs_consts &c) {
-    const double d = i_eval<PROC>(K, q, c);
+// Weighted value of a node, f h w of numerics.hh:86, from its DCS d (f = d q
+// or d q^2).
+__device__ __forceinline__ double i_weighted(double d, double q, double h, int node, int moment) {
     const double f = moment == 0 ? x_mul(d, q) : x_mul(x_mul(d, q), q);
     return x_mul(x_mul(f, h), kGL6W[node % 6]);
 }
 
-template <int PROC>
-__global__ void __launch_bounds__(I_THREADS) recoil_integral_kernel(const IntegralParams p, const noa_dcs_consts c) {
-    __shared__ double vals[I_PAIRS];   // weighted node values of the tile, [k][node]
-    __shared__ double qQ[I_QCAP];      // queued recoil energies
-    __shared__ int qS[I_QCAP];         // their slots in vals
+// The sum of a kinetic energy's node values by one warp, in every lane: lane
+// sums of every 32nd node, then a butterfly -- one fixed order, whatever the
+// scheduling.  (One thread's node-ordered sum of 180 nodes was 180 dependent
+// additions, 6 us at the end of a tile.)
+__device__ __forceinline__ double warp_node_sum(const double *v, int nodes) {
+    double s = 0.;
+    for (int i = threadIdx.x & 31; i < nodes; i += 32)
+        s += v[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+template <int PROC, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == I_NARROW ? 5 : 1)
+    recoil_integral_kernel(const IntegralParams p, const noa_dcs_consts c) {
+    extern __shared__ double vals[];          // weighted node values of the tile, [k][node]
+    __shared__ double qQ[I_BATCH + THREADS];  // queued recoil energies
+    __shared__ int qS[I_BATCH + THREADS];     // their slots in vals
+    __shared__ QuadSmem<PROC, I_BATCH> quad;
     __shared__ double sK[I_KMAX], sLb[I_KMAX], sH[I_KMAX];
-    __shared__ int warp_tot[I_THREADS / 32];
+    __shared__ int warp_tot[THREADS / 32];
     __shared__ int tile_open;
     const int pairs = p.kpt * p.nodes;
     const int64_t tiles = (p.n + p.kpt - 1) / p.kpt;
     const double ion_thr = c.io_k_rad;  // 0.5 (m - me)^2 / me, dcs.hh:962-963
+    constexpr int batch = is_quad(PROC) ? I_BATCH : THREADS;
+    static_assert(batch <= I_BATCH + THREADS, "queue capacity");
 
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t k0 = tile * p.kpt;
@@ -161,7 +145,7 @@ __global__ void __launch_bounds__(I_THREADS) recoil_integral_kernel(const Integr
         }
         __syncthreads();
         int qn = 0;
-        for (int base = 0;; base += I_THREADS) {
+        for (int base = 0;; base += THREADS) {
             const bool more = base < pairs;  // block-uniform
             if (more) {
                 const int slot = base + threadIdx.x;
@@ -178,7 +162,7 @@ __global__ void __launch_bounds__(I_THREADS) recoil_integral_kernel(const Integr
                         open = i_open<PROC>(K, q, c);
                     }
                 }
-                const int pos = qn + i_scan(open ? 1 : 0, warp_tot, &tile_open);
+                const int pos = qn + block_scan<THREADS>(open ? 1 : 0, warp_tot, &tile_open);
                 if (open) {
                     qQ[pos] = q;
                     qS[pos] = slot;
@@ -188,12 +172,25 @@ __global__ void __launch_bounds__(I_THREADS) recoil_integral_kernel(const Integr
             }
             // one call site of the evaluation (a pair's rounding must not
             // depend on its queue position): full batches, then the rest
-            while (qn >= I_THREADS || (!more && qn > 0)) {
-                const int take = qn < I_THREADS ? qn : I_THREADS;
-                if ((int)threadIdx.x < take) {
-                    const int e = qn - take + threadIdx.x;
-                    const int sl = qS[e], kk = sl / p.nodes;
-                    vals[sl] = i_node_value<PROC>(sK[kk], qQ[e], sH[kk], sl - kk * p.nodes, p.moment, c);
+            while (qn >= batch || (!more && qn > 0)) {
+                const int take = qn < batch ? qn : batch;
+                const int first = qn - take;
+                if constexpr (is_quad(PROC)) {
+                    quad_batch<PROC, THREADS>(
+                        quad, take, c,
+                        [&](int e, double &K, double &q) {
+                            K = sK[qS[first + e] / p.nodes];
+                            q = qQ[first + e];
+                        },
+                        [&](int e, double d) {
+                            const int sl = qS[first + e], kk = sl / p.nodes;
+                            vals[sl] = i_weighted(d, qQ[first + e], sH[kk], sl - kk * p.nodes, p.moment);
+                        });
+                } else if ((int)threadIdx.x < take) {
+                    const int sl = qS[first + threadIdx.x], kk = sl / p.nodes;
+                    const double K = sK[kk], q = qQ[first + threadIdx.x];
+                    const double d = PROC == NOA_DCS_PROC_BREMS ? brems_fp64(K, q, c) : ion_fp64(K, q, c);
+                    vals[sl] = i_weighted(d, q, sH[kk], sl - kk * p.nodes, p.moment);
                 }
                 qn -= take;
                 __syncthreads();
@@ -201,22 +198,13 @@ __global__ void __launch_bounds__(I_THREADS) recoil_integral_kernel(const Integr
             if (!more)
                 break;
         }
-        // one thread per kinetic energy: node-ordered sum, as the reference
-        if ((int)threadIdx.x < p.kpt) {
-            const int64_t ki = k0 + threadIdx.x;
-            if (ki < p.n) {
-                const double K = sK[threadIdx.x];
-                double r;
-                if (PROC == NOA_DCS_PROC_ION && K <= ion_thr) {
-                    r = ion_analytic(K, p.xlow, p.moment, c);
-                } else {
-                    double s = 0.;
-                    const double *v = vals + threadIdx.x * p.nodes;
-                    for (int i = 0; i < p.nodes; i++)
-                        s = x_add(s, v[i]);
-                    r = x_div(s, K + c.mass);
-                }
-                p.out[ki] = r;
+        // one warp per kinetic energy
+        for (int kk = threadIdx.x >> 5; kk < p.kpt && k0 + kk < p.n; kk += THREADS / 32) {
+            const double s = warp_node_sum(vals + kk * p.nodes, p.nodes);
+            if ((threadIdx.x & 31) == 0) {
+                const double K = sK[kk];
+                p.out[k0 + kk] = (PROC == NOA_DCS_PROC_ION && K <= ion_thr) ? ion_analytic(K, p.xlow, p.moment, c)
+                                                                            : x_div(s, K + c.mass);
             }
         }
         __syncthreads();
@@ -234,9 +222,8 @@ __global__ void __launch_bounds__(I_THREADS) recoil_integral_kernel(const Integr
  * 0 * ratio * nu (0, or NaN where the weight is not finite, as in the
  * reference), open ones are evaluated 256 at a time.
  */
-constexpr int S_NODES = 102;            // 6 * ceil(100 / 6)
-constexpr int S_KPT = I_PAIRS / S_NODES; // 15 kinetic energies per tile
-constexpr int S_PAIRS = S_KPT * S_NODES;
+constexpr int S_NODES = 102;             // 6 * ceil(100 / 6)
+constexpr int S_KMAX = 8;                // kinetic energies per tile at most
 
 struct SoftParams {
     const double *K;
@@ -244,54 +231,29 @@ struct SoftParams {
     int64_t n;
     double lb;  // log(1e-6)
     double h;   // -lb / 17
+    int kpt;    // kinetic energies per tile
 };
 
-// dcs.hh:913-934 in the reference's operation order.
+// The mu-integrated angular weight of dcs.hh:913-934.  The poles (q^2 = m02)
+// are decided in IEEE arithmetic as in the reference; the rest is lean.
 __device__ __forceinline__ double soft_ratio(double K, double q, double mass) {
-    const double E = x_add(K, mass);
-    const double m02 = 0.4;
-    const double q2 = x_mul(q, q);
-    const double tmax = x_mul(1.876544, q);
-    const double tmin = x_div(x_mul(x_mul(q2, mass), mass), x_mul(E, x_sub(E, q)));
-    const double b1 = x_div(1., x_sub(1., x_div(q2, m02)));
-    const double c1 = x_div(1., x_sub(1., x_div(m02, q2)));
-    double L1 = x_mul(b1, log(x_div(x_add(q2, tmax), x_add(q2, tmin))));
-    double L2 = x_mul(c1, log(x_div(x_add(m02, tmax), x_add(m02, tmin))));
-    const double I0 = x_sub(x_sub(log(x_div(tmax, tmin)), L1), L2);
-    L1 = x_mul(L1, q2);
-    L2 = x_mul(L2, m02);
-    const double I1 = x_add(L1, L2);
-    L1 = x_mul(L1, q2);
-    L2 = x_mul(L2, m02);
-    const double I2 = x_sub(x_sub(x_mul(x_sub(tmax, tmin), x_add(x_mul(b1, q2), x_mul(c1, m02))), L1), L2);
-    return x_div(x_sub(x_mul(I1, tmax), I2),
-                 x_mul(x_mul(x_sub(x_mul(I0, tmax), I1), K), x_add(K, x_mul(2., mass))));
-}
-
-// The same weight with the lean functions, for closed photonuclear nodes:
-// there the reference adds 0 * ratio * nu, which is 0 (of either sign, which
-// the node sum cannot tell apart) unless the ratio is not finite.  Only its
-// finiteness is used.
-__device__ __forceinline__ bool soft_ratio_finite(double K, double q, double mass) {
     const double E = K + mass;
     const double m02 = 0.4;
     const double q2 = x_mul(q, q);
     const double tmax = 1.876544 * q;
-    const double tmin = q2 * mass * mass * d_rcp(E * (E - q));
-    // the weight's poles (q^2 = m02) are decided in IEEE arithmetic as in the reference
-    const double b1 = d_rcp(x_sub(1., x_div(q2, m02)));
-    const double c1 = d_rcp(x_sub(1., x_div(m02, q2)));
-    double L1 = b1 * d_log((q2 + tmax) * d_rcp(q2 + tmin));
-    double L2 = c1 * d_log((m02 + tmax) * d_rcp(m02 + tmin));
-    const double I0 = d_log(tmax * d_rcp(tmin)) - L1 - L2;
+    const double tmin = q2 * mass * mass * ol_rcp(E * (E - q));
+    const double b1 = ol_rcp(x_sub(1., x_div(q2, m02)));
+    const double c1 = ol_rcp(x_sub(1., x_div(m02, q2)));
+    double L1 = b1 * ol_log((q2 + tmax) * ol_rcp(q2 + tmin));
+    double L2 = c1 * ol_log((m02 + tmax) * ol_rcp(m02 + tmin));
+    const double I0 = ol_log(tmax * ol_rcp(tmin)) - L1 - L2;
     L1 *= q2;
     L2 *= m02;
     const double I1 = L1 + L2;
     L1 *= q2;
     L2 *= m02;
     const double I2 = (tmax - tmin) * (b1 * q2 + c1 * m02) - L1 - L2;
-    const double r = (I1 * tmax - I2) * d_rcp((I0 * tmax - I1) * K * (K + 2. * mass));
-    return isfinite(r);
+    return (I1 * tmax - I2) * ol_rcp((I0 * tmax - I1) * K * (K + 2. * mass));
 }
 
 // dcs.hh:874-899 in the reference's operation order.
@@ -321,32 +283,36 @@ __device__ __forceinline__ double soft_ionisation(double K, const noa_dcs_consts
 // Node i of the rule for kinetic energy K: nu and q (numerics.hh:84-86, dcs.hh:910-911).
 __device__ __forceinline__ void soft_node(double K, int i, const SoftParams &p, double &nu, double &q) {
     const double t = x_add(p.lb, x_mul(p.h, fpconv::f64i(i / 6) + kGL6X[i % 6]));
-    nu = x_mul(NOA_X_FRACTION, exp(t));
+    nu = x_mul(NOA_X_FRACTION, lean_exp(t));
     q = x_mul(nu, K);
 }
 
-__global__ void __launch_bounds__(I_THREADS) soft_scattering_kernel(const SoftParams p, const noa_dcs_consts c) {
-    __shared__ double vals[S_PAIRS];
-    __shared__ int qS[S_PAIRS + I_THREADS];
-    __shared__ double sK[S_KPT];
-    __shared__ int warp_tot[I_THREADS / 32];
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == I_NARROW ? 5 : 1)
+    soft_scattering_kernel(const SoftParams p, const noa_dcs_consts c) {
+    __shared__ double vals[S_KMAX * S_NODES];
+    __shared__ int qS[I_BATCH + THREADS];
+    __shared__ QuadSmem<NOA_DCS_PROC_PHOTO, I_BATCH> quad;
+    __shared__ double sK[S_KMAX];
+    __shared__ int warp_tot[THREADS / 32];
     __shared__ int tile_open;
-    const int64_t tiles = (p.n + S_KPT - 1) / S_KPT;
+    const int pairs = p.kpt * S_NODES;
+    const int64_t tiles = (p.n + p.kpt - 1) / p.kpt;
 
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int64_t k0 = tile * S_KPT;
-        if ((int)threadIdx.x < S_KPT) {
+        const int64_t k0 = tile * p.kpt;
+        if ((int)threadIdx.x < p.kpt) {
             const int64_t ki = k0 + threadIdx.x;
             sK[threadIdx.x] = ki < p.n ? p.K[ki] : 1.;
         }
         __syncthreads();
         int qn = 0;
-        for (int base = 0;; base += I_THREADS) {
-            const bool more = base < S_PAIRS;  // block-uniform
+        for (int base = 0;; base += THREADS) {
+            const bool more = base < pairs;  // block-uniform
             if (more) {
                 const int slot = base + threadIdx.x;
                 bool open = false;
-                if (slot < S_PAIRS) {
+                if (slot < pairs) {
                     const int kk = slot / S_NODES, i = slot - kk * S_NODES;
                     vals[slot] = 0.;
                     if (k0 + kk < p.n) {
@@ -354,28 +320,36 @@ __global__ void __launch_bounds__(I_THREADS) soft_scattering_kernel(const SoftPa
                         double nu, q;
                         soft_node(K, i, p, nu, q);
                         open = photo_live(K, q, c);
-                        if (!open && !soft_ratio_finite(K, q, c.mass))  // photonuclear = 0: 0 * ratio * nu
+                        // closed: the reference adds 0 * ratio * nu, which is 0 (of either sign, which
+                        // the node sum cannot tell apart) unless the ratio is not finite
+                        if (!open && !isfinite(soft_ratio(K, q, c.mass)))
                             vals[slot] = __longlong_as_double(0x7FF8000000000000LL);   // NaN, as 0 * inf
                     }
                 }
-                const int pos = qn + i_scan(open ? 1 : 0, warp_tot, &tile_open);
+                const int pos = qn + block_scan<THREADS>(open ? 1 : 0, warp_tot, &tile_open);
                 if (open)
                     qS[pos] = slot;
                 __syncthreads();
                 qn += tile_open;
             }
             // one call site of the evaluation, as in the recoil integrals
-            while (qn >= I_THREADS || (!more && qn > 0)) {
-                const int take = qn < I_THREADS ? qn : I_THREADS;
-                if ((int)threadIdx.x < take) {
-                    const int sl = qS[qn - take + threadIdx.x];
-                    const int kk = sl / S_NODES, i = sl - kk * S_NODES;
-                    const double K = sK[kk];
-                    double nu, q;
-                    soft_node(K, i, p, nu, q);
-                    const double f = x_mul(x_mul(photo_fp64(K, q, c), soft_ratio(K, q, c.mass)), nu);
-                    vals[sl] = x_mul(x_mul(f, p.h), kGL6W[i % 6]);
-                }
+            while (qn >= I_BATCH || (!more && qn > 0)) {
+                const int take = qn < I_BATCH ? qn : I_BATCH;
+                const int first = qn - take;
+                double nu = 0.;  // of this thread's own pair
+                quad_batch<NOA_DCS_PROC_PHOTO, THREADS>(
+                    quad, take, c,
+                    [&](int e, double &K, double &q) {
+                        const int sl = qS[first + e], kk = sl / S_NODES;
+                        K = sK[kk];
+                        soft_node(K, sl - kk * S_NODES, p, nu, q);
+                    },
+                    [&](int e, double d) {
+                        const int sl = qS[first + e], kk = sl / S_NODES;
+                        const double K = sK[kk];
+                        const double f = x_mul(x_mul(d, soft_ratio(K, x_mul(nu, K), c.mass)), nu);
+                        vals[sl] = x_mul(x_mul(f, p.h), kGL6W[(sl - kk * S_NODES) % 6]);
+                    });
                 qn -= take;
                 __syncthreads();
             }
@@ -383,15 +357,10 @@ __global__ void __launch_bounds__(I_THREADS) soft_scattering_kernel(const SoftPa
                 break;
         }
         __syncthreads();
-        if ((int)threadIdx.x < S_KPT) {
-            const int64_t ki = k0 + threadIdx.x;
-            if (ki < p.n) {
-                double s = 0.;
-                const double *v = vals + threadIdx.x * S_NODES;
-                for (int i = 0; i < S_NODES; i++)
-                    s = x_add(s, v[i]);
-                p.out[ki] = x_add(soft_ionisation(sK[threadIdx.x], c), x_mul(2., s));
-            }
+        for (int kk = threadIdx.x >> 5; kk < p.kpt && k0 + kk < p.n; kk += THREADS / 32) {
+            const double s = warp_node_sum(vals + kk * S_NODES, S_NODES);
+            if ((threadIdx.x & 31) == 0)
+                p.out[k0 + kk] = x_add(soft_ionisation(sK[kk], c), x_mul(2., s));
         }
         __syncthreads();
     }
@@ -408,6 +377,41 @@ static int sm_count() {
 
 using namespace noa_dcs;
 
+namespace {
+
+// Energies per tile: one while the call has fewer than 20 tiles an SM, then
+// up to `most`.
+int energies_per_tile(int64_t n, int64_t sms, int most) {
+    const int64_t k = n / (sms * 20);
+    return (int)(k < 1 ? 1 : (k > most ? most : k));
+}
+
+template <int THREADS>
+cudaError_t launch_recoil(int process, const IntegralParams &p, const noa_dcs_consts &c, cudaStream_t stream) {
+    const int64_t tiles = (p.n + p.kpt - 1) / p.kpt;
+    const int grid = (int)(tiles < (1 << 30) ? tiles : (1 << 30));
+    const size_t smem = sizeof(double) * (size_t)(p.kpt * p.nodes);
+    switch (process) {
+    case NOA_DCS_PROC_BREMS:
+        recoil_integral_kernel<NOA_DCS_PROC_BREMS, THREADS><<<grid, THREADS, smem, stream>>>(p, c);
+        break;
+    case NOA_DCS_PROC_PPROD:
+        recoil_integral_kernel<NOA_DCS_PROC_PPROD, THREADS><<<grid, THREADS, smem, stream>>>(p, c);
+        break;
+    case NOA_DCS_PROC_PHOTO:
+        recoil_integral_kernel<NOA_DCS_PROC_PHOTO, THREADS><<<grid, THREADS, smem, stream>>>(p, c);
+        break;
+    case NOA_DCS_PROC_ION:
+        recoil_integral_kernel<NOA_DCS_PROC_ION, THREADS><<<grid, THREADS, smem, stream>>>(p, c);
+        break;
+    default:
+        return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+} // namespace
+
 cudaError_t noa_dcs_launch_recoil_integral(int process, int moment, const double *K, double *out, int64_t n,
                                            double xlow, int min_points, const noa_dcs_consts *c,
                                            cudaStream_t stream) {
@@ -422,30 +426,12 @@ cudaError_t noa_dcs_launch_recoil_integral(int process, int moment, const double
     p.nodes = 6 * p.n_itv;
     if (p.nodes > I_PAIRS || p.nodes < 6)
         return cudaErrorInvalidValue;
-    p.kpt = I_PAIRS / p.nodes;
-    if (p.kpt > I_KMAX)
-        p.kpt = I_KMAX;
+    const int64_t sms = sm_count();
+    const int most = p.nodes >= I_PAIRS / 2 ? 1 : I_PAIRS / 2 / p.nodes;
+    p.kpt = energies_per_tile(n, sms, most < I_KMAX ? most : I_KMAX);
     p.moment = moment;
-    const int64_t tiles = (n + p.kpt - 1) / p.kpt;
-    const int64_t cap = (int64_t)sm_count() * 3;
-    const int grid = (int)(tiles < cap ? tiles : cap);
-    switch (process) {
-    case NOA_DCS_PROC_BREMS:
-        recoil_integral_kernel<NOA_DCS_PROC_BREMS><<<grid, I_THREADS, 0, stream>>>(p, *c);
-        break;
-    case NOA_DCS_PROC_PPROD:
-        recoil_integral_kernel<NOA_DCS_PROC_PPROD><<<grid, I_THREADS, 0, stream>>>(p, *c);
-        break;
-    case NOA_DCS_PROC_PHOTO:
-        recoil_integral_kernel<NOA_DCS_PROC_PHOTO><<<grid, I_THREADS, 0, stream>>>(p, *c);
-        break;
-    case NOA_DCS_PROC_ION:
-        recoil_integral_kernel<NOA_DCS_PROC_ION><<<grid, I_THREADS, 0, stream>>>(p, *c);
-        break;
-    default:
-        return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+    return n <= sms ? launch_recoil<I_WIDE>(process, p, *c, stream)
+                    : launch_recoil<I_NARROW>(process, p, *c, stream);
 }
 
 cudaError_t noa_dcs_launch_soft_scattering(const double *K, double *out, int64_t n, const noa_dcs_consts *c,
@@ -458,9 +444,13 @@ cudaError_t noa_dcs_launch_soft_scattering(const double *K, double *out, int64_t
     p.n = n;
     p.lb = log(1E-06);                // dcs.hh:905
     p.h = (0. - p.lb) / (double)17u;  // numerics.hh:80-81, n_itv = ceil(100 / 6)
-    const int64_t tiles = (n + S_KPT - 1) / S_KPT;
-    const int64_t cap = (int64_t)sm_count() * 3;
-    const int grid = (int)(tiles < cap ? tiles : cap);
-    soft_scattering_kernel<<<grid, I_THREADS, 0, stream>>>(p, *c);
+    const int64_t sms = sm_count();
+    p.kpt = energies_per_tile(n, sms, S_KMAX);
+    const int64_t tiles = (n + p.kpt - 1) / p.kpt;
+    const int grid = (int)(tiles < (1 << 30) ? tiles : (1 << 30));
+    if (n <= sms)
+        soft_scattering_kernel<I_WIDE><<<grid, I_WIDE, 0, stream>>>(p, *c);
+    else
+        soft_scattering_kernel<I_NARROW><<<grid, I_NARROW, 0, stream>>>(p, *c);
     return cudaGetLastError();
 }
