@@ -13,11 +13,14 @@ import mpmath
 
 mpmath.mp.dps = 60
 
-LOG_BITS = 8        # 256 bins over the top 8 mantissa bits
-LOG_SPLIT = 106     # bins t >= 106 (m >= 1 + 106/256 > sqrt 2) are halved: m in [0.707, 1)
-C_BITS = 10         # c_t = C_t / 2^10: m * c_t is exact in 64-bit integers
+LOG_BITS = 9        # 512 bins over the top 9 mantissa bits
+LOG_SPLIT = 212     # bins t >= 212 (m >= 1 + 212/512 > sqrt 2) are halved: m in [0.707, 1)
+C_BITS = 11         # c_t = C_t / 2^11
 EXP_N = 128         # 2^(j/128)
-MAGIC = 0x4B400000  # bits of 1.5 2^23: a float there carries a 22-bit signed integer in its low bits
+# a float near these carries an integer in its low bits: 1.5 2^23 one of
+# +-2^22, 2^24 - 1 one of -2^23 .. 0
+MAGIC = 0x4B400000
+MAGIC_NEG = 0x4B7FFFFF
 
 
 def f32(x):
@@ -31,13 +34,13 @@ def ff(x):
 
 
 def log_tables():
-    """Per bin t: (c_t 2^11 / 2^h, L_t).
+    """Per bin t: (c_t 2^12 / 2^h, L_t).
 
-    c_t = C_t / 2^10 is 1 / (bin centre) rounded to 10 fractional bits and
-    m = M 2^-(52+h), so that r = m c_t - 1 is an exact 64-bit integer multiple
-    of 2^-63; |r| < 2^-8.7.  L_t is -log(c_t) in units of 2^-63, less the
-    offsets MAGIC 2^23 + MAGIC 2 that the two integer parts of the sum carry,
-    modulo 2^64.
+    c_t = C_t / 2^11 is 1 / (bin centre) rounded to 11 fractional bits and
+    m = M 2^-(52+h), so that r = m c_t - 1 is an exact multiple of 2^-64: the
+    product of the two integers modulo 2^64; |r| < 2^-9.5.  L_t is -log(c_t)
+    in units of 2^-64, less the offsets MAGIC_NEG 2^22 and MAGIC that the two
+    integer parts of the sum carry, modulo 2^64.
     """
     rows = []
     one = 1 << C_BITS
@@ -46,10 +49,10 @@ def log_tables():
         lo = (1 + mpmath.mpf(t) / (1 << LOG_BITS)) / 2 ** h
         hi = (1 + mpmath.mpf(t + 1) / (1 << LOG_BITS)) / 2 ** h
         C = int(mpmath.nint(one / ((lo + hi) / 2)))
-        for m in (lo, hi):  # |r| stays below 2^-8.7 over the bin
-            assert abs(m * C / one - 1) < mpmath.mpf(2) ** -8.7
-        L = int(mpmath.nint(-mpmath.log(mpmath.mpf(C) / one) * mpmath.mpf(2) ** 63))
-        L = (L - (MAGIC << 23) - (MAGIC << 1)) % (1 << 64)
+        for m in (lo, hi):  # |r| stays below 2^-9.5 over the bin
+            assert abs(m * C / one - 1) < mpmath.mpf(2) ** -9.5
+        L = int(mpmath.nint(-mpmath.log(mpmath.mpf(C) / one) * mpmath.mpf(2) ** 64))
+        L = (L - (MAGIC_NEG << 22) - MAGIC) % (1 << 64)
         rows.append((C << (1 - h), L - (1 << 64) if L >> 63 else L))
     return rows
 
@@ -69,7 +72,7 @@ def signed_words(v, n):
 def main():
     rows = log_tables()
     ln2 = mpmath.log(2)
-    ln2_l, ln2_h = signed_words(int(mpmath.nint(ln2 * mpmath.mpf(2) ** 63)), 2)
+    ln2_l, ln2_h = signed_words(int(mpmath.nint(ln2 * mpmath.mpf(2) ** 63)), 2)  # LN2_L doubles in units of 2^-64
     k_l, k_m, k_h = signed_words(int(mpmath.nint(ln2 / EXP_N * mpmath.mpf(2) ** 95)), 3)
     T = [int(mpmath.nint(mpmath.power(2, mpmath.mpf(j) / EXP_N) * mpmath.mpf(2) ** 61)) for j in range(EXP_N)]
     third_h, third_l = ff(mpmath.mpf(1) / 3)
@@ -93,9 +96,9 @@ def main():
     out.append(f"#define LEAN64_SIXTH_H {sixth_h!r}f")
     out.append(f"#define LEAN64_SIXTH_L {sixth_l!r}f")
     out.append("/* Per bin t, one 16-byte entry {c_t, L_t}: the reciprocal c_t of the bin")
-    out.append("   centre in units of 2^-11 (2^-10 for the halved bins t >= LOG_SPLIT; 10")
-    out.append("   fractional bits) and -log(c_t) in units of 2^-63, less the offsets of the")
-    out.append("   two float-carried integers that are added to it (MAGIC 2^23 + MAGIC 2). */")
+    out.append("   centre in units of 2^-12 (2^-11 for the halved bins t >= LOG_SPLIT; 11")
+    out.append("   fractional bits) and -log(c_t) in units of 2^-64, less the offsets of the")
+    out.append("   two float-carried integers that are added to it (MAGIC_NEG 2^22 + MAGIC). */")
     out.append("#define LEAN64_LOG_TAB_DATA {\\")
     out.append(",\\\n".join("    {%dLL, %dLL}" % r for r in rows) + "}")
     out.append("static __device__ const longlong2 lean64_log_tab[%d] = LEAN64_LOG_TAB_DATA;" % len(rows))

@@ -21,11 +21,11 @@
  * twice the ALU instructions), 35.3 ms as they are:
  *
  *   lean_log   0 FP64 ops.  Tang's table method (P. T. P. Tang, ACM TOMS
- *              16(4), 1990): x = 2^e m, c_t ~ 1/m with 10 fractional bits from
- *              the top 8 mantissa bits; r = m c_t - 1 exact in 64-bit integers;
+ *              16(4), 1990): x = 2^e m, c_t ~ 1/m with 11 fractional bits from
+ *              the top 9 mantissa bits; r = m c_t - 1 exact in 64-bit integers;
  *              log x = e ln2 - log c_t + r + (log1p(r) - r), summed in 64-bit
  *              fixed point at a scale that follows |e| and rounded once.
- *              Within 2^-8 of 1 c = 1 and the scale follows r: full
+ *              Within 2^-9 of 1 c = 1 and the scale follows r: full
  *              relative accuracy near 1.
  *   lean_exp   0 FP64 ops.  Tang's table method (ACM TOMS 15(2), 1989): x as a
  *              64-bit fixed-point number, k = round(x 128 / ln2),
@@ -156,22 +156,25 @@ LEAN64_FN double fix_to_double(long long S, int F) {
 }
 
 // Z 2^-F as a double, rounded half up in the last place, for |Z| >= 2^32: the
-// leading bit is then in the high word (one 32-bit count).
+// leading bit is then in the high word (one 32-bit count).  Z is a value cut
+// downwards; the one's complement of a negative Z is its magnitude cut
+// downwards, so that the last rounding is that of the uncut value.
 LEAN64_FN double fix_wide_to_double(long long Z, int F) {
-    const unsigned long long U = Z < 0 ? 0ull - (unsigned long long)Z : (unsigned long long)Z;
+    const unsigned long long U = (unsigned long long)(Z ^ (Z >> 63));
     const int lz = clz32((unsigned)(U >> 32)) - 1;  // the caller keeps |Z| < 2^63
     const unsigned long long m = ((U << lz) + 0x200ull) >> 10;  // leading bit at 52
     return ll2d((long long)((((unsigned long long)(1084 - lz - F) << 52) + m) |
                             ((unsigned long long)Z & 0x8000000000000000ull)));
 }
 
-// The pair dh + dl as an integer in units of 2^-(S + 22), in two parts of 22
-// bits that float adds round: i1 = round(d 2^S), i2 = round((d 2^S - i1) 2^22).
-// Returns their float carriers (bits MAGIC + i; MAGIC = 0x4B400000), whose
-// offsets the caller's constants take off.  Requires |d| 2^S < 2^22.
-LEAN64_FN void fix_parts(float dh, float dl, float scale, unsigned &b1, unsigned &b2) {
-    const float t1 = fmaf(fadd(dh, dl), scale, 12582912.f);
-    const float g = fmaf(dl, scale, fmaf(dh, scale, -fadd(t1, -12582912.f)));
+// The pair dh + dl as an integer in units of 2^-(S + 22), in two parts that
+// float adds round: i1 = round(d 2^S), i2 = round((d 2^S - i1) 2^22).  Returns
+// their float carriers, whose offsets the caller's constants take off:
+// `magic` (1.5 2^23 for |d| 2^S < 2^22, 2^24 - 1 for -2^23 < d 2^S <= 0) and
+// 1.5 2^23.
+LEAN64_FN void fix_parts(float dh, float dl, float scale, float magic, unsigned &b1, unsigned &b2) {
+    const float t1 = fmaf(fadd(dh, dl), scale, magic);
+    const float g = fmaf(dl, scale, fmaf(dh, scale, -fadd(t1, -magic)));
     b1 = f2u(t1);
     b2 = f2u(fmaf(g, 4194304.f, 12582912.f));
 }
@@ -179,14 +182,14 @@ LEAN64_FN void fix_parts(float dh, float dl, float scale, unsigned &b1, unsigned
 } // namespace detail
 
 // log x with no FP64 instruction.  x = 2^e m, m in [0.707, 1.414) (bin t of
-// the top 8 mantissa bits, halved above sqrt 2), c_t ~ 1/m:
-//   r = m c - 1 = R 2^-63          exact, one 64-bit integer multiply
+// the top 9 mantissa bits, halved above sqrt 2), c_t ~ 1/m:
+//   r = m c - 1 = R 2^-64          exact: one integer product modulo 2^64
 //   d = log1p(r) - r               float-float, ~2^-47 relative; r enters as
 //                                  rh + rl, the two words of R
-//   log x = e ln2 - log c + r + d  64-bit fixed point: 2^-63 for e = 0, 2^-58
-//                                  for |e| <= 15, 2^-51 beyond (|log x| >= 0.34,
-//                                  0.34 and 10.7: at least 2^-57 relative)
-// rounded once to double.  Within 2^-8 of 1 (e = 0) c = 1 and the scale
+//   log x = e ln2 - log c + r + d  64-bit fixed point: 2^-64 for e = 0, 2^-58
+//                                  for |e| <= 15, 2^-51 beyond (|log x| >= 2^-9,
+//                                  0.34 and 10.7: a few units of 2^-55 relative)
+// rounded once to double.  In [1 - 2^-9, 1 + 2^-9) c = 1 and the scale
 // follows r (log x = r + d), so log x keeps full relative accuracy at
 // x = 1 +- 2^-53.
 LEAN64_FN double lean_log(double x) {
@@ -196,18 +199,19 @@ LEAN64_FN double lean_log(double x) {
     // positive, normal and finite?
     if (hi - 0x00100000u >= 0x7FE00000u)
         return log(x);
-    const int e = (int)(hi + ((256u - LEAN64_LOG_SPLIT) << 12) - 0x3FF00000u) >> 20;  // bins above the split carry
-    const bool near1 = hi - 0x3FEFF000u < 0x2000u;
-    const longlong2 ent = log_entry((hi >> 12) & 0xFFu);  // {c_t, L_t}, one 16-byte load
-    const unsigned C = near1 ? (hi < 0x3FF00000u ? 1024u : 2048u) : (unsigned)ent.x;
+    const int e = (int)(hi + ((512u - LEAN64_LOG_SPLIT) << 11) - 0x3FF00000u) >> 20;  // bins above the split carry
+    const bool near1 = hi - 0x3FEFF000u < 0x1800u;
+    const longlong2 ent = log_entry((hi >> 11) & 0x1FFu);  // {c_t, L_t}, one 16-byte load
+    const unsigned C = near1 ? (hi < 0x3FF00000u ? 2048u : 4096u) : (unsigned)ent.x;
     const unsigned long long M = ((unsigned long long)((hi & 0x000FFFFFu) | 0x00100000u) << 32) | (unsigned)b;
-    const long long R = (long long)(M * C + 0x8000000000000000ull);
+    const long long R = (long long)(M * C);
     // r = rh + rl: the high word rounded and the signed low word, renormalised
-    const float rw = fmul(i2f((int)((R + 0x80000000ll) >> 32)), 0x1p-31f);
-    const float rv = fmul(i2f((int)(unsigned)R), 0x1p-63f);
+    const float rw = fmul(i2f((int)((R + 0x80000000ll) >> 32)), 0x1p-32f);
+    const float rv = fmul(i2f((int)(unsigned)R), 0x1p-64f);
     const float rh = fadd(rw, rv);
     const float rl = fadd(rv, -fadd(rh, -rw));
-    // d = -r^2/2 + r^3 w,  w = 1/3 - r/4 + r^2 (1/5 - r/6 + r^2/7)
+    // d = -r^2/2 + r^3 w,  w = 1/3 - r/4 + r^2 (1/5 - r/6 + r^2/7); the last
+    // term is below 2^-63 but in the window around 1
     const float sh = fmul(rh, rh);
     const float sl = fmaf(fmul(2.f, rh), rl, fmaf(rh, rh, -sh));
     const float zt = fmul(sh, fmaf(rh, fmaf(rh, 1.f / 7.f, -1.f / 6.f), 0.2f));
@@ -227,19 +231,18 @@ LEAN64_FN double lean_log(double x) {
         if (R == 0)
             return 0.0;
         const unsigned long long A = R < 0 ? 0ull - (unsigned long long)R : (unsigned long long)R;
-        const int lz = clz64(A);  // |r| < 2^-8: lz >= 8
-        const int F = 61 + lz;
+        const int lz = clz64(A);  // |r| < 2^-9: lz >= 9
+        const int F = 62 + lz;
         const long long Sr = (long long)(A << (lz - 2));
         return fix_to_double((R < 0 ? -Sr : Sr) + fix_from_float(dh, F) + fix_from_float(dl, F), F);
     }
     unsigned b1, b2;
-    fix_parts(dh, dl, 0x1p40f, b1, b2);
-    const long long T = R + (long long)((unsigned long long)ent.y + (unsigned long long)b1 * 0x800000ull +
-                                        (unsigned long long)b2 * 2ull);
-    const int s = e == 0 ? 0 : ((unsigned)(e + 15) <= 30u ? 5 : 12);
-    const long long Q = T + (long long)e * LEAN64_LN2_L;
-    const long long Z = (long long)(int)((unsigned)e << ((32 - s) & 31)) * LEAN64_LN2_H + (Q >> s);
-    return fix_wide_to_double(Z, 63 - s);
+    fix_parts(dh, dl, 0x1p42f, 16777215.f, b1, b2);  // -2^-19.9 < d <= 0
+    const long long T = R + (long long)((unsigned long long)ent.y + (unsigned long long)b1 * 0x400000ull + b2);
+    const int s = e == 0 ? 0 : ((unsigned)(e + 15) <= 30u ? 6 : 13);
+    const long long Q = T + (long long)e * (2ll * LEAN64_LN2_L);
+    const long long Z = (long long)(int)((unsigned)e << ((33 - s) & 31)) * LEAN64_LN2_H + (Q >> s);
+    return fix_wide_to_double(Z, 64 - s);
 }
 
 // exp x with no FP64 instruction.  k = round(x 128 / ln2) from a float,
@@ -282,7 +285,7 @@ LEAN64_FN double lean_exp(double x) {
     const float dl = fmaf(sh, ql, fmaf(sl, qh, fmaf(sh, qh, -dh)));
     // p = r + d in units of 2^-63
     unsigned b1, b2;
-    fix_parts(dh, dl, 0x1p39f, b1, b2);
+    fix_parts(dh, dl, 0x1p39f, 12582912.f, b1, b2);
     const long long p = (long long)((unsigned long long)r - (0x4B400000ull << 24) - (0x4B400000ull << 2) +
                                     (unsigned long long)b1 * 0x1000000ull + (unsigned long long)b2 * 4ull);
     // T (1 + p) in units of 2^-61: T = Th 2^31 + Tl, p = ph 2^32 + pl; the
