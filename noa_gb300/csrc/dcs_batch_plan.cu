@@ -62,9 +62,8 @@ bool counts_fit(const int64_t *counts, int n_segments) {
 }
 
 size_t smem_bytes(const noa_dcs_batch_plan *p, int threads, int items) {
-    const bool third = noa_dcs::batch_third_queue(p->process, p->precision);
-    return threads == 128 ? noa_dcs::BatchSmem<128>::bytes(items, third)
-                          : noa_dcs::BatchSmem<256>::bytes(items, third);
+    return threads == 128 ? noa_dcs::BatchSmem<128>::bytes(items, p->process, p->precision)
+                          : noa_dcs::BatchSmem<256>::bytes(items, p->process, p->precision);
 }
 
 int occupancy(const noa_dcs_batch_plan *p, int threads, int items) {
@@ -73,15 +72,37 @@ int occupancy(const noa_dcs_batch_plan *p, int threads, int items) {
                                         : noa_dcs_batched_occupancy32(p->process, threads, smem);
 }
 
-// Fills the tile prefix sums for the current tile shape.
-void set_tiles(noa_dcs_batch_plan *p) {
-    const int64_t tile = (int64_t)p->items * p->threads;
-    p->params.items = p->items;
-    p->params.tile_begin[0] = 0;
+// Fills the tile prefix sums for the current tile shape; the first
+// sample_per_segment pairs of each segment only, if > 0.  The tile spreads
+// the pairs over all CTAs in equal steps, with room for a partial tile per
+// segment (a few tiles more than CTAs cost a whole further step), at most the
+// shape's items x threads pairs, down to a warp: a short call left most CTAs
+// without work at the full tile (1000 pairs of ten elements: 10 CTAs).  With
+// more steps the full tile and the counter balance as well: at 1e6 pairs (4
+// steps) equal tiles still gain in FP64 (pair production 555 us against 624)
+// and lose in FP32C, whose tiles are short beside the counter's round trip
+// (photonuclear 72 us against 64).
+void set_tiles(noa_dcs_batch_plan *p, int64_t sample_per_segment = 0) {
+    const int64_t *begin = p->params.seg_begin;
+    int64_t count[NOA_DCS_MAX_SEGMENTS], total = 0;
     for (int s = 0; s < p->params.n_seg; s++) {
-        const int64_t cnt = p->params.seg_begin[s + 1] - p->params.seg_begin[s];
-        p->params.tile_begin[s + 1] = p->params.tile_begin[s] + (cnt + tile - 1) / tile;
+        count[s] = begin[s + 1] - begin[s];
+        if (sample_per_segment > 0 && count[s] > sample_per_segment)
+            count[s] = sample_per_segment;
+        total += count[s];
     }
+    const int64_t most = (int64_t)p->items * p->threads;
+    const int64_t ctas = (int64_t)p->sms * p->ctas_per_sm;
+    const int64_t steps = (total + p->params.n_seg * most + ctas * most - 1) / (ctas * most);
+    const int64_t whole = ctas * steps - p->params.n_seg;  // tiles beside the segments' partial ones
+    const int64_t equal_steps = p->precision == NOA_DCS_FP64 ? 8 : 2;
+    int64_t tile = whole > 0 && steps <= equal_steps ? (total + whole - 1) / whole : most;
+    tile = tile < 32 ? 32 : (tile > most ? most : tile);
+    p->params.items = p->items;
+    p->params.tile = (int)tile;
+    p->params.tile_begin[0] = 0;
+    for (int s = 0; s < p->params.n_seg; s++)
+        p->params.tile_begin[s + 1] = p->params.tile_begin[s] + (count[s] + tile - 1) / tile;
 }
 
 int launch(noa_dcs_batch_plan *p, double *out, const double *K, const double *q, cudaStream_t s) {
@@ -316,16 +337,7 @@ int noa_dcs_batch_plan_autotune(noa_dcs_batch_plan *p, double *result, const dou
                 t.threads = thread_opts[ti];
                 t.items = item_opts[ii];
                 t.ctas_per_sm = cta_opts[ci];
-                // tiles per segment of the sample, laid out on the full buffers
-                const int64_t tile = (int64_t)t.items * t.threads;
-                t.params.items = t.items;
-                t.params.tile_begin[0] = 0;
-                for (int s = 0; s < t.params.n_seg; s++) {
-                    int64_t cnt = p->params.seg_begin[s + 1] - p->params.seg_begin[s];
-                    if (sample_per_segment > 0 && cnt > sample_per_segment)
-                        cnt = sample_per_segment;
-                    t.params.tile_begin[s + 1] = t.params.tile_begin[s] + (cnt + tile - 1) / tile;
-                }
+                set_tiles(&t, sample_per_segment);  // laid out on the full buffers
                 float ms_sum = 0.f;
                 bool ok = true;
                 for (int rep = 0; rep < 3 && ok; rep++) {

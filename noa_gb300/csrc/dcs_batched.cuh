@@ -3,7 +3,8 @@
  * process for up to NOA_DCS_MAX_SEGMENTS elements, each with its own
  * (uneven) number of pairs, stored back to back in K, q and result.
  *
- *  - Work unit: a tile of THREADS x items consecutive pairs of one segment.
+ *  - Work unit: a tile of at most THREADS x items consecutive pairs of one
+ *    segment (fewer where the call would not give every CTA a few tiles).
  *    Tiles of all segments form one index space (prefix sums in the
  *    parameters); each CTA takes the next tile from a global counter
  *    (atomicAdd), so CTAs balance across the uneven segments without a
@@ -11,10 +12,11 @@
  *    zeroed by a memset node before each launch.
  *  - Inside a CTA the tile goes through the same compaction as the
  *    single-element kernels: open pairs are appended to a shared-memory work
- *    queue that is popped 256 (THREADS) at a time; for FP32C, pairs whose error
- *    estimate exceeds the tolerance go to a redo queue evaluated in FP64
- *    (pair production: evaluated again with its screening log in float-float
- *    arithmetic, and only what that still rejects in FP64).
+ *    queue that is popped THREADS at a time (FP64 pair production and
+ *    photonuclear: evaluated by the whole CTA, quad_batch); for FP32C, pairs
+ *    whose error estimate exceeds the tolerance go to a redo queue evaluated
+ *    in FP64 (pair production: evaluated again with its screening log in
+ *    float-float arithmetic, and only what that still rejects in FP64).
  *    When the next tile belongs to another segment the queues are drained
  *    first, so every warp evaluates pairs of a single element and the element
  *    constants stay warp-uniform (they are read from the parameter space).
@@ -26,8 +28,7 @@
 #pragma once
 
 #include "dcs_fp32c.cuh"
-#include "dcs_fp64.cuh"
-#include "dcs_launch.h"
+#include "dcs_quad.cuh"
 
 #include <atomic>
 
@@ -41,7 +42,7 @@ struct BatchParams {
     int n_seg;
     int items;
     float tol;
-    int pad_;
+    int tile;  // pairs per tile, at most items x THREADS
     int64_t seg_begin[NOA_DCS_MAX_SEGMENTS + 1];
     int64_t tile_begin[NOA_DCS_MAX_SEGMENTS + 1];
     noa_dcs_consts consts[NOA_DCS_MAX_SEGMENTS];
@@ -57,26 +58,10 @@ __device__ __forceinline__ bool batch_open(double K, double q, const noa_dcs_con
         return true;
 }
 
+// FP64 of the two processes without a quadrature.
 template <int PROC>
 __device__ __forceinline__ double batch_eval64(double K, double q, const noa_dcs_consts &c) {
-    if (PROC == NOA_DCS_PROC_BREMS)
-        return brems_fp64(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PPROD)
-        return pprod_fp64(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PHOTO)
-        return photo_fp64(K, q, c);
-    else
-        return ion_fp64(K, q, c);
-}
-
-// The FP32C engine's FP64 redo: out of line for the two quadrature processes.
-template <int PROC>
-__device__ __forceinline__ double batch_redo64(double K, double q, const noa_dcs_consts &c) {
-    if (PROC == NOA_DCS_PROC_PPROD)
-        return pprod_fp64_ol(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PHOTO)
-        return photo_fp64_ol(K, q, c);
-    return batch_eval64<PROC>(K, q, c);
+    return PROC == NOA_DCS_PROC_BREMS ? brems_fp64(K, q, c) : ion_fp64(K, q, c);
 }
 
 template <int PROC>
@@ -91,52 +76,34 @@ __device__ __forceinline__ double batch_eval32(double K, double q, const noa_dcs
         return ion_fp32c(K, q, c, est);
 }
 
-template <int THREADS>
-__device__ __forceinline__ int batch_scan(int v, int *warp_tot, int *total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o)
-            x += y;
-    }
-    if (lane == 31)
-        warp_tot[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        const int w = lane < (THREADS >> 5) ? warp_tot[lane] : 0;
-        int s = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o)
-                s += y;
-        }
-        if (lane < (THREADS >> 5))
-            warp_tot[lane] = s - w;
-        if (lane == 31)
-            *total = s;
-    }
-    __syncthreads();
-    return warp_tot[warp] + x - v;
-}
-
-// Shared memory of one CTA: work queue of capacity items*THREADS + THREADS,
-// then the redo queue (2*THREADS), then for FP32C pair production the third
-// queue (2*THREADS) of the pairs its float-float redo step still rejects, as
-// dynamic shared memory.
-template <int THREADS>
-struct BatchSmem {
-    static __host__ __device__ size_t bytes(int items, bool third) {
-        return (size_t)(items * THREADS + THREADS) * 24 + (size_t)(2 * THREADS) * 24 +
-               (third ? (size_t)(2 * THREADS) * 24 : 0);
-    }
-};
-
 __host__ __device__ constexpr bool batch_third_queue(int proc, int prec) {
     return proc == NOA_DCS_PROC_PPROD && prec != NOA_DCS_FP64;
 }
+
+// Dynamic shared memory of one CTA: the work queue (items*THREADS + THREADS
+// pairs); for FP32C the redo queue (2*THREADS), and for its pair production
+// the third queue (2*THREADS) of the pairs its float-float redo step still
+// rejects; for the quadrature processes the batch of quad_batch (FP64) or
+// quad_redo (FP32C).
+template <int THREADS>
+struct BatchSmem {
+    static constexpr size_t pair_bytes = 2 * sizeof(double) + sizeof(int64_t);
+    static __host__ __device__ constexpr size_t queues(int items, int proc, int prec) {
+        return pair_bytes * THREADS *
+               (items + 1 + (prec != NOA_DCS_FP64 ? 2 : 0) + (batch_third_queue(proc, prec) ? 2 : 0));
+    }
+    static __host__ __device__ constexpr size_t bytes(int items, int proc, int prec) {
+        return queues(items, proc, prec) +
+               (proc == NOA_DCS_PROC_PPROD
+                    ? (prec == NOA_DCS_FP64 ? sizeof(QuadSmem<NOA_DCS_PROC_PPROD, THREADS>)
+                                            : sizeof(QuadSmem<NOA_DCS_PROC_PPROD, QUAD_REDO>))
+                    : 0) +
+               (proc == NOA_DCS_PROC_PHOTO
+                    ? (prec == NOA_DCS_FP64 ? sizeof(QuadSmem<NOA_DCS_PROC_PHOTO, THREADS>)
+                                            : sizeof(QuadSmem<NOA_DCS_PROC_PHOTO, QUAD_REDO>))
+                    : 0);
+    }
+};
 
 // Appends (k, q, i) of the lanes with `push` to a queue (warp-aggregated).
 __device__ __forceinline__ void batch_push(bool push, double k, double q, int64_t i, double *QK, double *QQ,
@@ -179,17 +146,12 @@ __device__ __forceinline__ void batch_fine_step(double *rK, double *rQ, int64_t 
     batch_push(redo, k, q, i, xK, xQ, xI, xn);
 }
 
-// One evaluation step over work-queue entry e: FP64 writes directly; FP32C
-// writes or appends to the redo queue.
-template <int PROC, int PREC>
-__device__ __forceinline__ void batch_step(double *wK, double *wQ, int64_t *wI, double *rK, double *rQ,
-                                           int64_t *rI, int *rn, int e, bool valid, double *out,
-                                           const noa_dcs_consts &c, float tol) {
-    if (PREC == NOA_DCS_FP64) {
-        if (valid)
-            out[wI[e]] = batch_eval64<PROC>(wK[e], wQ[e], c);
-        return;
-    }
+// FP32C: evaluates work-queue entry e (if valid) and writes it or appends it
+// to the redo queue.
+template <int PROC>
+__device__ __forceinline__ void batch_step32(double *wK, double *wQ, int64_t *wI, double *rK, double *rQ,
+                                             int64_t *rI, int *rn, int e, bool valid, double *out,
+                                             const noa_dcs_consts &c, float tol) {
     bool redo = false;
     double k = 0., q = 0.;
     int64_t i = 0;
@@ -221,12 +183,14 @@ __global__ void __launch_bounds__(THREADS) dcs_batched_kernel(const __grid_const
     double *xQ = xK + 2 * THREADS;
     int64_t *xI = reinterpret_cast<int64_t *>(xQ + 2 * THREADS);
     constexpr bool third = batch_third_queue(PROC, PREC);
+    typedef QuadSmem<PROC, PREC == NOA_DCS_FP64 ? THREADS : QUAD_REDO> Quads;
+    Quads &quad = *reinterpret_cast<Quads *>(smem_raw + BatchSmem<THREADS>::queues(items, PROC, PREC));
     __shared__ int warp_tot[THREADS / 32];
     __shared__ int tile_open;
     __shared__ int rn, xn;
     __shared__ unsigned long long s_tile;
 
-    const int tile_size = items * THREADS;
+    const int tile_size = p.tile;
     const long long total_tiles = p.tile_begin[p.n_seg];
     if (threadIdx.x == 0) {
         rn = 0;
@@ -260,22 +224,41 @@ __global__ void __launch_bounds__(THREADS) dcs_batched_kernel(const __grid_const
                 bool did = false;
                 if (qn >= THREADS || (flush && qn > 0)) {
                     const int take = qn < THREADS ? qn : THREADS;
-                    batch_step<PROC, PREC>(wK, wQ, wI, rK, rQ, rI, &rn, qn - take + threadIdx.x,
+                    const int first = qn - take;
+                    if constexpr (PREC != NOA_DCS_FP64) {
+                        batch_step32<PROC>(wK, wQ, wI, rK, rQ, rI, &rn, first + threadIdx.x,
                                            (int)threadIdx.x < take, p.out, cc, p.tol);
+                    } else if constexpr (is_quad(PROC)) {
+                        quad_batch<PROC, THREADS>(
+                            quad, take, cc,
+                            [&](int e, double &K, double &q) {
+                                K = wK[first + e];
+                                q = wQ[first + e];
+                            },
+                            [&](int e, double v) { p.out[wI[first + e]] = v; });
+                    } else if ((int)threadIdx.x < take) {
+                        const int e = first + threadIdx.x;
+                        p.out[wI[e]] = batch_eval64<PROC>(wK[e], wQ[e], cc);
+                    }
                     qn -= take;
                     did = true;
                 }
                 __syncthreads();
-                if (PREC != NOA_DCS_FP64) {
+                if constexpr (PREC != NOA_DCS_FP64) {
+                    constexpr int redo_batch = PROC == NOA_DCS_PROC_PHOTO ? QUAD_REDO : THREADS;
                     const int r = rn;
-                    if (r >= THREADS || (flush && qn == 0 && r > 0)) {
-                        const int take = r < THREADS ? r : THREADS;
-                        if (third) {
+                    if (r >= redo_batch || (flush && qn == 0 && r > 0)) {
+                        const int take = r < redo_batch ? r : redo_batch;
+                        if constexpr (third) {
                             batch_fine_step(rK, rQ, rI, xK, xQ, xI, &xn, r - take + threadIdx.x,
                                             (int)threadIdx.x < take, p.out, cc, p.tol);
+                        } else if constexpr (is_quad(PROC)) {
+                            quad_redo<PROC, THREADS>(quad, take, cc, rK + r - take, rQ + r - take, rI + r - take,
+                                                     p.out);
                         } else if ((int)threadIdx.x < take) {
                             const int e = r - take + threadIdx.x;
-                            p.out[rI[e]] = batch_redo64<PROC>(rK[e], rQ[e], cc);
+                            p.out[rI[e]] = PROC == NOA_DCS_PROC_BREMS ? brems_reference(rK[e], rQ[e], cc)
+                                                                      : ion_fp64(rK[e], rQ[e], cc);
                         }
                         __syncthreads();
                         if (threadIdx.x == 0)
@@ -284,14 +267,11 @@ __global__ void __launch_bounds__(THREADS) dcs_batched_kernel(const __grid_const
                         did = true;
                     }
                 }
-                if (third) {
+                if constexpr (third) {
                     const int x = xn;
-                    if (x >= THREADS || (flush && qn == 0 && rn == 0 && x > 0)) {
-                        const int take = x < THREADS ? x : THREADS;
-                        if ((int)threadIdx.x < take) {
-                            const int e = x - take + threadIdx.x;
-                            p.out[xI[e]] = batch_redo64<PROC>(xK[e], xQ[e], cc);
-                        }
+                    if (x >= QUAD_REDO || (flush && qn == 0 && rn == 0 && x > 0)) {
+                        const int take = x < QUAD_REDO ? x : QUAD_REDO;
+                        quad_redo<PROC, THREADS>(quad, take, cc, xK + x - take, xQ + x - take, xI + x - take, p.out);
                         __syncthreads();
                         if (threadIdx.x == 0)
                             xn = x - take;
@@ -315,8 +295,9 @@ __global__ void __launch_bounds__(THREADS) dcs_batched_kernel(const __grid_const
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             if (j < items) {
-                const int64_t i = base + j * THREADS + threadIdx.x;
-                if (i < seg_end) {
+                const int o = j * THREADS + threadIdx.x;
+                const int64_t i = base + o;
+                if (o < tile_size && i < seg_end) {
                     k[j] = p.K[i];
                     r[j] = p.q[i];
                     if (batch_open<PROC>(k[j], r[j], c))
@@ -326,7 +307,7 @@ __global__ void __launch_bounds__(THREADS) dcs_batched_kernel(const __grid_const
                 }
             }
         }
-        int pos = qn + batch_scan<THREADS>(__popc(open), warp_tot, &tile_open);
+        int pos = qn + block_scan<THREADS>(__popc(open), warp_tot, &tile_open);
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             if (open & (1u << j)) {

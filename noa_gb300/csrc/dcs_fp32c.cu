@@ -12,20 +12,22 @@
  *      evaluates it in FP32 (dcs_fp32c.cuh), which also returns an estimate
  *      of its relative error; results within `tol` are written, the others
  *      are appended (warp-aggregated) to a shared-memory redo queue;
- *   3. whenever the redo queue holds 256 pairs, each thread pops one and
- *      evaluates it in FP64 (dcs_fp64.cuh) -- except for pair production,
- *      whose redo pairs are evaluated again in FP32 with the screening log in
- *      float-float arithmetic (pprod_fp32c<false, true>); the ~1% of those
- *      still above `tol` go to a third queue, evaluated in FP64 in batches of
- *      256 the same way.
+ *   3. the redo queue is evaluated in FP64 (bremsstrahlung and ionisation 256
+ *      pairs at a time, photonuclear by quad_redo) -- except for pair
+ *      production, whose redo pairs are evaluated again, 256 at a time, in
+ *      FP32 with the screening log in float-float arithmetic
+ *      (pprod_fp32c<false, true>); the ~1% of those still above `tol` go to a
+ *      third queue, evaluated in FP64 by quad_redo.
+ *
+ * The tile follows the size of the call, so that a short list spreads over
+ * the SMs.
  *
  * FP64 work is thus proportional to the redo fraction (0-0.5% of open pairs
  * at tol = 1e-6), and every warp of every phase runs with all lanes busy.
  * No global scratch.
  */
 #include "dcs_fp32c.cuh"
-#include "dcs_fp64.cuh"
-#include "dcs_launch.h"
+#include "dcs_quad.cuh"
 
 #include <cuda_runtime.h>
 
@@ -59,29 +61,6 @@ __device__ __forceinline__ double eval32(double K, double q, const noa_dcs_const
 }
 
 template <int PROC>
-__device__ __forceinline__ double eval64(double K, double q, const noa_dcs_consts &c) {
-    if (PROC == NOA_DCS_PROC_BREMS)
-        return brems_fp64(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PPROD)
-        return pprod_fp64(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PHOTO)
-        return photo_fp64(K, q, c);
-    else
-        return ion_fp64(K, q, c);
-}
-
-// The FP64 redo: out of line for the two quadrature processes
-// (pprod_fp64_ol, photo_fp64_ol).
-template <int PROC>
-__device__ __forceinline__ double redo64(double K, double q, const noa_dcs_consts &c) {
-    if (PROC == NOA_DCS_PROC_PPROD)
-        return pprod_fp64_ol(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PHOTO)
-        return photo_fp64_ol(K, q, c);
-    return eval64<PROC>(K, q, c);
-}
-
-template <int PROC>
 __device__ __forceinline__ bool open32(double K, double q, const noa_dcs_consts &c) {
     if (PROC == NOA_DCS_PROC_PPROD)
         return pprod_live(K, q, c);
@@ -89,36 +68,6 @@ __device__ __forceinline__ bool open32(double K, double q, const noa_dcs_consts 
         return photo_live(K, q, c);
     else
         return true;
-}
-
-__device__ __forceinline__ int scan_block(int v, int *warp_tot, int *total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o)
-            x += y;
-    }
-    if (lane == 31)
-        warp_tot[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        const int w = lane < (F_THREADS >> 5) ? warp_tot[lane] : 0;
-        int s = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o)
-                s += y;
-        }
-        if (lane < (F_THREADS >> 5))
-            warp_tot[lane] = s - w;
-        if (lane == 31)
-            *total = s;
-    }
-    __syncthreads();
-    return warp_tot[warp] + x - v;
 }
 
 // The third queue exists for pair production only.
@@ -135,6 +84,7 @@ struct Queues {
     int64_t rI[F_RCAP];
     double xK[f32_xcap<PROC>()], xQ[f32_xcap<PROC>()];
     int64_t xI[f32_xcap<PROC>()];
+    QuadSmem<PROC, QUAD_REDO> quad;
     int warp_tot[F_THREADS / 32];
     int tile_open;
     int rn, xn;
@@ -205,14 +155,15 @@ __device__ __forceinline__ void fine_step(Queues<PROC> &s, int e, bool valid, do
 template <int PROC>
 __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_kernel(const double *__restrict__ K,
                                                               const double *__restrict__ q, double *out, int64_t n,
-                                                              const noa_dcs_consts c, float tol) {
+                                                              int tile, const __grid_constant__ noa_dcs_consts c,
+                                                              float tol) {
     __shared__ Queues<PROC> s;
     if (threadIdx.x == 0) {
         s.rn = 0;
         s.xn = 0;
     }
     int qn = 0;
-    int64_t base = (int64_t)blockIdx.x * F_TILE;
+    int64_t base = (int64_t)blockIdx.x * tile;
     for (;;) {
         const bool more = base < n;  // block-uniform
         if (more) {
@@ -220,8 +171,9 @@ __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_ker
             unsigned open = 0;
 #pragma unroll
             for (int j = 0; j < F_ITEMS; j++) {
-                const int64_t i = base + j * F_THREADS + threadIdx.x;
-                if (i < n) {
+                const int o = j * F_THREADS + threadIdx.x;
+                const int64_t i = base + o;
+                if (o < tile && i < n) {
                     k[j] = K[i];
                     r[j] = q[i];
                     if (open32<PROC>(k[j], r[j], c))
@@ -230,7 +182,7 @@ __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_ker
                         out[i] = 0.;
                 }
             }
-            int pos = qn + scan_block(__popc(open), s.warp_tot, &s.tile_open);
+            int pos = qn + block_scan<F_THREADS>(__popc(open), s.warp_tot, &s.tile_open);
 #pragma unroll
             for (int j = 0; j < F_ITEMS; j++) {
                 if (open & (1u << j)) {
@@ -242,7 +194,7 @@ __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_ker
             }
             __syncthreads();
             qn += s.tile_open;
-            base += (int64_t)gridDim.x * F_TILE;
+            base += (int64_t)gridDim.x * tile;
         }
         // One call site each for the FP32 step, the redo step and the FP64
         // evaluation (see the FP64 kernels): full batches while tiles remain,
@@ -257,13 +209,19 @@ __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_ker
             }
             __syncthreads();
             const int rn = s.rn;
-            if (rn >= F_THREADS || (!more && qn == 0 && rn > 0)) {
-                const int take = rn < F_THREADS ? rn : F_THREADS;
-                if (PROC == NOA_DCS_PROC_PPROD) {
+            constexpr int redo_batch = PROC == NOA_DCS_PROC_PHOTO ? QUAD_REDO : F_THREADS;
+            if (rn >= redo_batch || (!more && qn == 0 && rn > 0)) {
+                const int take = rn < redo_batch ? rn : redo_batch;
+                if constexpr (PROC == NOA_DCS_PROC_PPROD) {
                     fine_step<PROC>(s, rn - take + threadIdx.x, (int)threadIdx.x < take, out, c, tol);
+                } else if constexpr (PROC == NOA_DCS_PROC_PHOTO) {
+                    quad_redo<PROC, F_THREADS>(s.quad, take, c, s.rK + rn - take, s.rQ + rn - take, s.rI + rn - take,
+                                               out);
                 } else if ((int)threadIdx.x < take) {
                     const int e = rn - take + threadIdx.x;
-                    out[s.rI[e]] = redo64<PROC>(s.rK[e], s.rQ[e], c);
+                    // bremsstrahlung's redo pairs are those at the edge
+                    out[s.rI[e]] = PROC == NOA_DCS_PROC_BREMS ? brems_reference(s.rK[e], s.rQ[e], c)
+                                                              : ion_fp64(s.rK[e], s.rQ[e], c);
                 }
                 __syncthreads();
                 if (threadIdx.x == 0)
@@ -271,14 +229,12 @@ __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_ker
                 __syncthreads();
                 did = true;
             }
-            if (PROC == NOA_DCS_PROC_PPROD) {
+            if constexpr (PROC == NOA_DCS_PROC_PPROD) {
                 const int xn = s.xn;
-                if (xn >= F_THREADS || (!more && qn == 0 && s.rn == 0 && xn > 0)) {
-                    const int take = xn < F_THREADS ? xn : F_THREADS;
-                    if ((int)threadIdx.x < take) {
-                        const int e = xn - take + threadIdx.x;
-                        out[s.xI[e]] = redo64<PROC>(s.xK[e], s.xQ[e], c);
-                    }
+                if (xn >= QUAD_REDO || (!more && qn == 0 && s.rn == 0 && xn > 0)) {
+                    const int take = xn < QUAD_REDO ? xn : QUAD_REDO;
+                    quad_redo<PROC, F_THREADS>(s.quad, take, c, s.xK + xn - take, s.xQ + xn - take, s.xI + xn - take,
+                                               out);
                     __syncthreads();
                     if (threadIdx.x == 0)
                         s.xn = xn - take;
@@ -304,10 +260,16 @@ static int sm_count() {
 template <int PROC>
 static cudaError_t launch(const double *K, const double *q, double *out, int64_t n, const noa_dcs_consts &c,
                           float tol, cudaStream_t s) {
-    const int64_t tiles = (n + F_TILE - 1) / F_TILE;
-    const int64_t cap = (int64_t)sm_count() * 4;
-    const int grid = (int)(tiles < cap ? tiles : cap);
-    dcs_fp32c_kernel<PROC><<<grid, F_THREADS, 0, s>>>(K, q, out, n, c, tol);
+    // One resident wave at most, in equal tiles: the largest tile while the
+    // call fills it, else n spread over all resident CTAs (a warp at least).
+    // Equal tiles of any length beat multiples of 32, 64 or 256 (1e7 pairs:
+    // bremsstrahlung 140 us against 143, 147 and 148).
+    const int64_t cap = (int64_t)sm_count() * f32_min_ctas<PROC>();
+    const int64_t steps = (n + cap * F_TILE - 1) / (cap * F_TILE);
+    int64_t tile = (n + cap * steps - 1) / (cap * steps);
+    tile = tile < 32 ? 32 : tile;
+    const int grid = (int)((n + tile * steps - 1) / (tile * steps));
+    dcs_fp32c_kernel<PROC><<<grid, F_THREADS, 0, s>>>(K, q, out, n, (int)tile, c, tol);
     return cudaGetLastError();
 }
 

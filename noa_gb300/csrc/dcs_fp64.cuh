@@ -95,9 +95,9 @@ __device__ __forceinline__ bool brems_below(double E, double q, const noa_dcs_co
     return dist < 0;
 }
 
-// The reference's form for pairs near the kinematic edge (nu -> 1, where its
+// The reference's form, for pairs near the kinematic edge (nu -> 1, where its
 // rounded nu = q / E shows in 1 - nu) and inputs of unusual size.
-static __device__ __noinline__ double brems_edge(double K, double q, const noa_dcs_consts &c) {
+__device__ __forceinline__ double brems_reference(double K, double q, const noa_dcs_consts &c) {
     const double mass = c.mass;
     const double sqrte = 1.648721271;
     const double E = K + mass;
@@ -111,6 +111,10 @@ static __device__ __noinline__ double brems_edge(double K, double q, const noa_d
                                 lean_rcp((1. + delta * c.br_phie_factor) * (ME + delta * sqrte * c.br_BZ_e))));
     const double dcs = c.br_dcs_factor * (c.Zd * Phi_n + Phi_e) * (4. / 3. * (lean_rcp(nu) - 1.) + nu);
     return (dcs < 0.) ? 0. : dcs * c.scale_A;
+}
+
+static __device__ __noinline__ double brems_edge(double K, double q, const noa_dcs_consts &c) {
+    return brems_reference(K, q, c);
 }
 
 // 25 FP64 instructions (42 in the reference's form): the element's factors

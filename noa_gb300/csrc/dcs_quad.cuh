@@ -123,6 +123,24 @@ __device__ __forceinline__ void quad_batch(QuadSmem<PROC, B> &s, int take, const
     }
 }
 
+// FP64 redo of the FP32C kernels: `take` (1 .. QUAD_REDO) pairs of a queue
+// into out[I].  Out of line, so that the rare FP64 path does not set the
+// kernel's register budget; 32 pairs at a time, whose nodes are one round of
+// 256 threads (one thread a pair ran its 8 nodes for 60 us at the end of a
+// call, for a handful of pairs).
+constexpr int QUAD_REDO = 32;
+template <int PROC, int THREADS>
+static __device__ __noinline__ void quad_redo(QuadSmem<PROC, QUAD_REDO> &s, int take, const noa_dcs_consts &c,
+                                              const double *qK, const double *qQ, const int64_t *qI, double *out) {
+    quad_batch<PROC, THREADS>(
+        s, take, c,
+        [&](int e, double &K, double &q) {
+            K = qK[e];
+            q = qQ[e];
+        },
+        [&](int e, double v) { out[qI[e]] = v; });
+}
+
 // Exclusive scan of one small count per thread over the CTA; `total` takes
 // the sum.  Two barriers.
 template <int THREADS>
