@@ -2,7 +2,8 @@
  * LibTorch layer of the drop-in (include/noa_gb300/dcs_cuda.hh): checks the
  * tensors, picks PyTorch's current CUDA stream and calls the C ABI of
  * include/noa_dcs.h.  Mirrors src/noa/pms/dcs.cuh:30-50 of the reference
- * (vmap_* writes result in place; map_* allocates it with zeros_like first),
+ * (vmap_* writes result in place; map_* allocates it first, unfilled: every
+ * element is written),
  * and gives GPU forms of the per-K functions of dcs.hh:89-130 and 499-952
  * with the reference's argument lists.
  */
@@ -48,7 +49,7 @@ void run(int process, int precision, const Calculation &result, const Energies &
 
 Calculation alloc_and_run(int process, const Energies &K, const Energies &q, const AtomicElement &element,
                           const ParticleMass &mass) {
-    const auto result = torch::zeros_like(K);
+    const auto result = torch::empty_like(K);
     run(process, NOA_DCS_FP64, result, K, q, element, mass);
     return result;
 }
