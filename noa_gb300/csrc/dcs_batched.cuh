@@ -127,7 +127,7 @@ __device__ __forceinline__ void batch_push(bool push, double k, double q, int64_
 // Pair production, FP32C: evaluates redo-queue entry e (if valid) with the
 // float-float screening log; pairs whose estimate still exceeds tol go to the
 // third queue.
-__device__ __forceinline__ void batch_fine_step(double *rK, double *rQ, int64_t *rI, double *xK, double *xQ,
+__device__ __forceinline__ bool batch_fine_step(double *rK, double *rQ, int64_t *rI, double *xK, double *xQ,
                                                 int64_t *xI, int *xn, int e, bool valid, double *out,
                                                 const noa_dcs_consts &c, float tol) {
     bool redo = false;
@@ -144,12 +144,13 @@ __device__ __forceinline__ void batch_fine_step(double *rK, double *rQ, int64_t 
             out[i] = v;
     }
     batch_push(redo, k, q, i, xK, xQ, xI, xn);
+    return redo;
 }
 
 // FP32C: evaluates work-queue entry e (if valid) and writes it or appends it
 // to the redo queue.
 template <int PROC>
-__device__ __forceinline__ void batch_step32(double *wK, double *wQ, int64_t *wI, double *rK, double *rQ,
+__device__ __forceinline__ bool batch_step32(double *wK, double *wQ, int64_t *wI, double *rK, double *rQ,
                                              int64_t *rI, int *rn, int e, bool valid, double *out,
                                              const noa_dcs_consts &c, float tol) {
     bool redo = false;
@@ -166,6 +167,7 @@ __device__ __forceinline__ void batch_step32(double *wK, double *wQ, int64_t *wI
             out[i] = v;
     }
     batch_push(redo, k, q, i, rK, rQ, rI, rn);
+    return redo;
 }
 
 template <int PROC, int PREC, int THREADS>
@@ -187,16 +189,16 @@ __global__ void __launch_bounds__(THREADS) dcs_batched_kernel(const __grid_const
     Quads &quad = *reinterpret_cast<Quads *>(smem_raw + BatchSmem<THREADS>::queues(items, PROC, PREC));
     __shared__ int warp_tot[THREADS / 32];
     __shared__ int tile_open;
-    __shared__ int rn, xn;
+    __shared__ int s_rn, s_xn;  // places in the redo queues
     __shared__ unsigned long long s_tile;
 
     const int tile_size = p.tile;
     const long long total_tiles = p.tile_begin[p.n_seg];
     if (threadIdx.x == 0) {
-        rn = 0;
-        xn = 0;
+        s_rn = 0;
+        s_xn = 0;
     }
-    int qn = 0;
+    int qn = 0, rn = 0, xn = 0;  // queue lengths, identical in every thread
     int cur = -1;
     for (;;) {
         if (threadIdx.x == 0)
@@ -220,63 +222,77 @@ __global__ void __launch_bounds__(THREADS) dcs_batched_kernel(const __grid_const
             // differently in separately inlined copies).
             const bool flush = done || seg != cur;
             const noa_dcs_consts &cc = p.consts[cur];
+            // The redo queues' lengths are counted by the barrier that ends a
+            // step; each queue is drained below its batch before anything is
+            // added to it again (its capacity is a batch and one step's THREADS).
             for (;;) {
-                bool did = false;
+                bool did = false, rejected = false;
                 if (qn >= THREADS || (flush && qn > 0)) {
                     const int take = qn < THREADS ? qn : THREADS;
-                    const int first = qn - take;
+                    qn -= take;
                     if constexpr (PREC != NOA_DCS_FP64) {
-                        batch_step32<PROC>(wK, wQ, wI, rK, rQ, rI, &rn, first + threadIdx.x,
-                                           (int)threadIdx.x < take, p.out, cc, p.tol);
+                        rejected = batch_step32<PROC>(wK, wQ, wI, rK, rQ, rI, &s_rn, qn + threadIdx.x,
+                                                      (int)threadIdx.x < take, p.out, cc, p.tol);
                     } else if constexpr (is_quad(PROC)) {
                         quad_batch<PROC, THREADS>(
                             quad, take, cc,
                             [&](int e, double &K, double &q) {
-                                K = wK[first + e];
-                                q = wQ[first + e];
+                                K = wK[qn + e];
+                                q = wQ[qn + e];
                             },
-                            [&](int e, double v) { p.out[wI[first + e]] = v; });
+                            [&](int e, double v) { p.out[wI[qn + e]] = v; });
                     } else if ((int)threadIdx.x < take) {
-                        const int e = first + threadIdx.x;
+                        const int e = qn + threadIdx.x;
                         p.out[wI[e]] = batch_eval64<PROC>(wK[e], wQ[e], cc);
                     }
-                    qn -= take;
                     did = true;
                 }
-                __syncthreads();
-                if constexpr (PREC != NOA_DCS_FP64) {
+                if constexpr (PREC == NOA_DCS_FP64) {
+                    __syncthreads();
+                } else {
                     constexpr int redo_batch = PROC == NOA_DCS_PROC_PHOTO ? QUAD_REDO : THREADS;
-                    const int r = rn;
-                    if (r >= redo_batch || (flush && qn == 0 && r > 0)) {
-                        const int take = r < redo_batch ? r : redo_batch;
-                        if constexpr (third) {
-                            batch_fine_step(rK, rQ, rI, xK, xQ, xI, &xn, r - take + threadIdx.x,
-                                            (int)threadIdx.x < take, p.out, cc, p.tol);
-                        } else if constexpr (is_quad(PROC)) {
-                            quad_redo<PROC, THREADS>(quad, take, cc, rK + r - take, rQ + r - take, rI + r - take,
-                                                     p.out);
-                        } else if ((int)threadIdx.x < take) {
-                            const int e = r - take + threadIdx.x;
-                            p.out[rI[e]] = PROC == NOA_DCS_PROC_BREMS ? brems_reference(rK[e], rQ[e], cc)
-                                                                      : ion_fp64(rK[e], rQ[e], cc);
-                        }
-                        __syncthreads();
+                    rn += __syncthreads_count(rejected);
+                    while (rn >= redo_batch || (flush && qn == 0 && rn > 0)) {
+                        const int take = rn < redo_batch ? rn : redo_batch;
+                        rn -= take;
                         if (threadIdx.x == 0)
-                            rn = r - take;
-                        __syncthreads();
+                            s_rn = rn;
+                        if constexpr (third) {
+                            rejected = batch_fine_step(rK, rQ, rI, xK, xQ, xI, &s_xn, rn + threadIdx.x,
+                                                       (int)threadIdx.x < take, p.out, cc, p.tol);
+                            xn += __syncthreads_count(rejected);
+                            while (xn >= QUAD_REDO || (flush && qn == 0 && rn == 0 && xn > 0)) {
+                                const int some = xn < QUAD_REDO ? xn : QUAD_REDO;
+                                xn -= some;
+                                if (threadIdx.x == 0)
+                                    s_xn = xn;
+                                quad_redo<PROC, THREADS>(quad, some, cc, xK + xn, xQ + xn, xI + xn, p.out);
+                                __syncthreads();
+                            }
+                        } else if constexpr (is_quad(PROC)) {
+                            quad_redo<PROC, THREADS>(quad, take, cc, rK + rn, rQ + rn, rI + rn, p.out);
+                            __syncthreads();
+                        } else {
+                            if ((int)threadIdx.x < take) {
+                                const int e = rn + threadIdx.x;
+                                p.out[rI[e]] = PROC == NOA_DCS_PROC_BREMS ? brems_reference(rK[e], rQ[e], cc)
+                                                                          : ion_fp64(rK[e], rQ[e], cc);
+                            }
+                            __syncthreads();
+                        }
                         did = true;
                     }
-                }
-                if constexpr (third) {
-                    const int x = xn;
-                    if (x >= QUAD_REDO || (flush && qn == 0 && rn == 0 && x > 0)) {
-                        const int take = x < QUAD_REDO ? x : QUAD_REDO;
-                        quad_redo<PROC, THREADS>(quad, take, cc, xK + x - take, xQ + x - take, xI + x - take, p.out);
-                        __syncthreads();
-                        if (threadIdx.x == 0)
-                            xn = x - take;
-                        __syncthreads();
-                        did = true;
+                    if constexpr (third) {
+                        // what earlier fine steps left below a batch
+                        while (flush && qn == 0 && rn == 0 && xn > 0) {
+                            const int some = xn < QUAD_REDO ? xn : QUAD_REDO;
+                            xn -= some;
+                            if (threadIdx.x == 0)
+                                s_xn = xn;
+                            quad_redo<PROC, THREADS>(quad, some, cc, xK + xn, xQ + xn, xI + xn, p.out);
+                            __syncthreads();
+                            did = true;
+                        }
                     }
                 }
                 if (!did)

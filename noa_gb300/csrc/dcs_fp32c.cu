@@ -40,12 +40,14 @@ constexpr int F_QCAP = F_TILE + F_THREADS;
 constexpr int F_RCAP = 2 * F_THREADS;
 
 // Resident CTAs per SM that each kernel is compiled for (its register budget
-// follows).  Measured on 1e8 pairs: pair production is fastest at 2 (12.1 ms;
-// 13.8 ms at 3, where it spills); photonuclear at 4 (4.32 ms against 4.60 ms
-// at 3), with its FP64 redo out of line; the short bodies fit 4.
+// follows) and its grid is made of.  Measured at 1e7 pairs: pair production
+// 1.21 ms at 2, 1.17 at 3 and 1.19 at 4 (with half the tile, for the shared
+// memory), but 63 us against 72 and 69 at 250007; photonuclear 463 us at 4
+// (64 registers, spilling), 445 at 3, 460 at 5; bremsstrahlung / ionisation
+// 136 / 142 us at 4, 141 / 148 at 3, 144 / 146 at 5.
 template <int PROC>
 constexpr int f32_min_ctas() {
-    return PROC == NOA_DCS_PROC_PPROD ? 2 : 4;
+    return PROC == NOA_DCS_PROC_PPROD ? 2 : (PROC == NOA_DCS_PROC_PHOTO ? 3 : 4);
 }
 
 template <int PROC>
@@ -73,7 +75,7 @@ __device__ __forceinline__ bool open32(double K, double q, const noa_dcs_consts 
 // The third queue exists for pair production only.
 template <int PROC>
 constexpr int f32_xcap() {
-    return PROC == NOA_DCS_PROC_PPROD ? F_RCAP : 1;
+    return PROC == NOA_DCS_PROC_PPROD ? F_THREADS + QUAD_REDO : 1;
 }
 
 template <int PROC>
@@ -110,9 +112,9 @@ __device__ __forceinline__ void push_queue(bool push, double k, double q, int64_
 }
 
 // Evaluates work-queue entry e (if valid) in FP32 and appends it to the redo
-// queue when its error estimate exceeds tol.
+// queue when its error estimate exceeds tol (and returns that).
 template <int PROC>
-__device__ __forceinline__ void fp32_step(Queues<PROC> &s, int e, bool valid, double *out,
+__device__ __forceinline__ bool fp32_step(Queues<PROC> &s, int e, bool valid, double *out,
                                           const noa_dcs_consts &c, float tol) {
     bool redo = false;
     double k = 0., q = 0.;
@@ -128,13 +130,14 @@ __device__ __forceinline__ void fp32_step(Queues<PROC> &s, int e, bool valid, do
             out[i] = v;
     }
     push_queue(redo, k, q, i, s.rK, s.rQ, s.rI, &s.rn);
+    return redo;
 }
 
 // Pair production: evaluates redo-queue entry e (if valid) with the
 // float-float screening log and appends it to the third queue when its
 // estimate still exceeds tol.
 template <int PROC>
-__device__ __forceinline__ void fine_step(Queues<PROC> &s, int e, bool valid, double *out,
+__device__ __forceinline__ bool fine_step(Queues<PROC> &s, int e, bool valid, double *out,
                                           const noa_dcs_consts &c, float tol) {
     bool redo = false;
     double k = 0., q = 0.;
@@ -150,6 +153,7 @@ __device__ __forceinline__ void fine_step(Queues<PROC> &s, int e, bool valid, do
             out[i] = v;
     }
     push_queue(redo, k, q, i, s.xK, s.xQ, s.xI, &s.xn);
+    return redo;
 }
 
 template <int PROC>
@@ -162,7 +166,7 @@ __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_ker
         s.rn = 0;
         s.xn = 0;
     }
-    int qn = 0;
+    int qn = 0, rn = 0, xn = 0;
     int64_t base = (int64_t)blockIdx.x * tile;
     for (;;) {
         const bool more = base < n;  // block-uniform
@@ -199,45 +203,59 @@ __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_ker
         // One call site each for the FP32 step, the redo step and the FP64
         // evaluation (see the FP64 kernels): full batches while tiles remain,
         // everything at the end.
+        // The lengths of the redo queues are counted by the barrier that ends a
+        // step, identical in every thread; the shared counters only hand out
+        // places.  Each queue is drained below its batch before anything is
+        // added to it again, so that its capacity (a batch and one step's 256)
+        // holds even when every pair is rejected.
         for (;;) {
-            bool did = false;
+            bool did = false, rejected = false;
             if (qn >= F_THREADS || (!more && qn > 0)) {
                 const int take = qn < F_THREADS ? qn : F_THREADS;
-                fp32_step<PROC>(s, qn - take + threadIdx.x, (int)threadIdx.x < take, out, c, tol);
+                rejected = fp32_step<PROC>(s, qn - take + threadIdx.x, (int)threadIdx.x < take, out, c, tol);
                 qn -= take;
                 did = true;
             }
-            __syncthreads();
-            const int rn = s.rn;
+            rn += __syncthreads_count(rejected);
             constexpr int redo_batch = PROC == NOA_DCS_PROC_PHOTO ? QUAD_REDO : F_THREADS;
-            if (rn >= redo_batch || (!more && qn == 0 && rn > 0)) {
+            while (rn >= redo_batch || (!more && qn == 0 && rn > 0)) {
                 const int take = rn < redo_batch ? rn : redo_batch;
-                if constexpr (PROC == NOA_DCS_PROC_PPROD) {
-                    fine_step<PROC>(s, rn - take + threadIdx.x, (int)threadIdx.x < take, out, c, tol);
-                } else if constexpr (PROC == NOA_DCS_PROC_PHOTO) {
-                    quad_redo<PROC, F_THREADS>(s.quad, take, c, s.rK + rn - take, s.rQ + rn - take, s.rI + rn - take,
-                                               out);
-                } else if ((int)threadIdx.x < take) {
-                    const int e = rn - take + threadIdx.x;
-                    // bremsstrahlung's redo pairs are those at the edge
-                    out[s.rI[e]] = PROC == NOA_DCS_PROC_BREMS ? brems_reference(s.rK[e], s.rQ[e], c)
-                                                              : ion_fp64(s.rK[e], s.rQ[e], c);
-                }
-                __syncthreads();
+                rn -= take;
                 if (threadIdx.x == 0)
-                    s.rn = rn - take;
-                __syncthreads();
+                    s.rn = rn;
+                if constexpr (PROC == NOA_DCS_PROC_PPROD) {
+                    rejected = fine_step<PROC>(s, rn + threadIdx.x, (int)threadIdx.x < take, out, c, tol);
+                    xn += __syncthreads_count(rejected);
+                    while (xn >= QUAD_REDO || (!more && qn == 0 && rn == 0 && xn > 0)) {
+                        const int some = xn < QUAD_REDO ? xn : QUAD_REDO;
+                        xn -= some;
+                        if (threadIdx.x == 0)
+                            s.xn = xn;
+                        quad_redo<PROC, F_THREADS>(s.quad, some, c, s.xK + xn, s.xQ + xn, s.xI + xn, out);
+                        __syncthreads();
+                    }
+                } else if constexpr (PROC == NOA_DCS_PROC_PHOTO) {
+                    quad_redo<PROC, F_THREADS>(s.quad, take, c, s.rK + rn, s.rQ + rn, s.rI + rn, out);
+                    __syncthreads();
+                } else {
+                    if ((int)threadIdx.x < take) {
+                        const int e = rn + threadIdx.x;
+                        // bremsstrahlung's redo pairs are those at the edge
+                        out[s.rI[e]] = PROC == NOA_DCS_PROC_BREMS ? brems_reference(s.rK[e], s.rQ[e], c)
+                                                                  : ion_fp64(s.rK[e], s.rQ[e], c);
+                    }
+                    __syncthreads();
+                }
                 did = true;
             }
             if constexpr (PROC == NOA_DCS_PROC_PPROD) {
-                const int xn = s.xn;
-                if (xn >= QUAD_REDO || (!more && qn == 0 && s.rn == 0 && xn > 0)) {
-                    const int take = xn < QUAD_REDO ? xn : QUAD_REDO;
-                    quad_redo<PROC, F_THREADS>(s.quad, take, c, s.xK + xn - take, s.xQ + xn - take, s.xI + xn - take,
-                                               out);
-                    __syncthreads();
+                // what earlier fine steps left below a batch
+                while (!more && qn == 0 && rn == 0 && xn > 0) {
+                    const int some = xn < QUAD_REDO ? xn : QUAD_REDO;
+                    xn -= some;
                     if (threadIdx.x == 0)
-                        s.xn = xn - take;
+                        s.xn = xn;
+                    quad_redo<PROC, F_THREADS>(s.quad, some, c, s.xK + xn, s.xQ + xn, s.xI + xn, out);
                     __syncthreads();
                     did = true;
                 }
