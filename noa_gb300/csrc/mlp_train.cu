@@ -4,7 +4,7 @@
  * noa_dcs_mlp_*).  No counterpart in the reference.
  *
  * Training runs on the 5th-generation tensor cores (tcgen05.mma, operands in
- * shared memory, FP32 accumulator in TMEM; tcgen05.cuh) in BF16 with FP32
+ * shared memory, FP32 accumulators in TMEM; tcgen05.cuh) in BF16 with FP32
  * accumulation: the 128 x 128 products of the two hidden layers, their input
  * gradients and their weight gradients.  The first layer (4 inputs) and
  * the output layer (1 output) are FP32 on the CUDA cores.  In the forward
@@ -13,6 +13,12 @@
  * A_hi W_hi + A_lo W_hi + A_hi W_lo with FP32 accumulation; the weight pairs
  * are refreshed from the FP32 master copy after every Adam step, so training
  * sees the numerics of inference.  Gradients flow in single BF16.
+ *
+ * One kernel takes a tile of 128 samples through the whole network and back
+ * (mlp_tile_kernel); a training step is that kernel and Adam.  A kernel per
+ * product, with every activation and gradient through global memory, took 15
+ * launches and 180 us a step at batch 8192, most of it staging, launch latency
+ * and 8192 atomics on the loss.
  *
  * Loss: mean squared error of the normalised residual (mlp.cuh).
  */
@@ -37,30 +43,29 @@ using namespace noa_mlp;
 namespace {
 
 constexpr int NPARAM_PAD = (NPARAM + 3) & ~3;  // parameter-sized buffers, padded to 16 bytes
-constexpr int G_THREADS = 256;
-constexpr int G_TMEM_COLS = 128;  // the 128 x 128 FP32 accumulator
+constexpr int TILE_THREADS = 512;
 using noa_tc::MAT_BYTES;
 
-enum { G_FWD = 0, G_DX = 1, G_DW = 2 };
+// Transposed operands (rows = units, K = samples) are written by threads that
+// own a sample: K-adjacent core matrices lie 144 bytes apart instead of 128,
+// so that the 32 samples of a warp reach different banks.
+constexpr uint32_t T_LBO = 144, T_SBO = 16 * T_LBO, T_BYTES = 16 * T_SBO;
 
-// Dynamic shared memory of a mode: FWD stages A hi / lo and W hi / lo, the
-// gradient modes one A and one B operand; 1 KB of alignment slack.
-template <int MODE>
-constexpr size_t gemm_smem() {
-    return (MODE == G_FWD ? 4u : 2u) * MAT_BYTES + 1024u;
-}
+// Dynamic shared memory: six 128 x 128 BF16 operands, the last with room for a
+// transposed one, and 1 KB of alignment slack.
+constexpr size_t TILE_SMEM = 5 * MAT_BYTES + T_BYTES + 1024;
 
-struct GemmArgs {
-    const float *A;         // FWD: layer input H [M][128]; DX, DW: dZ [M][128]
-    const float *B;         // DW: H_prev [M][128]
-    const __nv_bfloat16 *W; // FWD, DX: weights [128 out][128 in] (hi); FWD also reads lo at W + 2*128*128
-    const float *bias;      // FWD
-    const float *zprev;     // DX: pre-activation of the previous layer [M][128]
-    float *outZ;            // FWD: Z; DX: dZ_prev
-    float *outH;            // FWD: H = silu(Z)
-    float *dW;              // DW: [128 out][128 in], accumulated
-    float *db;              // DW: [128], accumulated
+struct TileArgs {
+    const float *X;         // [.][4] normalised features
+    const float *T;         // [.] targets (training)
+    const int32_t *perm;    // sample of row i, or nullptr: i itself
+    const float *P;         // parameters
+    const __nv_bfloat16 *Wb;  // six 128 x 128 matrices, see mlp_round_weights_kernel
+    float *G;               // gradient, accumulated (training)
+    float *loss;            // accumulated (training)
+    float *pred;            // predictions (not training)
     unsigned int *status;   // set to NOA_DCS_ERROR_TIMEOUT if an mbarrier wait expires
+    float inv_batch;
     int M;
 };
 
@@ -79,306 +84,424 @@ __device__ __forceinline__ void split8(const float (&v)[8], uint4 &hi, uint4 &lo
     lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-// One CTA per 128-row tile, on the 5th-generation tensor cores:
-//   FWD: Z = A W^T + b with A and W as BF16 hi + lo pairs (three products
-//        A_hi W_hi + A_lo W_hi + A_hi W_lo), H = silu(Z)
-//   DX : dZ_prev = (dZ W) * silu'(z_prev)          (B operand = W^T)
-//   DW : dW += dZ^T H_prev over this tile's samples  (M = out, N = in, K = samples)
-// The operands are staged as BF16 in shared memory in the canonical K-major
-// layout (tcgen05.cuh): item e covers row r = e % 128 and the 8 K-consecutive
-// elements k0 .. k0 + 7, k0 = 8 (e / 128), one 16-byte store per item (a warp
-// stores 32 rows of one K-block: conflict-free).  Where the product needs a
-// transposed operand (DX's W^T, DW's dZ^T and H_prev^T) the 8 elements come
-// from 8 source rows at column r, which across a warp are coalesced reads.
-// One thread issues the MMAs into a 128-column TMEM accumulator and commits
-// to an mbarrier; every thread waits (bounded), then warp w reads TMEM lanes
-// 32 (w % 4) .. + 31 (rows) and columns 64 (w / 4) .. + 63 for the epilogue.
-template <int MODE>
-__global__ void __launch_bounds__(G_THREADS, 1) mlp_gemm_kernel(const GemmArgs g) {
+__device__ __forceinline__ uint4 pack8(const float *v) {
+    uint32_t h[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const __nv_bfloat162 p = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        h[i] = *reinterpret_cast<const uint32_t *>(&p);
+    }
+    return make_uint4(h[0], h[1], h[2], h[3]);
+}
+
+// Column sums over the warp's 32 rows of v[0 .. 31] (columns): lane l returns
+// the sum of column l.  Recursive halving, 31 shuffles; destroys v.
+__device__ __forceinline__ float column_sum(float (&v)[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int w = 16; w >= 1; w >>= 1) {
+#pragma unroll
+        for (int i = 0; i < w; i++) {
+            const bool up = lane & w;
+            const float keep = up ? v[i + w] : v[i], send = up ? v[i] : v[i + w];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+        }
+    }
+    return v[0];
+}
+
+__device__ __forceinline__ uint64_t make_desc_t(uint32_t saddr) {
+    return (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)(T_LBO >> 4) << 16) | ((uint64_t)(T_SBO >> 4) << 32) |
+           (1ULL << 46);
+}
+
+// 32 units [u0, u0 + 32) of sample `row` into a transposed operand.
+__device__ __forceinline__ void store_transposed(unsigned char *buf, int row, int u0, const float (&v)[32]) {
+    unsigned char *p = buf + (row >> 3) * T_LBO + (row & 7) * 2;
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+        const int u = u0 + i;
+        *reinterpret_cast<__nv_bfloat16 *>(p + (u >> 3) * T_SBO + (u & 7) * 16) = __float2bfloat16_rn(v[i]);
+    }
+}
+
+// 32 units of sample `row` into a K-major operand (one 16-byte store per 8).
+__device__ __forceinline__ void store_rows(unsigned char *buf, int row, int u0, const float (&v)[32]) {
+#pragma unroll
+    for (int i = 0; i < 32; i += 8)
+        *reinterpret_cast<uint4 *>(buf + noa_tc::canon_off(row, u0 + i)) = pack8(v + i);
+}
+__device__ __forceinline__ void store_rows_split(unsigned char *hi, unsigned char *lo, int row, int u0,
+                                                 const float (&v)[32]) {
+#pragma unroll
+    for (int i = 0; i < 32; i += 8) {
+        float w[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            w[j] = v[i + j];
+        uint4 h, l;
+        split8(w, h, l);
+        *reinterpret_cast<uint4 *>(hi + noa_tc::canon_off(row, u0 + i)) = h;
+        *reinterpret_cast<uint4 *>(lo + noa_tc::canon_off(row, u0 + i)) = l;
+    }
+}
+
+// A 128 x 128 BF16 matrix (row-major) into a K-major operand, by asynchronous
+// copies of the calling thread's current group.
+__device__ __forceinline__ void stage_matrix(unsigned char *buf, const __nv_bfloat16 *W) {
+    const uint32_t base = noa_tc::smem_u32(buf);
+#pragma unroll
+    for (int e = threadIdx.x; e < H * H / 8; e += TILE_THREADS) {
+        const int r = e % H, k0 = (e / H) * 8;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(base + noa_tc::canon_off(r, k0)),
+                     "l"(W + r * H + k0)
+                     : "memory");
+    }
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copies_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+// One tile of 128 samples through the network (pred), or through the network
+// and back (TRAIN: loss and gradient accumulated).  Thread t owns sample
+// (t / 32 % 4) 32 + t % 32, its TMEM lane, and the 32 units from 32 (t / 128):
+// it computes their activations, writes them as the next product's operands
+// and keeps what the way back needs in registers; one thread issues each
+// product's MMAs and commits to an mbarrier, every thread waits (bounded).
+// The kernel is straight-line code that each warp runs once, so its length
+// counts (64 units a thread: 9200 instructions a warp, 4.5 "no instruction"
+// stalls an issue, 64 us): each sigmoid is computed once and serves the
+// activation and its derivative.
+//
+// Operands, six buffers of 32 KB:
+//   forward   P0 W2 hi, P1 W2 lo, P2 W3 hi, P3 W3 lo, P4 / P5 activations hi / lo
+//   backward  P0 W3^T, P1 W2^T (copied from the end of layer 2 on), P2 H_prev^T,
+//             P4 dZ, P5 dZ^T:  dZ_prev = dZ W  (acc0),  dW = dZ^T H_prev  (acc1)
+// Every buffer is rewritten only after the wait for the product that read it.
+template <bool TRAIN>
+__global__ void __launch_bounds__(TILE_THREADS, 1) mlp_tile_kernel(const TileArgs a) {
     using namespace noa_tc;
     extern __shared__ unsigned char smem_raw[];
-    unsigned char *sm = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    unsigned char *sA = sm, *sB = sm + MAT_BYTES;
-    unsigned char *sAl = sm + 2 * MAT_BYTES, *sBl = sm + 3 * MAT_BYTES;  // FWD only
+    unsigned char *const P0 = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+    unsigned char *const P1 = P0 + MAT_BYTES, *const P2 = P0 + 2 * MAT_BYTES, *const P3 = P0 + 3 * MAT_BYTES,
+                        *const P4 = P0 + 4 * MAT_BYTES, *const P5 = P0 + 5 * MAT_BYTES;
+    __shared__ float4 sW1[H], sX[H];
+    __shared__ float sb1[H], sb2[H], sb3[H], sWo[H], sy[4][H];
+    __shared__ float s_sum[3][H];  // dWo, db3, db2
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(8) unsigned long long mbar;
-    const int row0 = blockIdx.x * H;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row = (warp & 3) * 32 + lane, part = warp >> 2, u0 = part * 32;
+    constexpr uint32_t cols = TRAIN ? 256 : 128;
 
     if (warp == 0)
-        tmem_alloc(smem_u32(&tmem_slot), G_TMEM_COLS);
+        tmem_alloc(smem_u32(&tmem_slot), cols);
     if (tid == 0) {
         mbar_init(smem_u32(&mbar), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-
-    // stage the operands
-    for (int e = tid; e < H * H / 8; e += G_THREADS) {
-        const int r = e % H, k0 = (e / H) * 8;
-        const uint32_t o = canon_off(r, k0);
-        float v[8];
-        if (MODE == G_DW) {
-            // A(r = out, k = sample) = dZ[k][r]; B(r = in, k = sample) = H_prev[k][r]
-            float w[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const bool in = row0 + k0 + j < g.M;
-                v[j] = in ? g.A[(size_t)(row0 + k0 + j) * H + r] : 0.f;
-                w[j] = in ? g.B[(size_t)(row0 + k0 + j) * H + r] : 0.f;
-            }
-            uint4 hi, lo;
-            split8(v, hi, lo);
-            *reinterpret_cast<uint4 *>(sA + o) = hi;
-            split8(w, hi, lo);
-            *reinterpret_cast<uint4 *>(sB + o) = hi;
-        } else {
-            // A(r = sample, k) = A[r][k]
-            if (row0 + r < g.M) {
-                const float4 *src = reinterpret_cast<const float4 *>(g.A + (size_t)(row0 + r) * H + k0);
-                const float4 x = src[0], y = src[1];
-                v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    v[j] = 0.f;
-            }
-            uint4 hi, lo;
-            split8(v, hi, lo);
-            *reinterpret_cast<uint4 *>(sA + o) = hi;
-            if (MODE == G_FWD) {
-                *reinterpret_cast<uint4 *>(sAl + o) = lo;
-                // B(r = out, k = in) = W[r][k], hi and lo
-                *reinterpret_cast<uint4 *>(sB + o) = *reinterpret_cast<const uint4 *>(g.W + r * H + k0);
-                *reinterpret_cast<uint4 *>(sBl + o) = *reinterpret_cast<const uint4 *>(g.W + 2 * H * H + r * H + k0);
-            } else {
-                // DX: B(r = in, k = out) = W[k][r]
-                uint32_t b[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const __nv_bfloat162 t = __halves2bfloat162(g.W[(k0 + 2 * j) * H + r], g.W[(k0 + 2 * j + 1) * H + r]);
-                    b[j] = *reinterpret_cast<const uint32_t *>(&t);
-                }
-                *reinterpret_cast<uint4 *>(sB + o) = make_uint4(b[0], b[1], b[2], b[3]);
-            }
-        }
+    if (tid < H) {
+        const float *w = a.P + OFF_W1 + tid * IN;
+        sW1[tid] = make_float4(w[0], w[1], w[2], w[3]);
+        sb1[tid] = a.P[OFF_B1 + tid];
+        sb2[tid] = a.P[OFF_B2 + tid];
+        sb3[tid] = a.P[OFF_B3 + tid];
+        sWo[tid] = a.P[OFF_WO + tid];
     }
-    fence_async_smem();
+    const float bo = a.P[OFF_BO];
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t acc = tmem_slot;
+    const uint32_t acc0 = tmem_slot, acc1 = tmem_slot + 128;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t mb = smem_u32(&mbar);
+    uint32_t phase = 0;
+    bool ok = true;
 
-    if (tid == 0) {
-        const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB), al0 = smem_u32(sAl), bl0 = smem_u32(sBl);
+    // Makes the operands written so far visible and has thread 0 issue.
+    auto issue = [&](auto mmas) {
+        fence_async_smem();
+        fence_before();
+        __syncthreads();
+        fence_after();
+        if (tid == 0) {
+            mmas();
+            mma_commit(mb);
+        }
+    };
+    // True in every thread when the product is done.
+    auto wait = [&]() {
+        const bool done = mbar_wait(mb, phase);
+        phase ^= 1u;
+        fence_after();
+        return (bool)__syncthreads_and(done);
+    };
+    auto forward_mmas = [&](unsigned char *wh, unsigned char *wl) {
+        const uint32_t ah = smem_u32(P4), al = smem_u32(P5), bh = smem_u32(wh), bl = smem_u32(wl);
 #pragma unroll
-        for (int ks = 0; ks < 8; ks++) {
-            const uint32_t o = ks * 256;  // 16 K-elements = two core matrices
-            const uint64_t a = make_desc(a0 + o), b = make_desc(b0 + o);
-            mma_ss(acc, a, b, ks > 0);
-            if (MODE == G_FWD) {
-                mma_ss(acc, make_desc(al0 + o), b, 1);
-                mma_ss(acc, a, make_desc(bl0 + o), 1);
+        for (int o = 0; o < 8 * 256; o += 256) {  // 16 K-elements = two core matrices
+            mma_ss(acc0, make_desc(ah + o), make_desc(bh + o), o > 0);
+            mma_ss(acc0, make_desc(al + o), make_desc(bh + o), 1);
+            mma_ss(acc0, make_desc(ah + o), make_desc(bl + o), 1);
+        }
+    };
+    auto backward_mmas = [&](unsigned char *wt) {
+        const uint32_t d = smem_u32(P4), w = smem_u32(wt), dt = smem_u32(P5), ht = smem_u32(P2);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            mma_ss(acc0, make_desc(d + k * 256), make_desc(w + k * 256), k > 0);
+            mma_ss(acc1, make_desc_t(dt + k * 2 * T_LBO), make_desc_t(ht + k * 2 * T_LBO), k > 0);
+        }
+    };
+    // The weight gradient in acc1: row = out unit, 32 in units per thread.
+    auto add_dw = [&](float *dW) {
+        float v[32];
+        tmem_ld32(acc1 + lane_base + (uint32_t)u0, v);
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)  // 16-byte vector atomics (the weight blocks of G are 16-byte aligned)
+            atomicAdd(reinterpret_cast<float4 *>(&dW[row * H + u0 + j]),
+                      make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+    };
+    // silu(z), and its derivative in d
+    auto silu2 = [](float z, float &d) {
+        const float g = __fdividef(1.f, 1.f + __expf(-z));
+        d = g * (1.f + z * (1.f - g));
+        return silu(z);
+    };
+    auto layer1 = [&](float4 x, int u) {
+        const float4 w = sW1[u];
+        return fmaf(w.w, x.w, fmaf(w.z, x.z, fmaf(w.y, x.y, fmaf(w.x, x.x, sb1[u]))));
+    };
+
+    const int tiles = (a.M + H - 1) / H;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int s = tile * H + row;
+        const bool valid = s < a.M;
+        const int64_t src = valid ? (a.perm ? (int64_t)a.perm[s] : (int64_t)s) : 0;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (valid)
+            x = make_float4(a.X[src * IN], a.X[src * IN + 1], a.X[src * IN + 2], a.X[src * IN + 3]);
+        if (TRAIN || tile == blockIdx.x) {
+            stage_matrix(P0, a.Wb);
+            stage_matrix(P1, a.Wb + 2 * H * H);
+            copies_commit();
+            stage_matrix(P2, a.Wb + H * H);
+            stage_matrix(P3, a.Wb + 3 * H * H);
+            copies_commit();
+        }
+        if (TRAIN) {
+            if (part == 0)
+                sX[row] = x;
+            if (tid < H)
+                s_sum[0][tid] = s_sum[1][tid] = s_sum[2][tid] = 0.f;
+        }
+        // layer 1 (FP32)
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            v[j] = silu(layer1(x, u0 + j));
+        store_rows_split(P4, P5, row, u0, v);
+        // layer 2
+        copies_wait<1>();
+        issue([&] { forward_mmas(P0, P1); });
+        if (!(ok = wait()))
+            break;
+        if (TRAIN) {  // the transposed weights of the way back
+            stage_matrix(P0, a.Wb + 5 * H * H);
+            stage_matrix(P1, a.Wb + 4 * H * H);
+            copies_commit();
+        }
+        float z2[32];
+        tmem_ld32(acc0 + lane_base + (uint32_t)u0, z2);
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+            z2[j] += sb2[u0 + j];
+            v[j] = silu(z2[j]);
+        }
+        store_rows_split(P4, P5, row, u0, v);
+        // layer 3
+        copies_wait<TRAIN ? 1 : 0>();
+        issue([&] { forward_mmas(P2, P3); });
+        if (!(ok = wait()))
+            break;
+        // output layer (FP32); v = h3, d3 = silu'(z3)
+        float d3[32], y = 0.f;
+        tmem_ld32(acc0 + lane_base + (uint32_t)u0, v);
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+            v[j] = silu2(v[j] + sb3[u0 + j], d3[j]);
+            y = fmaf(sWo[u0 + j], v[j], y);
+        }
+        sy[part][row] = y;
+        __syncthreads();
+        y = bo + ((sy[0][row] + sy[1][row]) + (sy[2][row] + sy[3][row]));
+        if (!TRAIN) {
+            if (part == 0 && valid)
+                a.pred[s] = y;
+            fence_before();  // this tile's TMEM reads before the next tile's products
+            __syncthreads();
+            fence_after();
+            continue;
+        }
+        // loss and its gradient
+        const float d = valid ? y - a.T[src] : 0.f;
+        const float dp = 2.f * d * a.inv_batch;
+        if (part == 0) {
+            float l = d * d * a.inv_batch, b = dp;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                l += __shfl_xor_sync(0xffffffffu, l, o);
+                b += __shfl_xor_sync(0xffffffffu, b, o);
+            }
+            if (lane == 0) {
+                atomicAdd(a.loss, l);
+                atomicAdd(&a.G[OFF_BO], b);
             }
         }
-        mma_commit(mb);
-    }
-    const bool ok = mbar_wait(mb, 0);
-    fence_after();
-
-    if (ok) {
-        const int row = (warp & 3) * 32 + lane;
-        const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-#pragma unroll 1
-        for (int half = 0; half < 2; half++) {
-            const int c0 = (warp >> 2) * 64 + half * 32;
-            float v[32];
-            tmem_ld32(acc + lane_base + (uint32_t)c0, v);
-            if (MODE == G_DW) {
-                // row = out index, column = in index; 16-byte vector atomics
-                // (the weight blocks of G start 16-byte aligned)
+        // dZ3, H2^T; dWo, db3; z2 becomes silu'(z2)
 #pragma unroll
-                for (int j = 0; j < 32; j += 4)
-                    atomicAdd(reinterpret_cast<float4 *>(&g.dW[row * H + c0 + j]),
-                              make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
-            } else if (row0 + row < g.M) {
-                const size_t o = (size_t)(row0 + row) * H + c0;
-                if (MODE == G_FWD) {
-#pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        float4 z, h;
-                        z.x = v[j] + g.bias[c0 + j];
-                        z.y = v[j + 1] + g.bias[c0 + j + 1];
-                        z.z = v[j + 2] + g.bias[c0 + j + 2];
-                        z.w = v[j + 3] + g.bias[c0 + j + 3];
-                        h.x = silu(z.x), h.y = silu(z.y), h.z = silu(z.z), h.w = silu(z.w);
-                        *reinterpret_cast<float4 *>(g.outZ + o + j) = z;
-                        *reinterpret_cast<float4 *>(g.outH + o + j) = h;
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        const float4 zp = *reinterpret_cast<const float4 *>(g.zprev + o + j);
-                        float4 d;
-                        d.x = v[j] * dsilu(zp.x), d.y = v[j + 1] * dsilu(zp.y);
-                        d.z = v[j + 2] * dsilu(zp.z), d.w = v[j + 3] * dsilu(zp.w);
-                        *reinterpret_cast<float4 *>(g.outZ + o + j) = d;
-                    }
-                }
-            }
+        for (int j = 0; j < 32; j++) {
+            v[j] *= dp;
+            d3[j] *= dp * sWo[u0 + j];
         }
-    } else {
-        if (lane == 0)
-            atomicMax(g.status, (unsigned int)NOA_DCS_ERROR_TIMEOUT);
-        mbar_wait(mb, 0);  // one more bounded wait before the TMEM it writes is freed
+        atomicAdd(&s_sum[0][u0 + lane], column_sum(v));
+        store_rows(P4, row, u0, d3);
+        store_transposed(P5, row, u0, d3);
+        atomicAdd(&s_sum[1][u0 + lane], column_sum(d3));
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            v[j] = silu2(z2[j], z2[j]);
+        store_transposed(P2, row, u0, v);
+        // dW3 = dZ3^T H2, dZ2 = (dZ3 W3) silu'(Z2)
+        copies_wait<0>();
+        issue([&] { backward_mmas(P0); });
+        if (!(ok = wait()))
+            break;
+        add_dw(a.G + OFF_W3);
+        tmem_ld32(acc0 + lane_base + (uint32_t)u0, v);
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            v[j] *= z2[j];
+        store_rows(P4, row, u0, v);
+        store_transposed(P5, row, u0, v);
+        atomicAdd(&s_sum[2][u0 + lane], column_sum(v));
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            v[j] = silu2(layer1(x, u0 + j), z2[j]);  // z2: silu'(z1)
+        store_transposed(P2, row, u0, v);
+        // dW2 = dZ2^T H1, dZ1 = (dZ2 W2) silu'(Z1)
+        issue([&] { backward_mmas(P1); });
+        if (!(ok = wait()))
+            break;
+        add_dw(a.G + OFF_W2);
+        // layer 1: dZ1 in FP32 through shared memory (rows of 129 words over the
+        // staged weights), then a thread per unit and quarter of the samples
+        float *D1 = reinterpret_cast<float *>(P0);
+        tmem_ld32(acc0 + lane_base + (uint32_t)u0, v);
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            D1[row * (H + 1) + u0 + j] = v[j] * z2[j];
+        fence_before();
+        __syncthreads();
+        fence_after();
+        {
+            const int j = tid & (H - 1), first = (tid >> 7) * 32;
+            float gb = 0.f, gw[IN] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+            for (int i = first; i < first + 32; i++) {
+                const float g = D1[i * (H + 1) + j];
+                const float4 xi = sX[i];
+                gb += g;
+                gw[0] = fmaf(g, xi.x, gw[0]);
+                gw[1] = fmaf(g, xi.y, gw[1]);
+                gw[2] = fmaf(g, xi.z, gw[2]);
+                gw[3] = fmaf(g, xi.w, gw[3]);
+            }
+#pragma unroll
+            for (int c = 0; c < IN; c++)
+                atomicAdd(&a.G[OFF_W1 + j * IN + c], gw[c]);
+            atomicAdd(&a.G[OFF_B1 + j], gb);
+        }
+        if (tid < H) {
+            atomicAdd(&a.G[OFF_WO + tid], s_sum[0][tid]);
+            atomicAdd(&a.G[OFF_B3 + tid], s_sum[1][tid]);
+            atomicAdd(&a.G[OFF_B2 + tid], s_sum[2][tid]);
+        }
+        __syncthreads();  // the next tile stages over D1 and clears the sums
     }
-    if (MODE == G_DW && tid < H) {
-        float s = 0.f;
-        for (int k = 0; k < H && row0 + k < g.M; k++)
-            s += g.A[(size_t)(row0 + k) * H + tid];
-        atomicAdd(&g.db[tid], s);
+    if (!ok) {
+        if (tid == 0)
+            atomicMax(a.status, (unsigned int)NOA_DCS_ERROR_TIMEOUT);
+        mbar_wait(mb, phase ^ 1u);  // one more bounded wait before the TMEM it writes is freed
     }
     fence_before();
     __syncthreads();
     fence_after();
     if (warp == 0)
-        tmem_dealloc(acc, G_TMEM_COLS);
+        tmem_dealloc(acc0, cols);
 }
 
-// Layer 1 (FP32): Z1 = X W1^T + b1, H1 = silu(Z1).
-__global__ void mlp_fwd1_kernel(const float *__restrict__ X, const float *__restrict__ P, float *Z1, float *H1,
-                                int M) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < M * H; e += gridDim.x * blockDim.x) {
-        const int s = e / H, j = e % H;
-        float z = P[OFF_B1 + j];
-#pragma unroll
-        for (int i = 0; i < IN; i++)
-            z = fmaf(P[OFF_W1 + j * IN + i], X[s * IN + i], z);
-        Z1[e] = z;
-        H1[e] = silu(z);
-    }
-}
-
-// Output layer (FP32) and the loss gradient: pred = Wo h3 + bo,
-// loss = mean (pred - t)^2 over the batch of M samples (scaled by inv_batch);
-// dZ3 = dpred Wo * silu'(z3); dWo, dbo accumulated per CTA.  128 samples per CTA.
-__global__ void __launch_bounds__(128) mlp_out_kernel(const float *__restrict__ H3, const float *__restrict__ Z3,
-                                                      const float *__restrict__ T, const float *__restrict__ P,
-                                                      float *dZ3, float *G, float *loss, int M, float inv_batch,
-                                                      float *pred_out) {
-    __shared__ float sd[128];
-    const int s = blockIdx.x * 128 + threadIdx.x;
-    const int ns = min(128, M - (int)blockIdx.x * 128);  // samples of this CTA
-    float dp = 0.f;
-    if (s < M) {
-        // four partial sums: the row's loads are independent and overlap
-        float y4[4] = {P[OFF_BO], 0.f, 0.f, 0.f};
-#pragma unroll 8
-        for (int k = 0; k < H; k++)
-            y4[k & 3] = fmaf(P[OFF_WO + k], H3[(size_t)s * H + k], y4[k & 3]);
-        const float y = (y4[0] + y4[1]) + (y4[2] + y4[3]);
-        if (pred_out)
-            pred_out[s] = y;
-        if (T) {
-            const float d = y - T[s];
-            dp = 2.f * d * inv_batch;
-            atomicAdd(loss, d * d * inv_batch);
-        }
-    }
-    sd[threadIdx.x] = dp;
-    __syncthreads();
-    if (!T)
+// The BF16 forms of W2, W3 that the products read, six 128 x 128 matrices: W2
+// hi, W3 hi, W2 lo, W3 lo, and W2 hi, W3 hi transposed (the way back).
+//
+// UPDATE_CTAS CTAs of 1024 threads cover the parameters, one each: the first
+// 32 CTAs a 32 x 32 block of W2 or W3 each (its transposed half through shared
+// memory, so that both are written in rows), the others the rest.  f(i) gives
+// parameter i's new value.
+constexpr int UPDATE_CTAS = 32 + 2, UPDATE_THREADS = 1024;
+template <typename F>
+__device__ __forceinline__ void update_parameters(__nv_bfloat16 *Wb, F f) {
+    __shared__ __nv_bfloat16 t[32][33];
+    const int c = threadIdx.x & 31, r = threadIdx.x >> 5;
+    // W1 b1 | b2 | b3 Wo bo
+    constexpr int n1 = OFF_W2, n2 = n1 + H, n3 = n2 + NPARAM - OFF_B3;
+    static_assert((UPDATE_CTAS - 32) * UPDATE_THREADS >= n3, "every parameter has a thread");
+    const bool block = blockIdx.x < 32;
+    const int layer = blockIdx.x >> 4, row = (blockIdx.x >> 2 & 3) * 32, col = (blockIdx.x & 3) * 32;
+    const int w = (row + r) * H + col + c;
+    const int k = ((int)blockIdx.x - 32) * UPDATE_THREADS + threadIdx.x;
+    if (!block && k >= n3)
         return;
-    if (s < M) {
-#pragma unroll 8
-        for (int k = 0; k < H; k++)
-            dZ3[(size_t)s * H + k] = dp * P[OFF_WO + k] * dsilu(Z3[(size_t)s * H + k]);
+    const float p = f(block ? (layer ? OFF_W3 : OFF_W2) + w
+                            : (k < n1 ? k : (k < n2 ? OFF_B2 + k - n1 : OFF_B3 + k - n2)));
+    if (block) {
+        const __nv_bfloat16 hi = __float2bfloat16_rn(p);
+        Wb[layer * H * H + w] = hi;
+        Wb[(2 + layer) * H * H + w] = __float2bfloat16_rn(p - __bfloat162float(hi));
+        t[r][c] = hi;
+        __syncthreads();
+        Wb[(4 + layer) * H * H + (col + r) * H + row + c] = t[c][r];
     }
-    // dWo[k] = sum_s dp_s h3[s][k], thread k (coalesced across threads)
-    const int k = threadIdx.x;
-    float g4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-    for (int i = 0; i < ns; i++)
-        g4[i & 3] = fmaf(sd[i], H3[(size_t)(blockIdx.x * 128 + i) * H + k], g4[i & 3]);
-    const float g = (g4[0] + g4[1]) + (g4[2] + g4[3]);
-    atomicAdd(&G[OFF_WO + k], g);
-    if (k == 0) {
-        float b = 0.f;
-        for (int i = 0; i < 128; i++)
-            b += sd[i];
-        atomicAdd(&G[OFF_BO], b);
-    }
-}
-
-// Layer-1 gradients: dW1[j][i] += sum_s dZ1[s][j] X[s][i], db1 += sum dZ1.  128 samples per CTA.
-__global__ void __launch_bounds__(128) mlp_bwd1_kernel(const float *__restrict__ dZ1, const float *__restrict__ X,
-                                                       float *G, int M) {
-    const int j = threadIdx.x;
-    const int ns = min(128, M - (int)blockIdx.x * 128);  // samples of this CTA
-    float gw[IN] = {0.f, 0.f, 0.f, 0.f}, gb = 0.f;
-    // bounds hoisted out of the loop so that the unrolled loads overlap
-#pragma unroll 8
-    for (int i = 0; i < ns; i++) {
-        const int s = blockIdx.x * 128 + i;
-        const float d = dZ1[(size_t)s * H + j];
-        const float4 x = reinterpret_cast<const float4 *>(X)[s];
-        gb += d;
-        gw[0] = fmaf(d, x.x, gw[0]);
-        gw[1] = fmaf(d, x.y, gw[1]);
-        gw[2] = fmaf(d, x.z, gw[2]);
-        gw[3] = fmaf(d, x.w, gw[3]);
-    }
-#pragma unroll
-    for (int c = 0; c < IN; c++)
-        atomicAdd(&G[OFF_W1 + j * IN + c], gw[c]);
-    atomicAdd(&G[OFF_B1 + j], gb);
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master parameters; refreshes the BF16
-// copies of W2, W3 used by the tensor-core products.
-__global__ void mlp_adam_kernel(float *P, const float *G, float *Mm, float *V, __nv_bfloat16 *Wb, float lr,
-                                float b1, float b2, float eps, float c1, float c2) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NPARAM; i += gridDim.x * blockDim.x) {
+// weights, hands the step's loss out and leaves gradient and loss zero for
+// the next step.
+__global__ void __launch_bounds__(UPDATE_THREADS) mlp_adam_kernel(float *P, float *G, float *Mm, float *V, __nv_bfloat16 *Wb,
+                                                       float lr, float b1, float b2, float eps, float c1, float c2,
+                                                       float *loss, float *loss_out) {
+    update_parameters(Wb, [&](int i) {
         const float g = G[i];
+        G[i] = 0.f;
         const float m = b1 * Mm[i] + (1.f - b1) * g;
         const float v = b2 * V[i] + (1.f - b2) * g * g;
         Mm[i] = m;
         V[i] = v;
         const float p = P[i] - lr * (m * c1) / (sqrtf(v * c2) + eps);
         P[i] = p;
-        int w = -1;
-        if (i >= OFF_W2 && i < OFF_W2 + H * H)
-            w = i - OFF_W2;
-        else if (i >= OFF_W3 && i < OFF_W3 + H * H)
-            w = H * H + i - OFF_W3;
-        if (w >= 0) {
-            const __nv_bfloat16 hi = __float2bfloat16_rn(p);
-            Wb[w] = hi;
-            Wb[2 * H * H + w] = __float2bfloat16_rn(p - __bfloat162float(hi));
-        }
+        return p;
+    });
+    if (blockIdx.x == 32 && threadIdx.x == 0) {
+        if (loss_out)
+            *loss_out = *loss;
+        *loss = 0.f;
     }
 }
 
-// BF16 hi / lo pairs of W2, W3: Wb[0 .. 2HH) hi (W2 then W3), Wb[2HH .. 4HH) lo.
-__global__ void mlp_round_weights_kernel(const float *P, __nv_bfloat16 *Wb) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * H * H; i += gridDim.x * blockDim.x) {
-        const float p = i < H * H ? P[OFF_W2 + i] : P[OFF_W3 + i - H * H];
-        const __nv_bfloat16 hi = __float2bfloat16_rn(p);
-        Wb[i] = hi;
-        Wb[2 * H * H + i] = __float2bfloat16_rn(p - __bfloat162float(hi));
-    }
-}
-
-// Gathers a batch: Xb[i] = X[perm[i]], Tb[i] = T[perm[i]].
-__global__ void mlp_gather_kernel(const float *X, const float *T, const int32_t *perm, float *Xb, float *Tb, int M) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
-        const int s = perm[i];
-#pragma unroll
-        for (int c = 0; c < IN; c++)
-            Xb[i * IN + c] = X[(size_t)s * IN + c];
-        if (T)
-            Tb[i] = T[s];
-    }
+__global__ void __launch_bounds__(UPDATE_THREADS) mlp_round_weights_kernel(const float *P, __nv_bfloat16 *Wb) {
+    update_parameters(Wb, [&](int i) { return P[i]; });
 }
 
 // Training data: raw features and the residual target from the FP64 plain
@@ -417,9 +540,6 @@ struct noa_dcs_mlp {
     int batch = 0;
     float *P = nullptr, *G = nullptr, *Mm = nullptr, *V = nullptr;
     __nv_bfloat16 *Wb = nullptr;
-    float *Xb = nullptr, *Tb = nullptr;
-    float *Z1 = nullptr, *H1 = nullptr, *Z2 = nullptr, *H2 = nullptr, *Z3 = nullptr, *H3 = nullptr;
-    float *D3 = nullptr, *D2 = nullptr, *D1 = nullptr;
     float *loss = nullptr;
     unsigned int *status = nullptr;  // device word, see take_status
     int64_t step = 0;
@@ -438,9 +558,9 @@ int mfail(int st, const char *msg, cudaError_t e = cudaSuccess) {
     return st;
 }
 
-// Raises the three GEMM kernels' dynamic shared-memory limits once per device
+// Raises the tile kernels' dynamic shared-memory limits once per device
 // (called when a model is created).
-cudaError_t set_gemm_smem() {
+cudaError_t set_tile_smem() {
     static std::atomic<bool> done[64];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -448,14 +568,9 @@ cudaError_t set_gemm_smem() {
         return e;
     if (dev >= 0 && dev < 64 && done[dev].load())
         return cudaSuccess;
-    e = cudaFuncSetAttribute(mlp_gemm_kernel<G_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)gemm_smem<G_FWD>());
+    e = cudaFuncSetAttribute(mlp_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(mlp_gemm_kernel<G_DX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)gemm_smem<G_DX>());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(mlp_gemm_kernel<G_DW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)gemm_smem<G_DW>());
+        e = cudaFuncSetAttribute(mlp_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_SMEM);
     if (e == cudaSuccess && dev >= 0 && dev < 64)
         done[dev].store(true);
     return e;
@@ -466,65 +581,41 @@ cudaError_t set_gemm_smem() {
 // synchronises the stream.
 int take_status(noa_dcs_mlp *m, cudaStream_t s);
 
-// Forward over M <= batch rows already in m->Xb; prediction to pred if given.
-cudaError_t forward(noa_dcs_mlp *m, int M, float *pred, cudaStream_t s) {
-    const int tiles = (M + H - 1) / H;
-    mlp_fwd1_kernel<<<(M * H + 255) / 256, 256, 0, s>>>(m->Xb, m->P, m->Z1, m->H1, M);
-    GemmArgs g{};
-    g.M = M;
-    g.status = m->status;
-    g.A = m->H1;
-    g.W = m->Wb;
-    g.bias = m->P + OFF_B2;
-    g.outZ = m->Z2;
-    g.outH = m->H2;
-    mlp_gemm_kernel<G_FWD><<<tiles, G_THREADS, gemm_smem<G_FWD>(), s>>>(g);
-    g.A = m->H2;
-    g.W = m->Wb + H * H;
-    g.bias = m->P + OFF_B3;
-    g.outZ = m->Z3;
-    g.outH = m->H3;
-    mlp_gemm_kernel<G_FWD><<<tiles, G_THREADS, gemm_smem<G_FWD>(), s>>>(g);
-    if (pred)
-        mlp_out_kernel<<<tiles, 128, 0, s>>>(m->H3, m->Z3, nullptr, m->P, nullptr, nullptr, nullptr, M, 0.f, pred);
+int sm_count() {
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
+}
+
+// Prediction (pred) of M rows of X, or, with targets T, their loss and
+// gradient added to m->loss and m->G; rows perm[0 .. M) of X and T if given.
+cudaError_t run_tiles(noa_dcs_mlp *m, const float *X, const float *T, const int32_t *perm, int M, float *pred,
+                      cudaStream_t s) {
+    TileArgs a{};
+    a.X = X;
+    a.T = T;
+    a.perm = perm;
+    a.P = m->P;
+    a.Wb = m->Wb;
+    a.G = m->G;
+    a.loss = m->loss;
+    a.pred = pred;
+    a.status = m->status;
+    a.inv_batch = 1.f / (float)M;
+    a.M = M;
+    const int tiles = (M + H - 1) / H, sms = sm_count();
+    const int grid = tiles < sms ? tiles : sms;
+    if (T)
+        mlp_tile_kernel<true><<<grid, TILE_THREADS, TILE_SMEM, s>>>(a);
+    else
+        mlp_tile_kernel<false><<<grid, TILE_THREADS, TILE_SMEM, s>>>(a);
     return cudaGetLastError();
 }
 
-// Loss and gradient of one batch of M rows in Xb / Tb into m->G (zeroed first).
-cudaError_t backward(noa_dcs_mlp *m, int M, cudaStream_t s) {
-    const int tiles = (M + H - 1) / H;
-    cudaError_t e = cudaMemsetAsync(m->G, 0, sizeof(float) * NPARAM, s);
-    if (e != cudaSuccess)
-        return e;
-    if ((e = forward(m, M, nullptr, s)) != cudaSuccess)
-        return e;
-    mlp_out_kernel<<<tiles, 128, 0, s>>>(m->H3, m->Z3, m->Tb, m->P, m->D3, m->G, m->loss, M, 1.f / (float)M,
-                                         nullptr);
-    GemmArgs g{};
-    g.M = M;
-    g.status = m->status;
-    // layer 3: dW3 = dZ3^T H2, dZ2 = (dZ3 W3) silu'(Z2)
-    g.A = m->D3;
-    g.B = m->H2;
-    g.dW = m->G + OFF_W3;
-    g.db = m->G + OFF_B3;
-    mlp_gemm_kernel<G_DW><<<tiles, G_THREADS, gemm_smem<G_DW>(), s>>>(g);
-    g.W = m->Wb + H * H;
-    g.zprev = m->Z2;
-    g.outZ = m->D2;
-    mlp_gemm_kernel<G_DX><<<tiles, G_THREADS, gemm_smem<G_DX>(), s>>>(g);
-    // layer 2: dW2 = dZ2^T H1, dZ1 = (dZ2 W2) silu'(Z1)
-    g.A = m->D2;
-    g.B = m->H1;
-    g.dW = m->G + OFF_W2;
-    g.db = m->G + OFF_B2;
-    mlp_gemm_kernel<G_DW><<<tiles, G_THREADS, gemm_smem<G_DW>(), s>>>(g);
-    g.W = m->Wb;
-    g.zprev = m->Z1;
-    g.outZ = m->D1;
-    mlp_gemm_kernel<G_DX><<<tiles, G_THREADS, gemm_smem<G_DX>(), s>>>(g);
-    mlp_bwd1_kernel<<<tiles, 128, 0, s>>>(m->D1, m->Xb, m->G, M);
-    return cudaGetLastError();
+cudaError_t clear_gradient(noa_dcs_mlp *m, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(m->G, 0, sizeof(float) * NPARAM, s);
+    return e == cudaSuccess ? cudaMemsetAsync(m->loss, 0, sizeof(float), s) : e;
 }
 
 // Every buffer must be device (or managed) memory of the current device before
@@ -575,7 +666,7 @@ int noa_dcs_mlp_create(noa_dcs_mlp **out, int process, int batch) {
         return mfail(NOA_DCS_ERROR_NOT_SUPPORTED, "the surrogate covers pair production and photonuclear");
     if (batch < 128 || batch > (1 << 20) || batch % 128)
         return mfail(NOA_DCS_ERROR_INVALID_VALUE, "batch must be a multiple of 128 in [128, 2^20]");
-    cudaError_t e = set_gemm_smem();
+    cudaError_t e = set_tile_smem();
     if (e != cudaSuccess)
         return mfail(NOA_DCS_ERROR_CUDA, "cudaFuncSetAttribute", e);
     noa_dcs_mlp *m = new (std::nothrow) noa_dcs_mlp();
@@ -583,36 +674,25 @@ int noa_dcs_mlp_create(noa_dcs_mlp **out, int process, int batch) {
         return mfail(NOA_DCS_ERROR_INVALID_VALUE, "out of host memory");
     m->process = process;
     m->batch = batch;
-    const size_t act = sizeof(float) * (size_t)batch * H;
-    float **acts[] = {&m->Z1, &m->H1, &m->Z2, &m->H2, &m->Z3, &m->H3, &m->D3, &m->D2, &m->D1};
-    e = cudaSuccess;
-    for (float **a : acts)
-        if (e == cudaSuccess)
-            e = cudaMalloc((void **)a, act);
+    e = cudaMalloc((void **)&m->P, sizeof(float) * NPARAM_PAD * 4);
     if (e == cudaSuccess)
-        e = cudaMalloc((void **)&m->P, sizeof(float) * NPARAM_PAD * 4);
+        e = cudaMalloc((void **)&m->Wb, sizeof(__nv_bfloat16) * 6 * H * H);
     if (e == cudaSuccess)
-        e = cudaMalloc((void **)&m->Wb, sizeof(__nv_bfloat16) * 4 * H * H);
-    if (e == cudaSuccess)
-        e = cudaMalloc((void **)&m->Xb, sizeof(float) * (size_t)batch * (IN + 1) + 2 * sizeof(float));
+        e = cudaMalloc((void **)&m->loss, 2 * sizeof(float));
     if (e != cudaSuccess) {
-        for (float **a : acts)
-            cudaFree(*a);
         cudaFree(m->P);
         cudaFree(m->Wb);
-        cudaFree(m->Xb);
+        cudaFree(m->loss);
         delete m;
         return mfail(NOA_DCS_ERROR_CUDA, "model allocation", e);
     }
     m->G = m->P + NPARAM_PAD;  // each block 16-byte aligned (vector atomics on G)
     m->Mm = m->G + NPARAM_PAD;
     m->V = m->Mm + NPARAM_PAD;
-    m->Tb = m->Xb + (size_t)batch * IN;
-    m->loss = m->Tb + batch;
     m->status = reinterpret_cast<unsigned int *>(m->loss + 1);
     cudaMemset(m->P, 0, sizeof(float) * NPARAM_PAD * 4);
     cudaMemset(m->status, 0, sizeof(unsigned int));
-    cudaMemset(m->Wb, 0, sizeof(__nv_bfloat16) * 4 * H * H);
+    cudaMemset(m->Wb, 0, sizeof(__nv_bfloat16) * 6 * H * H);
     *out = m;
     return NOA_DCS_SUCCESS;
 }
@@ -630,7 +710,7 @@ int noa_dcs_mlp_set_params(noa_dcs_mlp *m, const float *params, const float *ada
                    : cudaMemset(m->V, 0, sizeof(float) * NPARAM);
     if (e != cudaSuccess)
         return mfail(NOA_DCS_ERROR_CUDA, "cudaMemcpy(params)", e);
-    mlp_round_weights_kernel<<<64, 256>>>(m->P, m->Wb);
+    mlp_round_weights_kernel<<<UPDATE_CTAS, UPDATE_THREADS>>>(m->P, m->Wb);
     if ((e = cudaDeviceSynchronize()) != cudaSuccess)
         return mfail(NOA_DCS_ERROR_CUDA, "round weights", e);
     m->step = step;
@@ -711,12 +791,10 @@ int noa_dcs_mlp_train(noa_dcs_mlp *m, const float *X, const float *T, int64_t n,
     cudaStream_t s = (cudaStream_t)stream;
     const int B = m->batch;
     const int64_t batches = n / B;
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = clear_gradient(m, s);
     for (int64_t i = 0; i < n_steps && e == cudaSuccess; i++) {
         const int64_t b = (m->step) % batches;
-        mlp_gather_kernel<<<(B + 255) / 256, 256, 0, s>>>(X, T, perm + b * B, m->Xb, m->Tb, B);
-        cudaMemsetAsync(m->loss, 0, sizeof(float), s);
-        if ((e = backward(m, B, s)) != cudaSuccess)
+        if ((e = run_tiles(m, X, T, perm + b * B, B, nullptr, s)) != cudaSuccess)
             break;
         // cosine decay from lr to lr_final over the n_steps of this call
         const double frac = n_steps > 1 ? (double)i / (double)(n_steps - 1) : 0.;
@@ -725,10 +803,8 @@ int noa_dcs_mlp_train(noa_dcs_mlp *m, const float *X, const float *T, int64_t n,
         const float b1 = 0.9f, b2 = 0.999f;
         const float c1 = 1.f / (1.f - std::pow(b1, (float)m->step));
         const float c2 = 1.f / (1.f - std::pow(b2, (float)m->step));
-        mlp_adam_kernel<<<(NPARAM + 255) / 256, 256, 0, s>>>(m->P, m->G, m->Mm, m->V, m->Wb, lr_i, b1, b2, 1e-8f,
-                                                             c1, c2);
-        if (losses)
-            cudaMemcpyAsync(losses + i, m->loss, sizeof(float), cudaMemcpyDeviceToDevice, s);
+        mlp_adam_kernel<<<UPDATE_CTAS, UPDATE_THREADS, 0, s>>>(m->P, m->G, m->Mm, m->V, m->Wb, lr_i, b1, b2, 1e-8f,
+                                                             c1, c2, m->loss, losses ? losses + i : nullptr);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess)
@@ -743,10 +819,10 @@ int noa_dcs_mlp_predict(noa_dcs_mlp *m, const float *X, float *out, int64_t n, v
     if (n > 0 && !device_ok({X, out}))
         return mfail(NOA_DCS_ERROR_NOT_DEVICE_MEMORY, "X and out must be device memory");
     cudaStream_t s = (cudaStream_t)stream;
-    for (int64_t off = 0; off < n; off += m->batch) {
-        const int M = (int)((n - off) < m->batch ? (n - off) : m->batch);
-        cudaMemcpyAsync(m->Xb, X + off * IN, sizeof(float) * IN * M, cudaMemcpyDeviceToDevice, s);
-        const cudaError_t e = forward(m, M, out + off, s);
+    constexpr int64_t most = (int64_t)1 << 24;  // rows of one launch
+    for (int64_t off = 0; off < n; off += most) {
+        const int M = (int)(n - off < most ? n - off : most);
+        const cudaError_t e = run_tiles(m, X + off * IN, nullptr, nullptr, M, out + off, s);
         if (e != cudaSuccess)
             return mfail(NOA_DCS_ERROR_CUDA, "forward", e);
     }
@@ -761,10 +837,9 @@ int noa_dcs_mlp_gradient(noa_dcs_mlp *m, const float *X, const float *T, int n, 
     if (!device_ok({X, T, grad, loss}))
         return mfail(NOA_DCS_ERROR_NOT_DEVICE_MEMORY, "X, T, grad and loss must be device memory");
     cudaStream_t s = (cudaStream_t)stream;
-    cudaMemcpyAsync(m->Xb, X, sizeof(float) * IN * n, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(m->Tb, T, sizeof(float) * n, cudaMemcpyDeviceToDevice, s);
-    cudaMemsetAsync(m->loss, 0, sizeof(float), s);
-    cudaError_t e = backward(m, n, s);
+    cudaError_t e = clear_gradient(m, s);
+    if (e == cudaSuccess)
+        e = run_tiles(m, X, T, nullptr, n, nullptr, s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(grad, m->G, sizeof(float) * NPARAM, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess && loss)
@@ -777,12 +852,9 @@ int noa_dcs_mlp_gradient(noa_dcs_mlp *m, const float *X, const float *T, int n, 
 int noa_dcs_mlp_destroy(noa_dcs_mlp *m) {
     if (!m)
         return NOA_DCS_SUCCESS;
-    float *acts[] = {m->Z1, m->H1, m->Z2, m->H2, m->Z3, m->H3, m->D3, m->D2, m->D1};
-    for (float *a : acts)
-        cudaFree(a);
     cudaFree(m->P);
     cudaFree(m->Wb);
-    cudaFree(m->Xb);
+    cudaFree(m->loss);
     delete m;
     return NOA_DCS_SUCCESS;
 }

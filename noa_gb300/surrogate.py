@@ -181,7 +181,7 @@ class Surrogate:
         epoch_batches = n // self.batch
         # one cosine schedule over all steps, issued in chunks of whole epochs
         while done < steps:
-            perm = torch.randperm(n, generator=g, device="cuda").to(torch.int32)
+            perm = torch.randperm(n, generator=g, device="cuda", dtype=torch.int32)
             todo = min(epoch_batches, steps - done, chunk_steps)
             a = lr_final + 0.5 * (lr - lr_final) * (1 + math.cos(math.pi * done / steps))
             b = lr_final + 0.5 * (lr - lr_final) * (1 + math.cos(math.pi * (done + todo) / steps))
