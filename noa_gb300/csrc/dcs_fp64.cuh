@@ -485,17 +485,6 @@ __device__ __forceinline__ double photo_fp64(double K, double q, const noa_dcs_c
     return photo_finish(K, q, p.hd, sum, c);
 }
 
-// Out-of-line entries of the two quadrature bodies for the FP32C redo paths
-// (FP32C, batched FP32C and surrogate fallback kernels): the redo runs for
-// 0-0.5% of the open pairs, and inlined it would set the register budget of
-// the whole kernel.  Photonuclear's FP32C kernel runs 7% faster with it.
-static __device__ __noinline__ double pprod_fp64_ol(double K, double q, const noa_dcs_consts &c) {
-    return pprod_fp64(K, q, c);
-}
-static __device__ __noinline__ double photo_fp64_ol(double K, double q, const noa_dcs_consts &c) {
-    return photo_fp64(K, q, c);
-}
-
 // ---------------------------------------------------------------- ionisation
 // ionisation's first exit (dcs.hh:413-419: W_max < 5% K or q > W_max),
 // decided in float first: W_max = 2 me K (K + 2 mass) / ((mass + me)^2 +

@@ -76,12 +76,12 @@ struct QuadSmem<NOA_DCS_PROC_ION, B> {};
 
 // Evaluates `take` (1 .. B) open pairs with all threads of the CTA: load(e, K,
 // q) gives pair e, store(e, dcs) takes its value, both called by one thread
-// per pair.  Called by every thread; starts and ends with work that only its
+// per pair; consts(e) are the constants of pair e's element.  Called by every thread; starts and ends with work that only its
 // own pairs' threads see, so the caller synchronises before it changes what
 // load reads and before it reuses the shared memory.
-template <int PROC, int THREADS, int B, typename Load, typename Store>
-__device__ __forceinline__ void quad_batch(QuadSmem<PROC, B> &s, int take, const noa_dcs_consts &c, Load load,
-                                           Store store) {
+template <int PROC, int THREADS, int B, typename Consts, typename Load, typename Store>
+__device__ __forceinline__ void quad_batch_mixed(QuadSmem<PROC, B> &s, int take, Consts consts, Load load,
+                                                 Store store) {
     typedef Quad<PROC> Q;
     typedef QuadSmem<PROC, B> S;
     static_assert(B <= THREADS, "one thread per pair");
@@ -90,7 +90,7 @@ __device__ __forceinline__ void quad_batch(QuadSmem<PROC, B> &s, int take, const
     if (t < take) {
         load(t, K, q);
         typename Q::Pair p;
-        Q::setup(K, q, c, p);
+        Q::setup(K, q, consts(t), p);
         const double *w = reinterpret_cast<const double *>(&p);
 #pragma unroll
         for (int i = 0; i < S::WORDS; i++)
@@ -106,7 +106,7 @@ __device__ __forceinline__ void quad_batch(QuadSmem<PROC, B> &s, int take, const
 #pragma unroll
         for (int i = 0; i < S::WORDS; i++)
             w[i] = s.pair[i][e];
-        s.val[j][e] = Q::node(p, j, c);
+        s.val[j][e] = Q::node(p, j, consts(e));
     }
     __syncthreads();
     if (t < take) {
@@ -119,8 +119,15 @@ __device__ __forceinline__ void quad_batch(QuadSmem<PROC, B> &s, int take, const
 #pragma unroll
         for (int j = 0; j < Q::NODES; j++)
             sum += s.val[j][t];
-        store(t, Q::finish(K, q, p, sum, c));
+        store(t, Q::finish(K, q, p, sum, consts(t)));
     }
+}
+
+// All pairs of one element.
+template <int PROC, int THREADS, int B, typename Load, typename Store>
+__device__ __forceinline__ void quad_batch(QuadSmem<PROC, B> &s, int take, const noa_dcs_consts &c, Load load,
+                                           Store store) {
+    quad_batch_mixed<PROC, THREADS>(s, take, [&](int) -> const noa_dcs_consts & { return c; }, load, store);
 }
 
 // FP64 redo of the FP32C kernels: `take` (1 .. QUAD_REDO) pairs of a queue

@@ -39,6 +39,7 @@
 #include "dcs_fp32c.cuh"
 #include "dcs_fp64.cuh"
 #include "dcs_launch.h"
+#include "dcs_quad.cuh"
 #include "mlp.cuh"
 #include "tcgen05.cuh"
 
@@ -301,96 +302,110 @@ __device__ __forceinline__ void push_index(bool push, int32_t i, uint8_t sg, int
     }
 }
 
+// FP64 evaluation of `take` (1 .. QUAD_REDO) listed pairs by the whole CTA.
+template <int PROC, int THREADS>
+static __device__ __noinline__ void quad_redo_listed(noa_dcs::QuadSmem<PROC, noa_dcs::QUAD_REDO> &s, int take,
+                                                     const InferParams &p, const int32_t *idx, const uint8_t *seg) {
+    noa_dcs::quad_batch_mixed<PROC, THREADS>(
+        s, take, [&](int e) -> const noa_dcs_consts & { return p.consts[seg[e]]; },
+        [&](int e, double &K, double &q) {
+            K = p.K[idx[e]];
+            q = p.q[idx[e]];
+        },
+        [&](int e, double v) { p.out[idx[e]] = v; });
+}
+
 // FP32C evaluation of the fallback list; pairs above the tolerance go to a
-// shared-memory redo queue that full warps drain in FP64, so the FP64 work is
-// proportional to the redo fraction (as in dcs_fp32c.cu).
-// Four CTAs per SM (at most 64 registers; pair production spills 24 bytes
-// and runs 2.7% faster than at three CTAs).
+// shared-memory redo queue that the whole CTA drains in FP64, 32 pairs at a
+// time (as in dcs_fp32c.cu).  With one thread per redo pair every CTA ended in
+// its nodes' serial chain: 4e4 / 4e5 / 4e6 / 1e7 queries over ten elements, all
+// answered here, take 117 / 147 / 550 / 1242 us against 169 / 225 / 820 / 1560
+// (pair production) and 70 / 80 / 234 / 504 against 70 / 83 / 222 / 500
+// (photonuclear, whose redo pairs are 0.1% of the list).
+// One resident grid; a list below one pair per thread of it is spread over
+// all CTAs in equal tiles, a longer one is taken 256 at a time (equal tiles:
+// 158 us and 247 us at 4e5 and 4e6).
+// Four CTAs per SM (at most 64 registers; pair production spills 48 bytes
+// and runs 3% faster at 4e6 than at three CTAs).
+constexpr int FB_THREADS = 256, FB_CTAS = 4;
 template <int PROC>
-__global__ void __launch_bounds__(256, 4) fallback_kernel(const __grid_constant__ InferParams p) {
+__global__ void __launch_bounds__(FB_THREADS, FB_CTAS) fallback_kernel(const __grid_constant__ InferParams p) {
+    using noa_dcs::QUAD_REDO;
     // pair production: redo pairs are evaluated again with the float-float
     // screening log, and the few it still rejects go to a third queue (FP64)
     constexpr bool fine = PROC == NOA_DCS_PAIR_PRODUCTION;
-    __shared__ int32_t rq[512], xq[fine ? 512 : 1];
-    __shared__ uint8_t rs[512], xs[fine ? 512 : 1];
-    __shared__ int rn, xn;
+    constexpr int redo_batch = fine ? FB_THREADS : QUAD_REDO;
+    // a batch left over and one step's pairs
+    __shared__ int32_t rq[redo_batch + FB_THREADS], xq[fine ? QUAD_REDO + FB_THREADS : 1];
+    __shared__ uint8_t rs[redo_batch + FB_THREADS], xs[fine ? QUAD_REDO + FB_THREADS : 1];
+    __shared__ noa_dcs::QuadSmem<PROC, QUAD_REDO> quad;
+    __shared__ int rn_next, xn_next;
     if (threadIdx.x == 0) {
-        rn = 0;
-        xn = 0;
+        rn_next = 0;
+        xn_next = 0;
     }
+    // queue lengths, identical in every thread (counted by the barrier that
+    // ends a step); rn_next and xn_next hand out places
+    int rn = 0, xn = 0;
+    const long long cnt = (long long)p.counters[1];
+    const long long threads = (long long)gridDim.x * FB_THREADS;
+    const long long tile = cnt < threads ? (cnt + gridDim.x - 1) / gridDim.x : FB_THREADS;
+    const long long stride = gridDim.x * tile;
     __syncthreads();
-    const unsigned long long cnt = p.counters[1];
-    for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x; base < cnt;
-         base += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned long long e = base + threadIdx.x;
+    for (long long base = blockIdx.x * tile; base < cnt; base += stride) {
+        const bool last = base + stride >= cnt;
+        const long long e = base + threadIdx.x;
         bool redo = false;
         int32_t i = 0;
         uint8_t sg = 0;
-        if (e < cnt) {
+        if ((int)threadIdx.x < tile && e < cnt) {
             i = p.fb_idx[e];
             sg = p.fb_seg[e];
             const noa_dcs_consts &c = p.consts[sg];
             float est;
             // classify_kernel listed only pairs that the exact bounds leave open
-            const double v = PROC == NOA_DCS_PAIR_PRODUCTION ? noa_dcs::pprod_fp32c<false>(p.K[i], p.q[i], c, est)
-                                                             : noa_dcs::photo_fp32c<false>(p.K[i], p.q[i], c, est);
+            const double v = fine ? noa_dcs::pprod_fp32c<false>(p.K[i], p.q[i], c, est)
+                                  : noa_dcs::photo_fp32c<false>(p.K[i], p.q[i], c, est);
             redo = !(est <= p.tol);
             if (!redo)
                 p.out[i] = v;
         }
-        push_index(redo, i, sg, rq, rs, &rn);
-        __syncthreads();
-        const bool last = base + (unsigned long long)gridDim.x * blockDim.x >= cnt;
-        // one call site each for the redo evaluation and the FP64 one
-        for (;;) {
-            bool did = false;
-            const int n = rn;
-            if (n >= (last ? 1 : 256)) {
-                const int take = n < 256 ? n : 256;
+        push_index(redo, i, sg, rq, rs, &rn_next);
+        rn += __syncthreads_count(redo);
+        // drained below a batch before anything is added again; one call site
+        // each for the redo evaluation and the FP64 one
+        while (rn >= redo_batch || (last && (rn > 0 || xn > 0))) {
+            const int take = rn < redo_batch ? rn : redo_batch;
+            rn -= take;
+            if (threadIdx.x == 0)
+                rn_next = rn;
+            if constexpr (fine) {
                 bool again = false;
                 int32_t j = 0;
                 uint8_t sj = 0;
                 if ((int)threadIdx.x < take) {
-                    const int k = n - take + threadIdx.x;
-                    j = rq[k];
-                    sj = rs[k];
-                    const noa_dcs_consts &c = p.consts[sj];
-                    if (fine) {
-                        float est;
-                        const double v = noa_dcs::pprod_fp32c<false, true>(p.K[j], p.q[j], c, est);
-                        again = !(est <= p.tol);
-                        if (!again)
-                            p.out[j] = v;
-                    } else {
-                        p.out[j] = noa_dcs::photo_fp64_ol(p.K[j], p.q[j], c);
-                    }
+                    j = rq[rn + threadIdx.x];
+                    sj = rs[rn + threadIdx.x];
+                    float est;
+                    const double v = noa_dcs::pprod_fp32c<false, true>(p.K[j], p.q[j], p.consts[sj], est);
+                    again = !(est <= p.tol);
+                    if (!again)
+                        p.out[j] = v;
                 }
-                if (fine)
-                    push_index(again, j, sj, xq, xs, &xn);
-                __syncthreads();
-                if (threadIdx.x == 0)
-                    rn = n - take;
-                __syncthreads();
-                did = true;
-            }
-            if (fine) {
-                const int nx = xn;
-                if (nx >= 256 || (last && rn == 0 && nx > 0)) {
-                    const int take = nx < 256 ? nx : 256;
-                    if ((int)threadIdx.x < take) {
-                        const int k = nx - take + threadIdx.x;
-                        const int32_t j = xq[k];
-                        p.out[j] = noa_dcs::pprod_fp64_ol(p.K[j], p.q[j], p.consts[xs[k]]);
-                    }
-                    __syncthreads();
+                push_index(again, j, sj, xq, xs, &xn_next);
+                xn += __syncthreads_count(again);
+                while (xn >= QUAD_REDO || (last && rn == 0 && xn > 0)) {
+                    const int some = xn < QUAD_REDO ? xn : QUAD_REDO;
+                    xn -= some;
                     if (threadIdx.x == 0)
-                        xn = nx - take;
+                        xn_next = xn;
+                    quad_redo_listed<PROC, FB_THREADS>(quad, some, p, xq + xn, xs + xn);
                     __syncthreads();
-                    did = true;
                 }
+            } else {
+                quad_redo_listed<PROC, FB_THREADS>(quad, take, p, rq + rn, rs + rn);
+                __syncthreads();
             }
-            if (!did)
-                break;
         }
     }
 }
@@ -755,9 +770,9 @@ extern "C" int noa_dcs_mlp_infer(noa_dcs_mlp *model, const uint8_t *trust, int n
     }
     if (e == cudaSuccess) {
         if (process == NOA_DCS_PAIR_PRODUCTION)
-            fallback_kernel<NOA_DCS_PAIR_PRODUCTION><<<sms * 8, 256, 0, s>>>(p);
+            fallback_kernel<NOA_DCS_PAIR_PRODUCTION><<<sms * FB_CTAS, FB_THREADS, 0, s>>>(p);
         else
-            fallback_kernel<NOA_DCS_PHOTONUCLEAR><<<sms * 8, 256, 0, s>>>(p);
+            fallback_kernel<NOA_DCS_PHOTONUCLEAR><<<sms * FB_CTAS, FB_THREADS, 0, s>>>(p);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && stats)
