@@ -76,8 +76,8 @@ typedef struct noa_dcs_consts {
     double pp_inv_AZ13;     /* 1 / AZ13 */
     double pp_2sm;          /* 2 sqrte me = cL / AZ13 */
     double pp_kappa;        /* 1.5 Z13 / r */
-    double pp_2_inv_r2;     /* 2 / (r r) */
     double pp_cZs;          /* cZ scale_A */
+    int64_t pp_log_kappa_fx; /* log kappa in units of 2^-57; INT64_MIN where it is not within 18 */
 
     /* photonuclear, dcs.hh:310-319, 370-375 */
     double ph_logA;         /* log(A) */
@@ -89,6 +89,8 @@ typedef struct noa_dcs_consts {
     double ph_scale_A;      /* ph_scale A */
     double ph_k1, ph_k0;    /* DRSS exponent (0.069 log10 x + 0.097) log A = k1 log x + k0 */
     double ph_m2;           /* mass mass */
+    int64_t ph_k1_fx;       /* k1 and -0.1 log A in units of 2^-57 (0 where k1 is not below 1) */
+    int64_t ph_log_a_low_fx;
 
     /* ionisation, dcs.hh:408-443 */
     double io_Wmin;         /* 0.62 I */
@@ -175,8 +177,9 @@ static inline void noa_dcs_fill_consts(noa_dcs_consts *c, double A, double I, in
         c->pp_inv_AZ13 = Z13 / A_;
         c->pp_2sm = 2. * sqrte * me;
         c->pp_kappa = 1.5 * Z13 / r;
-        c->pp_2_inv_r2 = 2. / (r * r);
         c->pp_cZs = c->pp_cZ * c->scale_A;
+        const double log_kappa = log(c->pp_kappa);
+        c->pp_log_kappa_fx = fabs(log_kappa) < 18. ? (int64_t)(log_kappa * 0x1p57) : INT64_MIN;
     }
     { // dcs.hh:290, 313-315, 370-374
         const double M = 0.931494, mpi = 0.134977;
@@ -191,6 +194,10 @@ static inline void noa_dcs_fill_consts(noa_dcs_consts *c, double A, double I, in
         c->ph_k1 = 0.069 * 0.43429448190325182765 * c->ph_logA;
         c->ph_k0 = 0.097 * c->ph_logA;
         c->ph_m2 = mass * mass;
+        if (fabs(c->ph_k1) < 1.) {
+            c->ph_k1_fx = (int64_t)(c->ph_k1 * 0x1p57);
+            c->ph_log_a_low_fx = (int64_t)(-0.1 * c->ph_logA * 0x1p57);
+        }
     }
     { // dcs.hh:422, 435-436
         c->io_Wmin = 0.62 * I;

@@ -42,19 +42,19 @@ constexpr int MAP_MIN_CTAS = 10;
 // SM, 1e6 pairs 69 / 52 against 72 / 53).
 constexpr int MAP_GRID_CTAS = 1000;
 constexpr int CMP_THREADS = 128;
-constexpr int CMP_ITEMS = 2;
+constexpr int CMP_ITEMS = 1;  // 2 items' queue takes the shared memory of the last resident CTA: 1% slower
 constexpr int CMP_TILE = CMP_THREADS * CMP_ITEMS;  // largest tile
 constexpr int CMP_QCAP = CMP_TILE + CMP_THREADS;
 
 // Resident CTAs per SM that the compacting kernels are compiled for (the
 // register budget per thread follows) and their grid is made of.  Measured at
-// 1e7 pairs: pair production 5.13 / 5.06 / 5.07 ms at 4 / 5 / 6; photonuclear
-// 2.56 / 2.49 / 2.45 / 2.48 ms at 5 / 6 / 7 / 8.
+// 1e7 pairs: pair production 3.44 / 3.34 / 3.36 ms at 5 / 6 / 7; photonuclear
+// 1.96 / 1.94 / 1.92 ms at 6 / 7 / 8 (the most that shared memory holds).
 #ifndef NOA_DCS_PPROD_MIN_CTAS
-#define NOA_DCS_PPROD_MIN_CTAS 5
+#define NOA_DCS_PPROD_MIN_CTAS 6
 #endif
 #ifndef NOA_DCS_PHOTO_MIN_CTAS
-#define NOA_DCS_PHOTO_MIN_CTAS 7
+#define NOA_DCS_PHOTO_MIN_CTAS 8
 #endif
 template <int PROC>
 constexpr int cmp_min_ctas() {

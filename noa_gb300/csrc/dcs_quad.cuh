@@ -36,6 +36,7 @@ struct Quad<NOA_DCS_PROC_PPROD> {
     static __device__ __forceinline__ double node(const Pair &p, int j, const noa_dcs_consts &c) {
         return pprod_node(p, j, c);
     }
+    static __device__ __forceinline__ double weight(int j) { return kGL8W[j]; }
     static __device__ __forceinline__ double finish(double K, double q, const Pair &p, double sum,
                                                     const noa_dcs_consts &c) {
         return pprod_finish(K, q, p.tmin, sum, c);
@@ -52,6 +53,7 @@ struct Quad<NOA_DCS_PROC_PHOTO> {
     static __device__ __forceinline__ double node(const Pair &p, int j, const noa_dcs_consts &c) {
         return photo_node(p, j, c);
     }
+    static __device__ __forceinline__ double weight(int j) { return kGL9W[j]; }
     static __device__ __forceinline__ double finish(double K, double q, const Pair &p, double sum,
                                                     const noa_dcs_consts &c) {
         return photo_finish(K, q, p.hd, sum, c);
@@ -118,7 +120,7 @@ __device__ __forceinline__ void quad_batch_mixed(QuadSmem<PROC, B> &s, int take,
         double sum = 0.;
 #pragma unroll
         for (int j = 0; j < Q::NODES; j++)
-            sum += s.val[j][t];
+            sum = fma(Q::weight(j), s.val[j][t], sum);
         store(t, Q::finish(K, q, p, sum, consts(t)));
     }
 }

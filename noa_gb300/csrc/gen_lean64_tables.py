@@ -87,6 +87,10 @@ def main():
     out.append("/* ln 2 = LN2_H 2^-31 + LN2_L 2^-63 */")
     out.append(f"#define LEAN64_LN2_H {ln2_h}")
     out.append(f"#define LEAN64_LN2_L {ln2_l}")
+    out.append("/* ln 2 in units of 2^-57 */")
+    out.append(f"#define LEAN64_LN2_57 {int(mpmath.nint(ln2 * mpmath.mpf(2) ** 57))}LL")
+    out.append("/* 128 / ln 2 in units of 2^-22 */")
+    out.append(f"#define LEAN64_INV_LN2N_22 {int(mpmath.nint(EXP_N / ln2 * 2 ** 22))}")
     out.append("/* ln 2 / 128 = K_H 2^-31 + K_M 2^-63 + K_L 2^-95 */")
     out.append(f"#define LEAN64_K_H {k_h}")
     out.append(f"#define LEAN64_K_M {k_m}")

@@ -111,6 +111,10 @@ __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ int clz32(unsigned x) { return __clz((int)x); }
 __device__ __forceinline__ float i2f(int i) { return __int2float_rn(i); }
 __device__ __forceinline__ unsigned mulhi_s(int a, int b) { return (unsigned)__mulhi(a, b); }
+__device__ __forceinline__ unsigned long long mulhi_u64(unsigned long long a, unsigned long long b) {
+    return __umul64hi(a, b);
+}
+__device__ __forceinline__ long long mulhi_s64(long long a, long long b) { return __mul64hi(a, b); }
 __device__ __forceinline__ longlong2 log_entry(int t) { return __ldg(&lean64_log_tab[t]); }
 __device__ __forceinline__ long long exp_entry(int j) { return __ldg(&lean64_exp_t[j]); }
 #elif defined(LEAN64_HOST_TABLES)
@@ -124,6 +128,10 @@ inline float fmul(float a, float b) { return a * b; }
 inline int clz32(unsigned x) { return __builtin_clz(x); }
 inline float i2f(int i) { return (float)i; }
 inline unsigned mulhi_s(int a, int b) { return (unsigned)(((long long)a * b) >> 32); }
+inline unsigned long long mulhi_u64(unsigned long long a, unsigned long long b) {
+    return (unsigned long long)(((unsigned __int128)a * b) >> 64);
+}
+inline long long mulhi_s64(long long a, long long b) { return (long long)(((__int128)a * b) >> 64); }
 inline longlong2 log_entry(int t) { return lean64_log_tab_host[t]; }
 inline long long exp_entry(int j) { return lean64_exp_t_host[j]; }
 #endif
@@ -179,32 +187,8 @@ LEAN64_FN void fix_parts(float dh, float dl, float scale, float magic, unsigned 
     b2 = f2u(fmaf(g, 4194304.f, 12582912.f));
 }
 
-} // namespace detail
-
-// log x with no FP64 instruction.  x = 2^e m, m in [0.707, 1.414) (bin t of
-// the top 9 mantissa bits, halved above sqrt 2), c_t ~ 1/m:
-//   r = m c - 1 = R 2^-64          exact: one integer product modulo 2^64
-//   d = log1p(r) - r               float-float, ~2^-47 relative; r enters as
-//                                  rh + rl, the two words of R
-//   log x = e ln2 - log c + r + d  64-bit fixed point: 2^-64 for e = 0, 2^-58
-//                                  for |e| <= 15, 2^-51 beyond (|log x| >= 2^-9,
-//                                  0.34 and 10.7: a few units of 2^-55 relative)
-// rounded once to double.  In [1 - 2^-9, 1 + 2^-9) c = 1 and the scale
-// follows r (log x = r + d), so log x keeps full relative accuracy at
-// x = 1 +- 2^-53.
-LEAN64_FN double lean_log(double x) {
-    using namespace detail;
-    const long long b = d2ll(x);
-    const unsigned hi = (unsigned)((unsigned long long)b >> 32);
-    // positive, normal and finite?
-    if (hi - 0x00100000u >= 0x7FE00000u)
-        return log(x);
-    const int e = (int)(hi + ((512u - LEAN64_LOG_SPLIT) << 11) - 0x3FF00000u) >> 20;  // bins above the split carry
-    const bool near1 = hi - 0x3FEFF000u < 0x1800u;
-    const longlong2 ent = log_entry((hi >> 11) & 0x1FFu);  // {c_t, L_t}, one 16-byte load
-    const unsigned C = near1 ? (hi < 0x3FF00000u ? 2048u : 4096u) : (unsigned)ent.x;
-    const unsigned long long M = ((unsigned long long)((hi & 0x000FFFFFu) | 0x00100000u) << 32) | (unsigned)b;
-    const long long R = (long long)(M * C);
+// d = log1p(r) - r as dh + dl, r = R 2^-64, |r| < 2^-9.
+LEAN64_FN void log_tail(long long R, float &dh, float &dl) {
     // r = rh + rl: the high word rounded and the signed low word, renormalised
     const float rw = fmul(i2f((int)((R + 0x80000000ll) >> 32)), 0x1p-32f);
     const float rv = fmul(i2f((int)(unsigned)R), 0x1p-64f);
@@ -225,49 +209,22 @@ LEAN64_FN double lean_log(double x) {
     const float uh = fmul(ch, wh);
     const float ul = fmaf(ch, wl, fmaf(cl, wh, fmaf(ch, wh, -uh)));
     const float hs = fmul(-0.5f, sh);
-    const float dh = fadd(hs, uh);
-    const float dl = fadd(fadd(uh, -fadd(dh, -hs)), fmaf(-0.5f, sl, ul));
-    if (near1) {
-        if (R == 0)
-            return 0.0;
-        const unsigned long long A = R < 0 ? 0ull - (unsigned long long)R : (unsigned long long)R;
-        const int lz = clz64(A);  // |r| < 2^-9: lz >= 9
-        const int F = 62 + lz;
-        const long long Sr = (long long)(A << (lz - 2));
-        return fix_to_double((R < 0 ? -Sr : Sr) + fix_from_float(dh, F) + fix_from_float(dl, F), F);
-    }
-    unsigned b1, b2;
-    fix_parts(dh, dl, 0x1p42f, 16777215.f, b1, b2);  // -2^-19.9 < d <= 0
-    const long long T = R + (long long)((unsigned long long)ent.y + (unsigned long long)b1 * 0x400000ull + b2);
-    const int s = e == 0 ? 0 : ((unsigned)(e + 15) <= 30u ? 6 : 13);
-    const long long Q = T + (long long)e * (2ll * LEAN64_LN2_L);
-    const long long Z = (long long)(int)((unsigned)e << ((33 - s) & 31)) * LEAN64_LN2_H + (Q >> s);
-    return fix_wide_to_double(Z, 64 - s);
+    dh = fadd(hs, uh);
+    dl = fadd(fadd(uh, -fadd(dh, -hs)), fmaf(-0.5f, sl, ul));
 }
 
-// exp x with no FP64 instruction.  k = round(x 128 / ln2) from a float,
-// 2^(k/128) = 2^k' T_j:
-//   r = x - k ln2 / 128            64-bit fixed point, 2^-63, modulo 2^64
-//   d = expm1(r) - r               float-float, ~2^-47 relative
-//   exp x = 2^k' T_j (1 + r + d)   integer products, rounded once
-LEAN64_FN double lean_exp(double x) {
-    using namespace detail;
-    const long long b = d2ll(x);
-    const unsigned hi = (unsigned)((unsigned long long)b >> 32), a = hi & 0x7FFFFFFFu;
-    if (a >= 0x4085E000u)  // |x| >= 700, inf, NaN
-        return exp(x);
-    // |x| as a float, cut to 24 bits (2^-126 for what is smaller), with x's sign
-    const unsigned am = a > 0x38100000u ? a : 0x38100000u;
-    const float xf = u2f((((am << 3) | ((unsigned)b >> 29)) - (896u << 23)) | (hi & 0x80000000u));
-    const int k = (int)(f2u(fmaf(xf, (float)LEAN64_INV_LN2N, 12582912.f)) - 0x4B400000u);
-    // x in units of 2^-63 modulo 2^64 (the high bits cancel in r; below 2^-11 cut at 2^-63)
-    const unsigned long long M = (((unsigned long long)b) & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
-    const int n = (int)(a >> 20) - 1012;  // -1012 .. 20
-    const unsigned long long X = n >= 0 ? M << n : M >> (n < -63 ? 63 : -n);
-    const long long sx = (long long)(int)hi >> 63;
-    const long long r = (((long long)X ^ sx) - sx) -
-                        ((long long)k * LEAN64_K_M + (long long)((unsigned long long)(long long)(k * LEAN64_K_H) << 32) +
-                         (int)mulhi_s(k, LEAN64_K_L));
+// log of the table bin's m (see lean_log) from R and the bin's L, in units of 2^-64.
+LEAN64_FN long long log_bin(long long R, long long L) {
+    float dh, dl;
+    log_tail(R, dh, dl);
+    unsigned b1, b2;
+    fix_parts(dh, dl, 0x1p42f, 16777215.f, b1, b2);  // -2^-19.9 < d <= 0
+    return R + (long long)((unsigned long long)L + (unsigned long long)b1 * 0x400000ull + b2);
+}
+
+// exp: T_j (1 + expm1 r) in units of 2^-61, in [2^61, 2^62), for k = 128 k' + j
+// and r = R 2^-63, |r| < 2^-8.4; q = k' or, where T_0 (1 + expm1 r) < 1, k' - 1.
+LEAN64_FN unsigned long long exp_bin(int k, long long r, int &q) {
     // r = rh + rl: the high word rounded and the signed low word
     const float rh = fmul(i2f((int)((r + 0x80000000ll) >> 32)), 0x1p-31f);
     const float rl = fmul(i2f((int)(unsigned)r), 0x1p-63f);
@@ -297,8 +254,80 @@ LEAN64_FN double lean_exp(double x) {
     const long long U = T + (long long)Th * ph + (long long)(V >> 32) - 0x01000000ll;
     // T_0 (1 + p) may lie below 1
     const int low = (int)(U >> 32) < 0x20000000 ? 1 : 0;
-    const unsigned long long m = (((unsigned long long)U << low) + 0x100ull) >> 9;  // leading bit at 52
-    return ll2d((long long)(((unsigned long long)((k >> 7) - low + 1022) << 52) + m));
+    q = (k >> 7) - low;
+    return (unsigned long long)U << low;
+}
+
+} // namespace detail
+
+// log x with no FP64 instruction.  x = 2^e m, m in [0.707, 1.414) (bin t of
+// the top 9 mantissa bits, halved above sqrt 2), c_t ~ 1/m:
+//   r = m c - 1 = R 2^-64          exact: one integer product modulo 2^64
+//   d = log1p(r) - r               float-float, ~2^-47 relative; r enters as
+//                                  rh + rl, the two words of R
+//   log x = e ln2 - log c + r + d  64-bit fixed point: 2^-64 for e = 0, 2^-58
+//                                  for |e| <= 15, 2^-51 beyond (|log x| >= 2^-9,
+//                                  0.34 and 10.7: a few units of 2^-55 relative)
+// rounded once to double.  In [1 - 2^-9, 1 + 2^-9) c = 1 and the scale
+// follows r (log x = r + d), so log x keeps full relative accuracy at
+// x = 1 +- 2^-53.
+LEAN64_FN double lean_log(double x) {
+    using namespace detail;
+    const long long b = d2ll(x);
+    const unsigned hi = (unsigned)((unsigned long long)b >> 32);
+    // positive, normal and finite?
+    if (hi - 0x00100000u >= 0x7FE00000u)
+        return log(x);
+    const int e = (int)(hi + ((512u - LEAN64_LOG_SPLIT) << 11) - 0x3FF00000u) >> 20;  // bins above the split carry
+    const bool near1 = hi - 0x3FEFF000u < 0x1800u;
+    const longlong2 ent = log_entry((hi >> 11) & 0x1FFu);  // {c_t, L_t}, one 16-byte load
+    const unsigned C = near1 ? (hi < 0x3FF00000u ? 2048u : 4096u) : (unsigned)ent.x;
+    const unsigned long long M = ((unsigned long long)((hi & 0x000FFFFFu) | 0x00100000u) << 32) | (unsigned)b;
+    const long long R = (long long)(M * C);
+    if (near1) {
+        if (R == 0)
+            return 0.0;
+        float dh, dl;
+        log_tail(R, dh, dl);
+        const unsigned long long A = R < 0 ? 0ull - (unsigned long long)R : (unsigned long long)R;
+        const int lz = clz64(A);  // |r| < 2^-9: lz >= 9
+        const int F = 62 + lz;
+        const long long Sr = (long long)(A << (lz - 2));
+        return fix_to_double((R < 0 ? -Sr : Sr) + fix_from_float(dh, F) + fix_from_float(dl, F), F);
+    }
+    const long long T = log_bin(R, ent.y);
+    const int s = e == 0 ? 0 : ((unsigned)(e + 15) <= 30u ? 6 : 13);
+    const long long Q = T + (long long)e * (2ll * LEAN64_LN2_L);
+    const long long Z = (long long)(int)((unsigned)e << ((33 - s) & 31)) * LEAN64_LN2_H + (Q >> s);
+    return fix_wide_to_double(Z, 64 - s);
+}
+
+// exp x with no FP64 instruction.  k = round(x 128 / ln2) from a float,
+// 2^(k/128) = 2^k' T_j:
+//   r = x - k ln2 / 128            64-bit fixed point, 2^-63, modulo 2^64
+//   d = expm1(r) - r               float-float, ~2^-47 relative
+//   exp x = 2^k' T_j (1 + r + d)   integer products, rounded once
+LEAN64_FN double lean_exp(double x) {
+    using namespace detail;
+    const long long b = d2ll(x);
+    const unsigned hi = (unsigned)((unsigned long long)b >> 32), a = hi & 0x7FFFFFFFu;
+    if (a >= 0x4085E000u)  // |x| >= 700, inf, NaN
+        return exp(x);
+    // |x| as a float, cut to 24 bits (2^-126 for what is smaller), with x's sign
+    const unsigned am = a > 0x38100000u ? a : 0x38100000u;
+    const float xf = u2f((((am << 3) | ((unsigned)b >> 29)) - (896u << 23)) | (hi & 0x80000000u));
+    const int k = (int)(f2u(fmaf(xf, (float)LEAN64_INV_LN2N, 12582912.f)) - 0x4B400000u);
+    // x in units of 2^-63 modulo 2^64 (the high bits cancel in r; below 2^-11 cut at 2^-63)
+    const unsigned long long M = (((unsigned long long)b) & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
+    const int n = (int)(a >> 20) - 1012;  // -1012 .. 20
+    const unsigned long long X = n >= 0 ? M << n : M >> (n < -63 ? 63 : -n);
+    const long long sx = (long long)(int)hi >> 63;
+    const long long r = (((long long)X ^ sx) - sx) -
+                        ((long long)k * LEAN64_K_M + (long long)((unsigned long long)(long long)(k * LEAN64_K_H) << 32) +
+                         (int)mulhi_s(k, LEAN64_K_L));
+    int q;
+    const unsigned long long m = (exp_bin(k, r, q) + 0x100ull) >> 9;  // leading bit at 52
+    return ll2d((long long)(((unsigned long long)(q + 1022) << 52) + m));
 }
 
 // 1/b with no FP64 instruction.  b = +-2^E m, m = M 2^-52 in [1, 2);
@@ -324,6 +353,145 @@ LEAN64_FN double lean_rcp(double b) {
     const unsigned long long m = (unsigned long long)((C >> 30) + ((long long)Y << 30));  // 1/m in units of 2^-53
     const unsigned mh = (unsigned)(m >> 32) + 0x7FC00000u - (hi & 0xFFF00000u);
     return ll2d((long long)(((unsigned long long)mh << 32) | (unsigned)m));
+}
+
+// ---------------------------------------------------------------- fixed point
+// Values between elementary functions as 64-bit integers in units of 2^-57
+// (|v| < 64): the functions above spend a third of their instructions on
+// taking doubles apart and putting them together, and a product or a sum
+// between two of them is an FP64 instruction, 16 clocks of its pipe, where 64-bit
+// integer sums and products take 1 - 5 of the integer pipes.  The caller
+// keeps arguments in range.
+
+// The literal x in units of 2^-F.
+__host__ __device__ constexpr long long fx_const(double x, int F = 57) { return (long long)(x * (double)(1ull << F)); }
+
+// a b 2^-F, rounded down: units of 2^-F times another unit.
+LEAN64_FN long long fx_mul(long long a, long long b, int F = 57) {
+    const unsigned long long lo = (unsigned long long)a * (unsigned long long)b;
+    return (long long)(((unsigned long long)detail::mulhi_s64(a, b) << (64 - F)) | (lo >> F));
+}
+
+// log x, x positive, normal and finite; to about 2^-57 absolute.
+LEAN64_FN long long lean_log_fx(double x) {
+    using namespace detail;
+    const long long b = d2ll(x);
+    const unsigned hi = (unsigned)((unsigned long long)b >> 32);
+    const int e = (int)(hi + ((512u - LEAN64_LOG_SPLIT) << 11) - 0x3FF00000u) >> 20;
+    const longlong2 ent = log_entry((hi >> 11) & 0x1FFu);
+    const unsigned long long M = ((unsigned long long)((hi & 0x000FFFFFu) | 0x00100000u) << 32) | (unsigned)b;
+    return (log_bin((long long)(M * (unsigned)ent.x), ent.y) >> 7) + (long long)e * LEAN64_LN2_57;
+}
+
+// log(N 2^E), N with its leading bit at 63 (taken as its top 53 bits and the
+// middle of the rest: 2^-54 relative).
+LEAN64_FN long long log_wide_fx(unsigned long long N, int E) {
+    using namespace detail;
+    const unsigned hi = (unsigned)(N >> 43);  // 1 and 20 mantissa bits
+    const longlong2 ent = log_entry((hi >> 11) & 0x1FFu);
+    const unsigned C = (unsigned)ent.x;
+    const int e = 63 + E + (int)((hi + ((512u - LEAN64_LOG_SPLIT) << 11)) >> 21);
+    return (log_bin((long long)((N >> 11) * C + (C >> 1)), ent.y) >> 7) + (long long)e * LEAN64_LN2_57;
+}
+
+// log(3 + x), x positive and normal.
+LEAN64_FN long long lean_log3p_fx(double x) {
+    using namespace detail;
+    const unsigned long long b = (unsigned long long)d2ll(x);
+    const int ex = (int)(b >> 52) - 1023;
+    const unsigned long long B = ((b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << 9;  // 2^-61 at x = 1
+    const unsigned long long A = 0x6000000000000000ull;                                       // 3
+    const int n = ex < 0 ? -ex : ex, sh = n > 63 ? 63 : n;
+    const unsigned long long Y = (ex > 0 ? B : A) + ((ex > 0 ? A : B) >> sh);
+    const int lz = clz32((unsigned)(Y >> 32));
+    return log_wide_fx(Y << lz, (ex > 0 ? ex : 0) - 61 - lz);
+}
+
+// log of a fixed-point value, v > 0.
+LEAN64_FN long long log_of_fx(long long v) {
+    const int lz = detail::clz64((unsigned long long)v);
+    return log_wide_fx((unsigned long long)v << lz, -57 - lz);
+}
+
+// exp of a fixed-point value: k and r of lean_exp.
+LEAN64_FN unsigned long long exp_fx_bin(long long x, int &q) {
+    using namespace detail;
+    const int k = (int)(((long long)(int)(x >> 32) * LEAN64_INV_LN2N_22 + (1ll << 46)) >> 47);
+    const long long r = (long long)((unsigned long long)x << 6) -
+                        ((long long)k * LEAN64_K_M + (long long)((unsigned long long)(long long)(k * LEAN64_K_H) << 32) +
+                         (int)mulhi_s(k, LEAN64_K_L));
+    return exp_bin(k, r, q);
+}
+LEAN64_FN double lean_exp_fx(long long x) {
+    int q;
+    const unsigned long long m = (exp_fx_bin(x, q) + 0x100ull) >> 9;
+    return detail::ll2d((long long)(((unsigned long long)(q + 1022) << 52) + m));
+}
+// exp x as a fixed-point value, x < log 64.
+LEAN64_FN long long exp_to_fx(long long x) {
+    int q;
+    const unsigned long long U = exp_fx_bin(x, q);  // U 2^(q - 61)
+    const int sh = 5 - q;
+    return (long long)((U << 1) >> (sh > 63 ? 63 : sh));
+}
+
+// 1/m of D = m 2^63 (leading bit at 63) in units of 2^-62, in (2^61, 2^62], to
+// about 2^-60: lean_rcp's steps with the residual of all 64 bits.
+LEAN64_FN unsigned long long rcp_wide(unsigned long long D) {
+    using namespace detail;
+    const float m1 = u2f(((unsigned)(D >> 40) & 0x007FFFFFu) | 0x3F800000u);
+    const unsigned Y = f2u(fadd(rcp_approx(m1), 1.f)) - 0x3F800000u;
+    const long long N = (long long)((D >> 11) * Y) + (long long)((((unsigned)D & 0x7FFu) * (unsigned long long)Y) >> 11);
+    const int nh = (int)(N >> 32);
+    const long long c = (N - (long long)((unsigned long long)((long long)nh * nh) >> 11) + 0x4000ll) >> 15;
+    return (unsigned long long)(((long long)Y << 39) - ((c * (long long)Y) >> 21));
+}
+
+// A fixed-point value as a double, |v| >= 2^-25.
+LEAN64_FN double from_fx(long long v, int F = 57) { return detail::fix_wide_to_double(v, F); }
+// The same for any v (the last bit of the magnitude is lost).
+LEAN64_FN double from_fx_any(long long v, int F = 57) {
+    const unsigned long long U = (unsigned long long)(v ^ (v >> 63)) | 1ull;
+    const int lz = detail::clz64(U) - 1;  // |v| < 2^63
+    const unsigned long long m = ((U << lz) + 0x200ull) >> 10;
+    return detail::ll2d((long long)((((unsigned long long)(1084 - lz - F) << 52) + m) |
+                                    ((unsigned long long)v & 0x8000000000000000ull)));
+}
+
+// N / D as a double, 0 < N, D < 2^63 in the same units, to 0.5 ulp and a little.
+LEAN64_FN double ratio_fx(unsigned long long N, unsigned long long D) {
+    using namespace detail;
+    const int ln = clz64(N), ld = clz64(D);
+    return fix_wide_to_double((long long)mulhi_u64(N << ln, rcp_wide(D << ld)), 61 - ld + ln);
+}
+
+// A double in [0, 1] in units of 2^-62; |x| < 2^(62 - F) in units of 2^-F,
+// rounded down in magnitude.
+LEAN64_FN unsigned long long unit_to_fx62(double x) {
+    const unsigned long long b = (unsigned long long)detail::d2ll(x);
+    const int sh = 1023 - (int)(b >> 52);
+    const unsigned long long M = ((b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << 10;
+    return M >> (sh > 63 ? 63 : sh);
+}
+LEAN64_FN long long to_fx(double x, int F) {
+    const unsigned long long b = (unsigned long long)detail::d2ll(x);
+    const int n = ((int)(b >> 52) & 0x7FF) - 1075 + F;
+    const unsigned long long M = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
+    const unsigned long long v = n >= 0 ? M << (n & 63) : M >> (n < -63 ? 63 : -n);
+    return (long long)b < 0 ? -(long long)v : (long long)v;
+}
+
+// 1 - (1 - x) with both subtractions rounded, 0 < x <= 1: x rounded to a
+// multiple of 2^-53 (half to even), on the bits of x.
+LEAN64_FN double round_by_one(double x) {
+    const unsigned long long b = (unsigned long long)detail::d2ll(x);
+    const int sh = 1022 - (int)(b >> 52);  // bits below 2^-53
+    if (sh <= 0)
+        return x;
+    if (sh > 52)
+        return sh > 53 || (sh == 53 && (b & 0x000FFFFFFFFFFFFFull) == 0) ? 0.0 : 0x1p-53;
+    const unsigned long long unit = 1ull << sh, lsb = (((b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) >> sh) & 1ull;
+    return detail::ll2d((long long)((b + (unit >> 1) - 1ull + lsb) & ~(unit - 1ull)));
 }
 
 LEAN64_FN double lean_div(double a, double b) { return a * lean_rcp(b); }
