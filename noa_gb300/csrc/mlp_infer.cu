@@ -8,8 +8,6 @@
  *     the trained domain whose cell passed the held-out error check go to the
  *     network list; the others to the fallback list (both in the model's
  *     scratch, positions from block-wide scans).
- *     Then netprep: the float baseline of mlp.cuh for each listed pair,
- *     densely over the list.
  *  2. network (tcgen05): a persistent CTA of four warpgroups keeps two tiles
  *     of 128 listed pairs in flight, two warpgroups each, so that the tensor
  *     core works on one tile while the CUDA cores run the other's SiLU
@@ -26,7 +24,8 @@
  *     mbarrier; the epilogue reads the accumulator with tcgen05.ld, adds the
  *     bias and applies SiLU.  TMEM per tile: accumulator 128 columns, A hi 64,
  *     A lo 64 (512 for the two).
- *     DCS = exp(baseline + residual), in float (1e-6 relative).
+ *     DCS = exp(baseline + residual), in float (1e-6 relative); the float
+ *     baseline of mlp.cuh is computed while the first MMAs run.
  *  3. fallback: the FP32C evaluation (dcs_fp32c.cuh) of the fallback list,
  *     with FP64 (dcs_fp64.cuh) for pairs above its tolerance (pair
  *     production: after a second FP32 pass with the float-float screening
@@ -76,7 +75,6 @@ struct InferParams {
     float logk_lo, logk_scale, lognu_lo, lognu_scale;  // cell = floor((log - lo) * scale)
     // lists
     int32_t *net_idx;
-    float *net_base;
     float4 *net_feat;
     int32_t *fb_idx;
     uint8_t *fb_seg;
@@ -108,7 +106,11 @@ __device__ __forceinline__ void append(unsigned long long *counter, bool flag, i
 //     atomicAdd per list per tile.
 // Only open pairs (20% for photonuclear, 54% for pair production on the
 // benchmark law) pay for features.
-constexpr int CL_THREADS = 256, CL_ITEMS = 4, CL_TILE = CL_THREADS * CL_ITEMS;
+// 512 pairs a tile, eight CTAs an SM (32 registers: this phase waits for memory
+// and for the lists' counters): 4e6 queries with 6% of the cells trusted 604 ->
+// 591 us (pair production) and 266 -> 263 us (photonuclear) against four
+// pairs a thread, 4e4 135 -> 128 and 83 -> 81.
+constexpr int CL_THREADS = 256, CL_ITEMS = 2, CL_TILE = CL_THREADS * CL_ITEMS, CL_CTAS = 8;
 
 // Exclusive block-wide scan of two counts (256 threads); returns this
 // thread's offsets and writes the totals to *tot_a, *tot_b (shared).
@@ -147,11 +149,11 @@ __device__ __forceinline__ void block_scan2(int ca, int cb, int &oa, int &ob, in
 }
 
 template <int PROC>
-__global__ void __launch_bounds__(CL_THREADS) classify_kernel(const __grid_constant__ InferParams p) {
+__global__ void __launch_bounds__(CL_THREADS, CL_CTAS) classify_kernel(const __grid_constant__ InferParams p) {
     __shared__ int warp_a[CL_THREADS / 32], warp_b[CL_THREADS / 32];
     __shared__ int tot_a, tot_b;
     __shared__ unsigned long long base_n, base_f;
-    // per-warp queues of the open pairs: warp w owns entries [128 w, 128 w + 128)
+    // per-warp queues of the open pairs: warp w owns entries [64 w, 64 w + 64)
     __shared__ double qK[CL_TILE], qq[CL_TILE];
     __shared__ int32_t qi[CL_TILE];
     __shared__ uint8_t qs[CL_TILE];
@@ -251,39 +253,6 @@ __global__ void __launch_bounds__(CL_THREADS) classify_kernel(const __grid_const
     }
 }
 
-// Baselines of the network list, computed densely over the list (in the
-// classify kernel only the trusted lanes would need them, and the others
-// would wait).  A pair whose baseline float cannot form moves to the
-// fallback list; its network row is computed but not written (index -1).
-template <int PROC>
-__global__ void __launch_bounds__(256) netprep_kernel(const __grid_constant__ InferParams p) {
-    const unsigned long long cnt = p.counters[0];
-    for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x; base < cnt;
-         base += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned long long e = base + threadIdx.x;
-        bool to_fb = false;
-        int32_t i = 0;
-        uint8_t sg = 0;
-        if (e < cnt) {
-            i = p.net_idx[e];
-            sg = p.net_seg[e];
-            float bf;
-            if (baseline_value<PROC>(p.K[i], p.q[i], p.consts[sg], bf) && isfinite(bf)) {
-                p.net_base[e] = bf;
-            } else {
-                p.net_idx[e] = -1;
-                to_fb = true;
-            }
-        }
-        int s_fb;
-        append(&p.counters[1], to_fb, s_fb);
-        if (to_fb) {
-            p.fb_idx[s_fb] = i;
-            p.fb_seg[s_fb] = sg;
-        }
-    }
-}
-
 // Appends (index, segment) of the lanes with `push` to a shared-memory queue
 // (warp-aggregated).
 __device__ __forceinline__ void push_index(bool push, int32_t i, uint8_t sg, int32_t *q, uint8_t *qs, int *qn) {
@@ -325,11 +294,17 @@ static __device__ __noinline__ void quad_redo_listed(noa_dcs::QuadSmem<PROC, noa
 // One resident grid; a list below one pair per thread of it is spread over
 // all CTAs in equal tiles, a longer one is taken 256 at a time (equal tiles:
 // 158 us and 247 us at 4e5 and 4e6).
-// Four CTAs per SM (at most 64 registers; pair production spills 48 bytes
-// and runs 3% faster at 4e6 than at three CTAs).
-constexpr int FB_THREADS = 256, FB_CTAS = 4;
+// At most 64 registers (pair production spills 48 bytes and runs 3% faster at
+// 4e6 than with 80).  The CTA's barriers keep its warps in the same form, which
+// their instruction cache needs: pair production, whose forms are the longest,
+// takes 611 / 547 / 529 us at 4e6 with 128 / 256 / 512 threads (and 560 as one
+// kernel a form without barriers), photonuclear 231 / 233 / 238.
+__host__ __device__ constexpr int fb_threads(int proc) { return proc == NOA_DCS_PAIR_PRODUCTION ? 512 : 256; }
+constexpr int FB_WARPS = 32;  // per SM
 template <int PROC>
-__global__ void __launch_bounds__(FB_THREADS, FB_CTAS) fallback_kernel(const __grid_constant__ InferParams p) {
+__global__ void __launch_bounds__(fb_threads(PROC), FB_WARPS * 32 / fb_threads(PROC))
+    fallback_kernel(const __grid_constant__ InferParams p) {
+    constexpr int FB_THREADS = fb_threads(PROC);
     using noa_dcs::QUAD_REDO;
     // pair production: redo pairs are evaluated again with the float-float
     // screening log, and the few it still rejects go to a third queue (FP64)
@@ -465,7 +440,7 @@ __global__ void __launch_bounds__(NT, 1) network_kernel(const __grid_constant__ 
     unsigned char *W2h = sm, *W2l = sm + MAT, *W3h = sm + 2 * MAT, *W3l = sm + 3 * MAT;
     __shared__ __align__(16) float sW1[H * IN];
     __shared__ float sb1[H], sb2[H], sb3[H], sWo[H];
-    __shared__ float spart[SLOTS][TILE];
+    __shared__ float spart[SLOTS][TILE], sbase[SLOTS][TILE];
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(8) unsigned long long mbar[SLOTS];
     __shared__ int s_abort[SLOTS];
@@ -530,12 +505,7 @@ __global__ void __launch_bounds__(NT, 1) network_kernel(const __grid_constant__ 
     for (long long t = (long long)blockIdx.x * SLOTS + slot; t < tiles; t += stride) {
         const long long e = t * TILE + row;
         const bool valid = e < (long long)cnt;
-        int32_t oi = -1;
-        float obase = 0.f;
-        if (half == 0 && valid) {
-            oi = p.net_idx[e];
-            obase = p.net_base[e];
-        }
+        const int32_t oi = valid ? p.net_idx[e] : -1;
         const float4 f_next = load_feat(t + stride);
         // layer 1 (FP32): 64 hidden units of this row, written to TMEM as A
 #pragma unroll 1
@@ -569,6 +539,21 @@ __global__ void __launch_bounds__(NT, 1) network_kernel(const __grid_constant__ 
             if (issuer)
                 issue_layer_ts(acc, a_hi, a_lo, smem_u32(layer ? W3h : W2h), smem_u32(layer ? W3l : W2l), mb);
             pending = true;
+            // Meanwhile the second half's threads compute their rows' baselines.  A
+            // pair whose baseline float cannot form moves to the fallback
+            // list; its network row is computed but not written.
+            if (layer == 0 && half == 1) {
+                float base = 0.f;
+                const uint8_t sg = valid ? p.net_seg[e] : 0;
+                const bool formed = valid && baseline_value<PROC>(p.K[oi], p.q[oi], p.consts[sg], base) && isfinite(base);
+                sbase[slot][row] = formed ? base : INFINITY;
+                int at;
+                append(&p.counters[1], valid && !formed, at);
+                if (valid && !formed) {
+                    p.fb_idx[at] = oi;
+                    p.fb_seg[at] = sg;
+                }
+            }
             const bool ok = mbar_wait(mb, phase);
             if (!ok)
                 s_abort[slot] = 1;
@@ -609,8 +594,9 @@ __global__ void __launch_bounds__(NT, 1) network_kernel(const __grid_constant__ 
         if (half == 0 && valid) {
             const float yy = y + spart[slot][row] + bo;
             const float r = p.norm.out_shift + yy / p.norm.out_scale;
-            if (oi >= 0)
-                p.out[oi] = fpconv::f64(expf(obase + r));
+            const float base = sbase[slot][row];
+            if (base < INFINITY)
+                p.out[oi] = fpconv::f64(expf(base + r));
         }
     }
     // after an expired wait, give the slot's MMAs in flight one more bounded
@@ -716,7 +702,7 @@ extern "C" int noa_dcs_mlp_infer(noa_dcs_mlp *model, const uint8_t *trust, int n
         return ifail(NOA_DCS_ERROR_NOT_DEVICE_MEMORY, "K, q, result and the trust grid must be device memory");
     // one call at a time owns the scratch (calls from several host threads serialise here)
     std::lock_guard<std::mutex> lock(g_scratch_mu);
-    const size_t per = sizeof(int32_t) + sizeof(float) + sizeof(float4) + 1 + sizeof(int32_t) + 1;
+    const size_t per = sizeof(int32_t) + sizeof(float4) + 1 + sizeof(int32_t) + 1;
     if (g_scratch.device != dev || g_scratch.cap < n) {
         if (g_scratch.buf)
             cudaFree(g_scratch.buf);
@@ -733,30 +719,20 @@ extern "C" int noa_dcs_mlp_infer(noa_dcs_mlp *model, const uint8_t *trust, int n
     p.counters = reinterpret_cast<unsigned long long *>(b);
     p.net_feat = reinterpret_cast<float4 *>(b + 64);
     p.net_idx = reinterpret_cast<int32_t *>(p.net_feat + n);
-    p.net_base = reinterpret_cast<float *>(p.net_idx + n);
-    p.fb_idx = reinterpret_cast<int32_t *>(p.net_base + n);
+    p.fb_idx = p.net_idx + n;
     p.net_seg = reinterpret_cast<uint8_t *>(p.fb_idx + n);
     p.fb_seg = p.net_seg + n;
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = cudaMemsetAsync(p.counters, 0, 64, s);
     int sms = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t blocks = (n + 255) / 256;
-    const int cgrid = (int)(blocks < sms * 8 ? blocks : sms * 8);
     const int64_t ctiles = (n + CL_THREADS * CL_ITEMS - 1) / (CL_THREADS * CL_ITEMS);
-    const int clgrid = (int)(ctiles < sms * 8 ? ctiles : sms * 8);
+    const int clgrid = (int)(ctiles < sms * CL_CTAS ? ctiles : sms * CL_CTAS);
     if (e == cudaSuccess) {
         if (process == NOA_DCS_PAIR_PRODUCTION)
             classify_kernel<NOA_DCS_PAIR_PRODUCTION><<<clgrid, CL_THREADS, 0, s>>>(p);
         else
             classify_kernel<NOA_DCS_PHOTONUCLEAR><<<clgrid, CL_THREADS, 0, s>>>(p);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) {
-        if (process == NOA_DCS_PAIR_PRODUCTION)
-            netprep_kernel<NOA_DCS_PAIR_PRODUCTION><<<cgrid, 256, 0, s>>>(p);
-        else
-            netprep_kernel<NOA_DCS_PHOTONUCLEAR><<<cgrid, 256, 0, s>>>(p);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
@@ -770,9 +746,11 @@ extern "C" int noa_dcs_mlp_infer(noa_dcs_mlp *model, const uint8_t *trust, int n
     }
     if (e == cudaSuccess) {
         if (process == NOA_DCS_PAIR_PRODUCTION)
-            fallback_kernel<NOA_DCS_PAIR_PRODUCTION><<<sms * FB_CTAS, FB_THREADS, 0, s>>>(p);
+            fallback_kernel<NOA_DCS_PAIR_PRODUCTION>
+                <<<sms * FB_WARPS * 32 / fb_threads(NOA_DCS_PAIR_PRODUCTION), fb_threads(NOA_DCS_PAIR_PRODUCTION), 0, s>>>(p);
         else
-            fallback_kernel<NOA_DCS_PHOTONUCLEAR><<<sms * FB_CTAS, FB_THREADS, 0, s>>>(p);
+            fallback_kernel<NOA_DCS_PHOTONUCLEAR>
+                <<<sms * FB_WARPS * 32 / fb_threads(NOA_DCS_PHOTONUCLEAR), fb_threads(NOA_DCS_PHOTONUCLEAR), 0, s>>>(p);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && stats)

@@ -31,3 +31,20 @@ def test_all_rejected(cuda_device, process, counts):
     # pair-production pairs move by 1e-11
     assert torch.equal(got == 0, exp == 0)
     assert torch.allclose(got, exp, rtol=1e-9, atol=0.0)
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 513, 5000])
+@pytest.mark.parametrize("process", [1, 2], ids=["pair_production", "photonuclear"])
+def test_network_tiles(cuda_device, process, n):
+    """Every cell trusted: a pair's value does not depend on the tiles around
+    it, nor on where its list ends."""
+    g = np.random.default_rng(10)
+    K = 10.0 ** g.uniform(1.5, 5, 20_000)
+    K, q = (torch.from_numpy(a).cuda() for a in (K, K * g.uniform(0.003, 0.999, K.size)))
+    s = Surrogate(process)
+    s.set_params(init_params(3), np.array([0, 0, 0, 0, 0.1, 0.1, 1, 1, 0, 1], dtype=np.float32))
+    ones = np.ones((len(BATCH_Z), *GRID), dtype=np.uint8)
+    every, stats = s.infer(K, q, [K.numel()], trust=ones)
+    some, few = s.infer(K[:n].clone(), q[:n].clone(), [n], trust=ones)
+    assert stats["status"] == few["status"] == 0 and stats["network"] > 0.9 * K.numel()
+    assert torch.equal(some, every[:n])
