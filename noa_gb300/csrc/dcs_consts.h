@@ -106,6 +106,15 @@ typedef struct noa_dcs_consts {
     float mass2_f;                 /* mass^2 rounded to float */
     float pp_kmax_shift_f;         /* pp_kmax_shift rounded to float */
     float ph_q_min_f;              /* ph_q_min rounded to float */
+
+    /* the FP32C bodies' constants: the fields above rounded to float, here and
+     * not in every evaluation (a rounding is about 12 integer instructions,
+     * and a third of bremsstrahlung's were these) */
+    float Zd_f, A_f, inv_m2_f;
+    float br_phie_factor_f, br_BZ_n_f, br_BZ_e_f, br_D_n_f, br_half_m2_f, br_Dn_sqrte_m2_f, br_BZe_mass_f;
+    float pp_Z13_f, pp_AZ13_f, pp_cL_f, pp_cLe_f, pp_inv_r2_f, pp_r_AZ13_f, pp_15_Z13_f, pp_gamma1_f, pp_gamma2_f;
+    float ph_logA_f, ph_a_low_f, ph_inv_log_q02_f;
+    float io_cZA_f;
 } noa_dcs_consts;
 
 /* Fills c from (A, I, Z, mass) with the reference's expressions (host code;
@@ -207,6 +216,29 @@ static inline void noa_dcs_fill_consts(noa_dcs_consts *c, double A, double I, in
         c->io_cW = 0.5 * (mass * mass + me * me) / me;
         c->io_4_inv_m2 = 4. / (mass * mass);
     }
+    c->Zd_f = (float)c->Zd;
+    c->A_f = (float)c->A;
+    c->inv_m2_f = (float)c->inv_m2;
+    c->br_phie_factor_f = (float)c->br_phie_factor;
+    c->br_BZ_n_f = (float)c->br_BZ_n;
+    c->br_BZ_e_f = (float)c->br_BZ_e;
+    c->br_D_n_f = (float)c->br_D_n;
+    c->br_half_m2_f = (float)c->br_half_m2;
+    c->br_Dn_sqrte_m2_f = (float)c->br_Dn_sqrte_m2;
+    c->br_BZe_mass_f = (float)c->br_BZe_mass;
+    c->pp_Z13_f = (float)c->pp_Z13;
+    c->pp_AZ13_f = (float)c->pp_AZ13;
+    c->pp_cL_f = (float)c->pp_cL;
+    c->pp_cLe_f = (float)c->pp_cLe;
+    c->pp_inv_r2_f = (float)c->pp_inv_r2;
+    c->pp_r_AZ13_f = (float)c->pp_r_AZ13;
+    c->pp_15_Z13_f = (float)c->pp_15_Z13;
+    c->pp_gamma1_f = (float)c->pp_gamma1;
+    c->pp_gamma2_f = (float)c->pp_gamma2;
+    c->ph_logA_f = (float)c->ph_logA;
+    c->ph_a_low_f = (float)c->ph_a_low;
+    c->ph_inv_log_q02_f = (float)c->ph_inv_log_q02;
+    c->io_cZA_f = (float)c->io_cZA;
 }
 
 #ifdef __cplusplus

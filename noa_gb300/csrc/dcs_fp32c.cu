@@ -1,23 +1,27 @@
 /*
  * FP32-compensated DCS kernels (precision NOA_DCS_FP32C) for sm_103a.
  *
- * One kernel shape for all four processes, built on the compacting kernel of
- * the FP64 path (dcs_fp64.cu) with a second queue:
+ * Pair production and photonuclear use the compacting kernel of the FP64 path
+ * (dcs_fp64.cu) with a second queue:
  *
- *   1. a CTA classifies a 1024-pair tile with the exact kinematic bounds
- *      (pair production, photonuclear; bremsstrahlung and ionisation are
- *      evaluated for every pair), writes the zeros, and appends the open
- *      pairs to the shared-memory work queue;
+ *   1. a CTA classifies a 1024-pair tile with the exact kinematic bounds,
+ *      writes the zeros, and appends the open pairs to the shared-memory work
+ *      queue;
  *   2. whenever the work queue holds 256 pairs, each thread pops one and
  *      evaluates it in FP32 (dcs_fp32c.cuh), which also returns an estimate
  *      of its relative error; results within `tol` are written, the others
  *      are appended (warp-aggregated) to a shared-memory redo queue;
- *   3. the redo queue is evaluated in FP64 (bremsstrahlung and ionisation 256
- *      pairs at a time, photonuclear by quad_redo) -- except for pair
- *      production, whose redo pairs are evaluated again, 256 at a time, in
- *      FP32 with the screening log in float-float arithmetic
- *      (pprod_fp32c<false, true>); the ~1% of those still above `tol` go to a
- *      third queue, evaluated in FP64 by quad_redo.
+ *   3. the redo queue is evaluated in FP64 by quad_redo (photonuclear), or
+ *      (pair production) again in FP32, 256 pairs at a time, with the
+ *      screening log in float-float arithmetic (pprod_fp32c<false, true>);
+ *      the ~1% of those still above `tol` go to a third queue, evaluated in
+ *      FP64 by quad_redo.
+ *
+ * Bremsstrahlung and ionisation are evaluated for every pair, so they have no
+ * work queue: a thread evaluates the pairs it loads, and the rejected ones go
+ * through a redo queue, 256 at a time.  With the work queue, 1e7 pairs of iron
+ * took 138 / 144 us (barriers were the largest stall), now 107 / 118; 61 pairs
+ * 3.7 / 3.2 us, now 2.1 / 2.4.
  *
  * The tile follows the size of the call, so that a short list spreads over
  * the SMs.
@@ -44,7 +48,9 @@ constexpr int F_RCAP = 2 * F_THREADS;
 // 1.21 ms at 2, 1.17 at 3 and 1.19 at 4 (with half the tile, for the shared
 // memory), but 63 us against 72 and 69 at 250007; photonuclear 463 us at 4
 // (64 registers, spilling), 445 at 3, 460 at 5; bremsstrahlung / ionisation
-// 136 / 142 us at 4, 141 / 148 at 3, 144 / 146 at 5.
+// with their pairs through a work queue 136 / 142 us at 4, 141 / 148 at 3,
+// 144 / 146 at 5.  (Since then 12% fewer instructions: pair production 1.07 ms,
+// photonuclear 438 us.)
 template <int PROC>
 constexpr int f32_min_ctas() {
     return PROC == NOA_DCS_PROC_PPROD ? 2 : (PROC == NOA_DCS_PROC_PHOTO ? 3 : 4);
@@ -52,24 +58,18 @@ constexpr int f32_min_ctas() {
 
 template <int PROC>
 __device__ __forceinline__ double eval32(double K, double q, const noa_dcs_consts &c, float &est) {
-    if (PROC == NOA_DCS_PROC_BREMS)
-        return brems_fp32c(K, q, c, est);
-    else if (PROC == NOA_DCS_PROC_PPROD)
+    if (PROC == NOA_DCS_PROC_PPROD)
         return pprod_fp32c<false>(K, q, c, est);
-    else if (PROC == NOA_DCS_PROC_PHOTO)
-        return photo_fp32c<false>(K, q, c, est);
     else
-        return ion_fp32c(K, q, c, est);
+        return photo_fp32c<false>(K, q, c, est);
 }
 
 template <int PROC>
 __device__ __forceinline__ bool open32(double K, double q, const noa_dcs_consts &c) {
     if (PROC == NOA_DCS_PROC_PPROD)
         return pprod_live(K, q, c);
-    else if (PROC == NOA_DCS_PROC_PHOTO)
-        return photo_live(K, q, c);
     else
-        return true;
+        return photo_live(K, q, c);
 }
 
 // The third queue exists for pair production only.
@@ -156,6 +156,74 @@ __device__ __forceinline__ bool fine_step(Queues<PROC> &s, int e, bool valid, do
     return redo;
 }
 
+// Bremsstrahlung and ionisation: every pair is evaluated where it was loaded,
+// and only the rejected ones (0.3 - 0.6% and less) go through a queue, which
+// holds what is left of a batch and one tile of which every pair is rejected.
+struct RedoQueue {
+    double K[F_THREADS + F_TILE], Q[F_THREADS + F_TILE];
+    int64_t I[F_THREADS + F_TILE];
+    int n;
+};
+
+template <int PROC>
+__global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_map_kernel(
+    const double *__restrict__ K, const double *__restrict__ q, double *out, int64_t n, int tile,
+    const __grid_constant__ noa_dcs_consts c, float tol) {
+    static_assert(!is_quad(PROC), "the quadrature processes compact their open pairs");
+    __shared__ RedoQueue s;
+    if (threadIdx.x == 0)
+        s.n = 0;
+    __syncthreads();
+    const int64_t stride = (int64_t)gridDim.x * tile;
+    for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += stride) {
+        const int here = n - base < tile ? (int)(n - base) : tile;
+        int o = threadIdx.x;
+        double k_next = 1., r_next = 1.;
+        if (o < here) {
+            k_next = K[base + o];
+            r_next = q[base + o];
+        }
+        // one call site of the evaluation, the next pair requested before it
+#pragma unroll 1
+        for (int first = 0; first < here; first += F_THREADS, o += F_THREADS) {
+            const double k = k_next, r = r_next;
+            if (o + F_THREADS < here) {
+                k_next = K[base + o + F_THREADS];
+                r_next = q[base + o + F_THREADS];
+            }
+            bool redo = false;
+            if (o < here) {
+                float est;
+                const double v = PROC == NOA_DCS_PROC_BREMS ? brems_fp32c(k, r, c, est) : ion_fp32c(k, r, c, est);
+                redo = !(est <= tol);
+                if (!redo)
+                    out[base + o] = v;
+            }
+            push_queue(redo, k, r, base + o, s.K, s.Q, s.I, &s.n);
+        }
+        // All of this tile's entries are in; the second barrier keeps the next
+        // tile's (and the drain's new length) behind every thread's reading.
+        __syncthreads();
+        int rn = s.n;
+        __syncthreads();
+        const bool last = base + stride >= n;
+        while (rn >= F_THREADS || (last && rn > 0)) {
+            const int take = rn < F_THREADS ? rn : F_THREADS;
+            rn -= take;
+            if (threadIdx.x == 0)
+                s.n = rn;
+            if ((int)threadIdx.x < take) {
+                const int e = rn + threadIdx.x;
+                // bremsstrahlung's redo pairs are those at the edge
+                out[s.I[e]] = PROC == NOA_DCS_PROC_BREMS ? brems_reference(s.K[e], s.Q[e], c)
+                                                         : ion_fp64(s.K[e], s.Q[e], c);
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// Pair production and photonuclear.
 template <int PROC>
 __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_kernel(const double *__restrict__ K,
                                                               const double *__restrict__ q, double *out, int64_t n,
@@ -234,16 +302,8 @@ __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_ker
                         quad_redo<PROC, F_THREADS>(s.quad, some, c, s.xK + xn, s.xQ + xn, s.xI + xn, out);
                         __syncthreads();
                     }
-                } else if constexpr (PROC == NOA_DCS_PROC_PHOTO) {
-                    quad_redo<PROC, F_THREADS>(s.quad, take, c, s.rK + rn, s.rQ + rn, s.rI + rn, out);
-                    __syncthreads();
                 } else {
-                    if ((int)threadIdx.x < take) {
-                        const int e = rn + threadIdx.x;
-                        // bremsstrahlung's redo pairs are those at the edge
-                        out[s.rI[e]] = PROC == NOA_DCS_PROC_BREMS ? brems_reference(s.rK[e], s.rQ[e], c)
-                                                                  : ion_fp64(s.rK[e], s.rQ[e], c);
-                    }
+                    quad_redo<PROC, F_THREADS>(s.quad, take, c, s.rK + rn, s.rQ + rn, s.rI + rn, out);
                     __syncthreads();
                 }
                 did = true;
@@ -287,7 +347,10 @@ static cudaError_t launch(const double *K, const double *q, double *out, int64_t
     int64_t tile = (n + cap * steps - 1) / (cap * steps);
     tile = tile < 32 ? 32 : tile;
     const int grid = (int)((n + tile * steps - 1) / (tile * steps));
-    dcs_fp32c_kernel<PROC><<<grid, F_THREADS, 0, s>>>(K, q, out, n, (int)tile, c, tol);
+    if constexpr (is_quad(PROC))
+        dcs_fp32c_kernel<PROC><<<grid, F_THREADS, 0, s>>>(K, q, out, n, (int)tile, c, tol);
+    else
+        dcs_fp32c_map_kernel<PROC><<<grid, F_THREADS, 0, s>>>(K, q, out, n, (int)tile, c, tol);
     return cudaGetLastError();
 }
 

@@ -86,7 +86,20 @@ NOA_HD float f_rcp(float x) {
     return 1.f / x;
 #endif
 }
+// The same for a normal x below 2^126, without the selection (3 of 7
+// instructions); 1/0 and 1/inf may come out as NaN.  In the node loops, where a
+// denominator leaves that range only for arguments that the estimate rejects
+// anyway (a NaN node makes the estimate NaN, and FP64 evaluates the pair).
+NOA_HD float f_rcp_n(float x) {
+#if defined(__CUDA_ARCH__)
+    const float y = lean64::rcp_approx(x);
+    return fmaf(y, fmaf(-x, y, 1.f), y);
+#else
+    return 1.f / x;
+#endif
+}
 NOA_HD float f_div(float a, float b) { return a * f_rcp(b); }
+NOA_HD float f_div_n(float a, float b) { return a * f_rcp_n(b); }
 NOA_HD float f_clamp0(float v) { return v < 0.f ? 0.f : v; }
 
 // H(u) = (log1p(u) - u) / u^2 on [0, 1] (gen_fp32c_poly.py, 9.7e-9 truncation).
@@ -223,7 +236,7 @@ NOA_HD FF ff_log(FF x) {
 // ---------------------------------------------------------------- bremsstrahlung
 NOA_HD double brems_fp32c(double K, double q, const noa_dcs_consts &c, float &est) {
     est = 0.f;
-    const float Kf = fpconv::f32(K), qf = fpconv::f32(q);
+    const float Kf = fpconv::f32_normal(K), qf = fpconv::f32_normal(q);  // NaN outside the normal range
     if (!(Kf > 1e-20f && Kf < 1e30f && qf > 1e-20f && qf < 1e30f)) {  // NaN, q <= 0, extreme ranges: FP64
         est = INFINITY;
         return 0.;
@@ -238,21 +251,21 @@ NOA_HD double brems_fp32c(double K, double q, const noa_dcs_consts &c, float &es
         return 0.;
     }
     // q < qe_max (physics.hh:142): float decision, exact when close
-    const float qe = f_div(Ef, 1.f + fpconv::f32(c.br_half_m2) * f_rcp((float)ME * Ef));
+    const float qe = f_div(Ef, 1.f + c.br_half_m2_f * f_rcp((float)ME * Ef));
     bool below = qf < qe;
     if (fabsf(qf - qe) <= 1e-5f * qe)
         below = brems_below_qe(K + c.mass, q, c);
     const float sqrte = 1.648721271f;
     // delta = 0.5 m^2 nu / (E (1 - nu)) = 0.5 m^2 q / (E (E - q))
-    const float delta = fpconv::f32(c.br_half_m2) * qf * f_rcp(Ef * Emq);
-    const float BZn = fpconv::f32(c.br_BZ_n), Dn = fpconv::f32(c.br_D_n), BZe = fpconv::f32(c.br_BZ_e);
-    const float Phi_n = logf((BZn * (fpconv::f32(c.mass) + delta * fpconv::f32(c.br_Dn_sqrte_m2))) *
+    const float delta = c.br_half_m2_f * qf * f_rcp(Ef * Emq);
+    const float BZn = c.br_BZ_n_f, Dn = c.br_D_n_f, BZe = c.br_BZ_e_f;
+    const float Phi_n = logf((BZn * (c.mass_h + delta * c.br_Dn_sqrte_m2_f)) *
                              f_rcp(Dn * ((float)ME + delta * sqrte * BZn)));
     float Phi_e = 0.f;
     if (below)
-        Phi_e = logf(fpconv::f32(c.br_BZe_mass) *
-                     f_rcp((1.f + delta * fpconv::f32(c.br_phie_factor)) * ((float)ME + delta * sqrte * BZe)));
-    const float Zf = fpconv::f32(c.Zd);
+        Phi_e = logf(c.br_BZe_mass_f *
+                     f_rcp((1.f + delta * c.br_phie_factor_f) * ((float)ME + delta * sqrte * BZe)));
+    const float Zf = c.Zd_f;
     const float S = Zf * f_clamp0(Phi_n) + f_clamp0(Phi_e);
     // 4/3 (1/nu - 1) + nu = 4/3 (E - q)/q + q/E
     const float fac = 1.33333333f * Emq * f_rcp(qf) + qf * f_rcp(Ef);
@@ -301,11 +314,12 @@ NOA_HD double pprod_fp32c(double K, double q, const noa_dcs_consts &c, float &es
     // tmin = log(argmin) = tmin + tmin_lo, float-float log (~2^-44, no FP64)
     const FF tminF0 = ff_log(argmin);
     const float tmin = tminF0.h, tmin_lo = tminF0.l;
-    const float beta = fpconv::f32(beta_d);
-    const float xi_factor = fpconv::f32(c.pp_half_r2 * beta_d);
-    const float qf = fpconv::f32(q);
-    const float AZ13 = fpconv::f32(c.pp_AZ13), cL = fpconv::f32(c.pp_cL), cLe = fpconv::f32(c.pp_cLe);
-    const float rAZ13 = fpconv::f32(c.pp_r_AZ13), Z13_15 = fpconv::f32(c.pp_15_Z13), inv_r2 = fpconv::f32(c.pp_inv_r2);
+    // NaN outside the normal float range: the estimate is then NaN and FP64 decides
+    const float beta = fpconv::f32_normal(beta_d);
+    const float xi_factor = fpconv::f32_normal(c.pp_half_r2 * beta_d);
+    const float qf = fpconv::f32_normal(q);
+    const float AZ13 = c.pp_AZ13_f, cL = c.pp_cL_f, cLe = c.pp_cLe_f;
+    const float rAZ13 = c.pp_r_AZ13_f, Z13_15 = c.pp_15_Z13_f, inv_r2 = c.pp_inv_r2_f;
     const float b2 = 2.f * beta, b15 = 1.5f * beta, b3 = 3.f * beta, b4 = 4.f * beta;
 
     // float-float inputs of the screening log (FINE only)
@@ -331,11 +345,22 @@ NOA_HD double pprod_fp32c(double K, double q, const noa_dcs_consts &c, float &es
         const float rho2 = rho * rho;
         const float rho21 = eps * (2.f - eps);
         const float xi = xi_factor * rho21;
-        const float xi_i = f_rcp(xi);
+        const float xi_i = f_rcp_n(xi);
         const float opxi = 1.f + xi;
-        const float inv_opxi = f_rcp(opxi);
+        const float inv_opxi = f_rcp_n(opxi);
         // branch thresholds of the reference (1e3, 1e-3) must be taken as it takes them
         edge |= fabsf(xi - 1e3f) <= 2e-4f || fabsf(xi - 1e-3f) <= 2e-10f;
+
+        // One H and one log1p a node serve both screening functions: Be takes
+        // log(1 + 1/xi) and Bmu log(1 + xi), one of them at u = min(xi, 1/xi),
+        // from H, and the other at 1/u.  As branches of their own, the lanes of
+        // a warp on either side of xi = 1 made it run two of each.
+        const bool above = xi >= 1.f;
+        const float u = above ? xi_i : xi;
+        const float Gs = u * poly_H(u);                     // log1p(u)/u - 1
+        const float Ls = u * (1.f + Gs);                    // log1p(u)
+        const float Ll = log1pf(above ? xi : xi_i);         // log1p(1/u)
+        const float Gl = fmaf(Ll, u, -1.f);                 // u log1p(1/u) - 1
 
         float Be, eBe;
         if (xi >= 1E+03f) {
@@ -343,22 +368,16 @@ NOA_HD double pprod_fp32c(double K, double q, const noa_dcs_consts &c, float &es
             eBe = 2.f * U32 * Be;
         } else {
             const float A = (2.f + rho2) * (1.f + beta);
-            float L, G;
-            if (xi >= 1.f) {
-                G = xi_i * poly_H(xi_i);  // xi log(1 + 1/xi) - 1
-                L = xi_i * (1.f + G);     // log(1 + 1/xi)
-            } else {
-                L = log1pf(xi_i);
-                G = xi * L - 1.f;
-            }
+            const float L = above ? Ls : Ll;  // log(1 + 1/xi)
+            const float G = above ? Gs : Gl;  // xi L - 1
             const float t1 = A * L, t2 = (3.f + rho2) * G, t3 = (rho21 - beta) * inv_opxi;
             Be = t1 + t2 + t3;
             eBe = 2.f * U32 * (fabsf(t1) + fabsf(t2) + fabsf(t3) + fabsf(beta) * inv_opxi);
         }
-        const float Ye = f_div(5.f - rho2 + b4 * (1.f + rho2), 2.f * (1.f + b3) * logf(3.f + xi_i) - rho2 -
+        const float Ye = f_div_n(5.f - rho2 + b4 * (1.f + rho2), 2.f * (1.f + b3) * logf(3.f + xi_i) - rho2 -
                                                                   b2 * (2.f - rho2));
         const float xe = opxi * (1.f + Ye);
-        const float cLi = cL * f_rcp(rho21);
+        const float cLi = cL * f_rcp_n(rho21);
         float Le;
         if (FINE) {
             // Le = log(AZ13 q sqrt(xe) / D1) - log(D2) / 2 (dcs.hh:199-202) as one
@@ -377,8 +396,8 @@ NOA_HD double pprod_fp32c(double K, double q, const noa_dcs_consts &c, float &es
             const FF lg = ff_log(ff_div(ff_mul(aq2F, xeF), ff_mul(ff_mul(d1, d1), ff_add(1.f, ff_mul(cLeF, xeF)))));
             Le = 0.5f * (lg.h + lg.l);
         } else {
-            const float r1 = AZ13 * qf * f_rcp(qf + cLi * xe);
-            const float r2 = xe * f_rcp(1.f + cLe * xe);
+            const float r1 = AZ13 * qf * f_rcp_n(qf + cLi * xe);
+            const float r2 = xe * f_rcp_n(1.f + cLe * xe);
             Le = 0.5f * logf(r1 * r1 * r2);
         }
         const float Phi_e = f_clamp0(Be * Le);
@@ -388,23 +407,17 @@ NOA_HD double pprod_fp32c(double K, double q, const noa_dcs_consts &c, float &es
             Bmu = 0.5f * xi * (5.f - rho2 + beta * (3.f + rho2));
             eBmu = 2.f * U32 * Bmu;
         } else {
-            float L1, G2;
-            if (xi <= 1.f) {
-                G2 = xi * poly_H(xi);  // log(1 + xi)/xi - 1
-                L1 = xi * (1.f + G2);  // log(1 + xi)
-            } else {
-                L1 = log1pf(xi);
-                G2 = L1 * xi_i - 1.f;
-            }
+            const float L1 = xi > 1.f ? Ll : Ls;  // log(1 + xi)
+            const float G2 = xi > 1.f ? Gl : Gs;  // L1 / xi - 1
             const float s1 = (1.f + rho2) * (1.f + b15) * L1, s2 = (1.f + b2) * rho21 * G2,
                         s3 = xi * (rho21 - beta) * inv_opxi;
             Bmu = s1 - s2 + s3;
             eBmu = 2.f * U32 * (fabsf(s1) + fabsf(s2) + fabsf(s3) + xi * fabsf(beta) * inv_opxi);
         }
-        const float Ymu = f_div(4.f + rho2 + b3 * (1.f + rho2),
+        const float Ymu = f_div_n(4.f + rho2 + b3 * (1.f + rho2),
                                 (1.f + rho2) * (1.5f + b2) * logf(3.f + xi) + 1.f - 1.5f * rho2);
         const float xmu = opxi * (1.f + Ymu);
-        const float Lmu = logf(rAZ13 * qf * f_rcp(Z13_15 * (qf + cLi * xmu)));
+        const float Lmu = logf(rAZ13 * qf * f_rcp_n(Z13_15 * (qf + cLi * xmu)));
         const float Phi_mu = f_clamp0(Bmu * Lmu);
         const float g = -(Phi_e + Phi_mu * inv_r2) * eps * tmin;
         I.add(g * kF8W[j]);
@@ -427,19 +440,19 @@ NOA_HD double pprod_fp32c(double K, double q, const noa_dcs_consts &c, float &es
     // FP64 as in the plain kernel
     float zeta = 0.f, zeta_err = 0.f;
     if (!(gamma <= 35.)) {
-        const float gf = fpconv::f32(gamma), Z13 = fpconv::f32(c.pp_Z13);
-        const float L1 = logf(gf * f_rcp(1.f + fpconv::f32(c.pp_gamma1) * gf * Z13 * Z13));
+        const float gf = fpconv::f32_normal(gamma), Z13 = c.pp_Z13_f;
+        const float L1 = logf(gf * f_rcp(1.f + c.pp_gamma1_f * gf * Z13 * Z13));
         zeta = 0.073f * L1 - 0.26f;
         if (zeta <= 0.f) {
             zeta = 0.f;
         } else {
-            const float L2 = logf(gf * f_rcp(1.f + fpconv::f32(c.pp_gamma2) * gf * Z13));
+            const float L2 = logf(gf * f_rcp(1.f + c.pp_gamma2_f * gf * Z13));
             const float den = 0.058f * L2 - 0.14f;
             const float ez = ((0.073f * (fabsf(L1) + 3.f) + 0.26f) * f_rcp(zeta) +
                               (0.058f * (fabsf(L2) + 3.f) + 0.14f) * f_rcp(fabsf(den)) + 2.f) * U32;
             zeta = f_div(zeta, den);
             zeta_err = fabsf(zeta) * ez;
-            if (!(zeta_err <= 1e-7f * (fpconv::f32(c.Zd) + zeta))) {
+            if (!(zeta_err <= 1e-7f * (c.Zd_f + zeta))) {
                 double zd = 0.073 * d_log(gamma * d_rcp(1. + c.pp_gamma1 * gamma * c.pp_Z13 * c.pp_Z13)) - 0.26;
                 zd = zd <= 0. ? 0. : zd * d_rcp(0.058 * d_log(gamma * d_rcp(1. + c.pp_gamma2 * gamma * c.pp_Z13)) - 0.14);
                 zeta = fpconv::f32(zd);
@@ -453,7 +466,7 @@ NOA_HD double pprod_fp32c(double K, double q, const noa_dcs_consts &c, float &es
     // ranges of 4e6 seeded pairs, both forms): no pair above 1e-6 has an
     // estimate below 1.2e-6 (the estimate bounds the error with 17% to spare
     // at the tolerance); largest accepted error 7.5e-7
-    est = edge ? INFINITY : 1.2f * err * f_rcp(fpconv::f32(fabs(Id))) + zeta_err * f_rcp(fpconv::f32(c.Zd) + zeta);
+    est = edge ? INFINITY : 1.2f * err * f_rcp(fpconv::f32_normal(fabs(Id))) + zeta_err * f_rcp(c.Zd_f + zeta);
     const double dcs = c.pp_cZ * (c.Zd + fpconv::f64(zeta)) * Emq * Id * d_rcp(q * E);
     return (dcs < 0.) ? 0. : dcs * (mass + K) * c.scale_A;
 }
@@ -493,7 +506,7 @@ NOA_HD double photo_fp32c(double K, double q, const noa_dcs_consts &c, float &es
     } else {
         // the caller established the window (1 <= q < K); float-float holds
         // q^2 and the window for K below 1e15, FP64 takes the rest
-        if (!(fpconv::f32(K) < 1e15f)) {
+        if (!(fpconv::f32_normal(K) < 1e15f)) {
             est = INFINITY;
             return 0.;
         }
@@ -531,8 +544,8 @@ NOA_HD double photo_fp32c(double K, double q, const noa_dcs_consts &c, float &es
     const float inv_P = ff_div(FF{1.f, 0.f}, ff_add(FF{kMP2H, kMP2L}, two_MqF)).h;
     const float inv_R = ff_div(FF{1.f, 0.f}, ff_add(FF{kMR2H, kMR2L}, two_MqF)).h;
     const float inv_Q02 = 1.f / 0.52544f;
-    const float inv_LQ = fpconv::f32(c.ph_inv_log_q02);
-    const float Af = fpconv::f32(c.A), logA = fpconv::f32(c.ph_logA), a_low = fpconv::f32(c.ph_a_low);
+    const float inv_LQ = c.ph_inv_log_q02_f;
+    const float Af = c.A_f, logA = c.ph_logA_f, a_low = c.ph_a_low_f;
     const float two_m2 = 2.f * c.mass2_f;
     const float invEE = inv_EF.h * inv_EF.h;
     const float yy = y * y;
@@ -543,7 +556,7 @@ NOA_HD double photo_fp32c(double K, double q, const noa_dcs_consts &c, float &es
     for (int j = 0; j < 9; j++) {
         float Q2, unused;
         f_exp_split_aff(pc_h, pc_l, hd_h, hd_l, kF9XH[j], kF9XL[j], Q2, unused);
-        const float invQ2 = f_rcp(Q2);
+        const float invQ2 = f_rcp_n(Q2);
         const float x = 0.5f * Q2 * inv_Mq;
         // ALLM, dcs.hh:288-306
         const float t = log1pf(log1pf(Q2 * inv_Q02) * inv_LQ);
@@ -551,8 +564,8 @@ NOA_HD double photo_fp32c(double K, double q, const noa_dcs_consts &c, float &es
         const float xR = (Q2 + mR2) * inv_R;
         const float lnt = logf(t);
         const float ecP = expf(cP3 * lnt), eaP = expf(aP3 * lnt);
-        const float cP = cP1 - (cP1 - cP2) * ecP * f_rcp(1.f + ecP);
-        const float aP = aP1 - (aP1 - aP2) * eaP * f_rcp(1.f + eaP);
+        const float cP = cP1 - (cP1 - cP2) * ecP * f_rcp_n(1.f + ecP);
+        const float aP = aP1 - (aP1 - aP2) * eaP * f_rcp_n(1.f + eaP);
         const float bP = bP1 + bP2 * expf(bP3 * lnt);
         const float cR = cR1 + cR2 * expf(cR3 * lnt);
         const float aR = aR1 + aR2 * expf(aR3 * lnt);
@@ -564,12 +577,12 @@ NOA_HD double photo_fp32c(double K, double q, const noa_dcs_consts &c, float &es
         const float eP = aP * lxP + bP * l1x, eR = aR * lxR + bR * l1x;
         const float F2P = cP * expf(eP);
         const float F2R = cR * expf(eR);
-        const float F2p = Q2 * f_rcp(Q2 + m02) * (F2P + F2R);
+        const float F2p = Q2 * f_rcp_n(Q2 + m02) * (F2P + F2R);
         // float error of F2: the exponents carry ~3 u of each |term|
         const float eF2 = U32 *
                               (F2P * (fabsf(aP * lxP) + fabsf(bP * l1x) + 2.f) +
                                F2R * (fabsf(aR * lxR) + fabsf(bR * l1x) + 2.f)) *
-                              f_rcp(F2P + F2R) +
+                              f_rcp_n(F2P + F2R) +
                           3.f * U32;
         // DRSS shadowing, dcs.hh:310-319
         float a = 1.f, ea = 0.f;
@@ -586,21 +599,21 @@ NOA_HD double photo_fp32c(double K, double q, const noa_dcs_consts &c, float &es
         const bool low = Q2 < 0.3f;
         const float q2 = low ? 0.3f : Q2;
         const float inv_q2 = low ? 3.33333333f : invQ2;
-        const float theta = 1.f + 12.f * q2 * 0.015625f * f_rcp((1.f + q2) * (0.015625f + x * x));
-        const float R = 0.635f * theta * f_rcp(logf(q2 * 25.f)) + 0.5747f * inv_q2 - 0.3534f * f_rcp(0.09f + q2 * q2);
+        const float theta = 1.f + 12.f * q2 * 0.015625f * f_rcp_n((1.f + q2) * (0.015625f + x * x));
+        const float R = 0.635f * theta * f_rcp_n(logf(q2 * 25.f)) + 0.5747f * inv_q2 - 0.3534f * f_rcp_n(0.09f + q2 * q2);
         // d2sigma, dcs.hh:348-354, without cf / q (applied in double below)
-        const float T2 = 0.5f * (1.f - two_m2 * invQ2) * (yy + Q2 * invEE) * f_rcp(1.f + R);
+        const float T2 = 0.5f * (1.f - two_m2 * invQ2) * (yy + Q2 * invEE) * f_rcp_n(1.f + R);
         const float X = omy + T2;
         const float d_a = X * invQ2 * invQ2, d_b = 0.25f * invEE * invQ2;
         const float dds = d_a - d_b;
         const float g = F2A * dds * Q2;
         S.add(g * kF9W[j]);
         const float e_dds = 2.f * U32 * (fabsf(d_a) + fabsf(d_b)) +
-                            fabsf(d_a) * 3.f * U32 * (fabsf(omy) + fabsf(T2)) * f_rcp(fabsf(X));
+                            fabsf(d_a) * 3.f * U32 * (fabsf(omy) + fabsf(T2)) * f_rcp_n(fabsf(X));
         err += kF9W[j] * (fabsf(g) * (eF2 + ea + 4.f * U32) + fabsf(F2A * Q2) * e_dds);
     }
     const double ds_f = S.value();
-    est = edge ? INFINITY : 0.6f * err * f_rcp(fpconv::f32(fabs(ds_f)));  // calibrated: max error <= est
+    est = edge ? INFINITY : 0.6f * err * f_rcp(fpconv::f32_normal(fabs(ds_f)));  // calibrated: max error <= est
     // 0.5 ds dpQ2 cf (m + K) / q N_A 1e3 / A (dcs.hh:402-404), cf = 2.603096e-35
     const double fac = ff_to_double(ff_mul(dpQ2F, ff_div(ff_add(massF, KF), qF)));
     const double ds = ds_f * fac;
@@ -629,7 +642,7 @@ NOA_HD double ion_fp32c(double K, double q, const noa_dcs_consts &c, float &est)
     const long long qb = dbits(q);
     if (qb >= 0 && qb <= dbits(c.io_Wmin))  // +0 <= q <= Wmin
         return 0.;
-    const float Kf = fpconv::f32(K), qf = fpconv::f32(q);
+    const float Kf = fpconv::f32_normal(K), qf = fpconv::f32_normal(q);  // NaN outside the normal range
     if (!(Kf > 1e-20f && Kf < 1e12f && qf > 1e-20f && qf < 1e12f)) {  // NaN, q < 0, extreme ranges
         est = INFINITY;
         return 0.;
@@ -655,12 +668,12 @@ NOA_HD double ion_fp32c(double K, double q, const noa_dcs_consts &c, float &est)
     // E and E - q in float-float (E - q >= m: no cancellation beyond E / m)
     const FF EF = ff_add(Kx, FF{c.mass_h, c.mass_l});
     const float Ef = EF.h;
-    float cs = fpconv::f32(c.io_cZA) * Ef * bracket;
+    float cs = c.io_cZA_f * Ef * bracket;
     float Delta = 0.f;
     if (dbits(K) >= dbits(c.io_k_rad)) {  // K >= k_rad, both positive
         const float L1 = log1pf(qf * (float)(2. / ME));
         const FF Emq = ff_add(EF, ff_neg(qx));
-        Delta = 1.16141E-03f * L1 * (logf(4.f * Ef * (Emq.h + Emq.l) * fpconv::f32(c.inv_m2)) - L1);
+        Delta = 1.16141E-03f * L1 * (logf(4.f * Ef * (Emq.h + Emq.l) * c.inv_m2_f) - L1);
         cs *= 1.f + Delta;
     }
     // the close-collision term (max observed 8.7 u) and Delta relative to 1 + Delta
