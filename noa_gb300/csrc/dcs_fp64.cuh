@@ -655,7 +655,8 @@ static __device__ __noinline__ double photo_node_wide(const double pc, const dou
 }
 
 __device__ __forceinline__ double photo_finish(double K, double q, double hd, double sum, const noa_dcs_consts &c) {
-    return clamp0(c.ph_scale_A * sum * hd * (K + c.mass) * ol_rcp(q));
+    // E / q first: E times the rest overflows for K above 1e245, where the value does not
+    return clamp0(c.ph_scale_A * sum * hd * ((K + c.mass) * ol_rcp(q)));
 }
 
 // An open pair (photo_live), its nodes one after the other.
