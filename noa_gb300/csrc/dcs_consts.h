@@ -113,6 +113,8 @@ typedef struct noa_dcs_consts {
     float Zd_f, A_f, inv_m2_f;
     float br_phie_factor_f, br_BZ_n_f, br_BZ_e_f, br_D_n_f, br_half_m2_f, br_Dn_sqrte_m2_f, br_BZe_mass_f;
     float pp_Z13_f, pp_AZ13_f, pp_cL_f, pp_cLe_f, pp_inv_r2_f, pp_r_AZ13_f, pp_15_Z13_f, pp_gamma1_f, pp_gamma2_f;
+    float pp_cL_l, pp_cLe_l;       /* the rest of pp_cL_f, pp_cLe_f as float pairs */
+    float pp_AZ13sq_h, pp_AZ13sq_l;  /* AZ13 AZ13 */
     float ph_logA_f, ph_a_low_f, ph_inv_log_q02_f;
     float io_cZA_f;
 } noa_dcs_consts;
@@ -235,6 +237,13 @@ static inline void noa_dcs_fill_consts(noa_dcs_consts *c, double A, double I, in
     c->pp_15_Z13_f = (float)c->pp_15_Z13;
     c->pp_gamma1_f = (float)c->pp_gamma1;
     c->pp_gamma2_f = (float)c->pp_gamma2;
+    c->pp_cL_l = (float)(c->pp_cL - (double)c->pp_cL_f);
+    c->pp_cLe_l = (float)(c->pp_cLe - (double)c->pp_cLe_f);
+    {
+        const double a2 = c->pp_AZ13 * c->pp_AZ13;
+        c->pp_AZ13sq_h = (float)a2;
+        c->pp_AZ13sq_l = (float)(a2 - (double)c->pp_AZ13sq_h);
+    }
     c->ph_logA_f = (float)c->ph_logA;
     c->ph_a_low_f = (float)c->ph_a_low;
     c->ph_inv_log_q02_f = (float)c->ph_inv_log_q02;

@@ -12,10 +12,10 @@
  *      of its relative error; results within `tol` are written, the others
  *      are appended (warp-aggregated) to a shared-memory redo queue;
  *   3. the redo queue is evaluated in FP64 by quad_redo (photonuclear), or
- *      (pair production) again in FP32, 256 pairs at a time, with the
- *      screening log in float-float arithmetic (pprod_fp32c<false, true>);
- *      the ~1% of those still above `tol` go to a third queue, evaluated in
- *      FP64 by quad_redo.
+ *      (pair production) again in FP32, 256 pairs at a time and one (pair,
+ *      node) a thread, with the screening log in float-float arithmetic
+ *      (pprod32_batch); the ~1% of those still above `tol` go to a third
+ *      queue, evaluated in FP64 by quad_redo.
  *
  * Bremsstrahlung and ionisation are evaluated for every pair, so they have no
  * work queue: a thread evaluates the pairs it loads, and the rejected ones go
@@ -31,6 +31,7 @@
  * No global scratch.
  */
 #include "dcs_fp32c.cuh"
+#include "dcs_fp32c_batch.cuh"
 #include "dcs_quad.cuh"
 
 #include <cuda_runtime.h>
@@ -72,6 +73,12 @@ __device__ __forceinline__ bool open32(double K, double q, const noa_dcs_consts 
         return photo_live(K, q, c);
 }
 
+// Pair production's float-float step.
+template <int PROC>
+struct FineSmem {};
+template <>
+struct FineSmem<NOA_DCS_PROC_PPROD> : Pprod32Smem<F_THREADS> {};
+
 // The third queue exists for pair production only.
 template <int PROC>
 constexpr int f32_xcap() {
@@ -87,6 +94,7 @@ struct Queues {
     double xK[f32_xcap<PROC>()], xQ[f32_xcap<PROC>()];
     int64_t xI[f32_xcap<PROC>()];
     QuadSmem<PROC, QUAD_REDO> quad;
+    FineSmem<PROC> fine;
     int warp_tot[F_THREADS / 32];
     int tile_open;
     int rn, xn;
@@ -114,8 +122,10 @@ __device__ __forceinline__ void push_queue(bool push, double k, double q, int64_
 // Evaluates work-queue entry e (if valid) in FP32 and appends it to the redo
 // queue when its error estimate exceeds tol (and returns that).
 template <int PROC>
-__device__ __forceinline__ bool fp32_step(Queues<PROC> &s, int e, bool valid, double *out,
-                                          const noa_dcs_consts &c, float tol) {
+__device__ __forceinline__ bool fp32_step(Queues<PROC> &s, int at, int take, double *out, const noa_dcs_consts &c,
+                                          float tol) {
+    const int e = at + threadIdx.x;
+    const bool valid = (int)threadIdx.x < take;
     bool redo = false;
     double k = 0., q = 0.;
     int64_t i = 0;
@@ -133,12 +143,14 @@ __device__ __forceinline__ bool fp32_step(Queues<PROC> &s, int e, bool valid, do
     return redo;
 }
 
-// Pair production: evaluates redo-queue entry e (if valid) with the
-// float-float screening log and appends it to the third queue when its
-// estimate still exceeds tol.
+// Pair production: evaluates `take` redo-queue entries from `at` with the
+// float-float screening log and appends to the third queue those whose
+// estimate still exceeds tol (true for this thread's).
 template <int PROC>
-__device__ __forceinline__ bool fine_step(Queues<PROC> &s, int e, bool valid, double *out,
-                                          const noa_dcs_consts &c, float tol) {
+__device__ __forceinline__ bool fine_step(Queues<PROC> &s, int at, int take, double *out, const noa_dcs_consts &c,
+                                          float tol) {
+    const int e = at + threadIdx.x;
+    const bool valid = (int)threadIdx.x < take;
     bool redo = false;
     double k = 0., q = 0.;
     int64_t i = 0;
@@ -146,8 +158,10 @@ __device__ __forceinline__ bool fine_step(Queues<PROC> &s, int e, bool valid, do
         k = s.rK[e];
         q = s.rQ[e];
         i = s.rI[e];
-        float est;
-        const double v = pprod_fp32c<false, true>(k, q, c, est);
+    }
+    float est;
+    const double v = pprod32_batch<true>(s.fine, take, k, q, c, est);
+    if (valid) {
         redo = !(est <= tol);
         if (!redo)
             out[i] = v;
@@ -280,7 +294,7 @@ __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_ker
             bool did = false, rejected = false;
             if (qn >= F_THREADS || (!more && qn > 0)) {
                 const int take = qn < F_THREADS ? qn : F_THREADS;
-                rejected = fp32_step<PROC>(s, qn - take + threadIdx.x, (int)threadIdx.x < take, out, c, tol);
+                rejected = fp32_step<PROC>(s, qn - take, take, out, c, tol);
                 qn -= take;
                 did = true;
             }
@@ -292,7 +306,7 @@ __global__ void __launch_bounds__(F_THREADS, f32_min_ctas<PROC>()) dcs_fp32c_ker
                 if (threadIdx.x == 0)
                     s.rn = rn;
                 if constexpr (PROC == NOA_DCS_PROC_PPROD) {
-                    rejected = fine_step<PROC>(s, rn + threadIdx.x, (int)threadIdx.x < take, out, c, tol);
+                    rejected = fine_step<PROC>(s, rn, take, out, c, tol);
                     xn += __syncthreads_count(rejected);
                     while (xn >= QUAD_REDO || (!more && qn == 0 && rn == 0 && xn > 0)) {
                         const int some = xn < QUAD_REDO ? xn : QUAD_REDO;

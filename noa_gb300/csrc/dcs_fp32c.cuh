@@ -290,149 +290,151 @@ NOA_HD double brems_fp32c(double K, double q, const noa_dcs_consts &c, float &es
 // what sends ~4% of the open pairs past a 1e-6 estimate; with Le to ~1e-13
 // relative about one in a hundred of those stays above it.  About twice the
 // FP32 work of the float form, for the pairs the float form rejects.
-template <bool CHECKED = true, bool FINE = false>
-NOA_HD double pprod_fp32c(double K, double q, const noa_dcs_consts &c, float &est) {
-    est = 0.f;
-    FF argmin;
-    if (CHECKED) {
-        if (q <= 4. * ME)
-            return 0.;
-        if (q >= K + c.pp_kmax_shift)
-            return 0.;
-        const double a = pprod_argmin_exact(K, q, c);
-        if ((a >= 1.) || (a <= 0.))
-            return 0.;
-        argmin = ff_from(a);
-    } else {
-        argmin = pprod_argmin_ff(K, q, c);
-    }
-    const double mass = c.mass;
-    const double E = K + mass;
+//
+// Three parts, so that a CTA can evaluate a batch of pairs by (pair, node):
+// what is formed once a pair, one node, and the end.
+template <bool FINE>
+struct Pprod32 {
+    FF tmin;  // log(argmin)
+    float beta, xi_factor, qf;
+};
+template <>
+struct Pprod32<true> {
+    FF tmin;
+    float beta, xi_factor, qf;
+    FF betaF, xfF, qF, aq2F;  // float-float inputs of the screening log
+};
+
+template <bool FINE>
+NOA_HD void pprod32_setup(double K, double q, FF argmin, const noa_dcs_consts &c, Pprod32<FINE> &p) {
+    const double E = K + c.mass;
     const double Emq = E - q;
     // beta = 0.5 nu^2 / (1 - nu) = 0.5 q^2 / (E (E - q))
     const double beta_d = 0.5 * q * q * d_rcp(E * Emq);
-    // tmin = log(argmin) = tmin + tmin_lo, float-float log (~2^-44, no FP64)
-    const FF tminF0 = ff_log(argmin);
-    const float tmin = tminF0.h, tmin_lo = tminF0.l;
+    p.tmin = ff_log(argmin);  // float-float log (~2^-44, no FP64)
     // NaN outside the normal float range: the estimate is then NaN and FP64 decides
-    const float beta = fpconv::f32_normal(beta_d);
-    const float xi_factor = fpconv::f32_normal(c.pp_half_r2 * beta_d);
-    const float qf = fpconv::f32_normal(q);
+    p.beta = fpconv::f32_normal(beta_d);
+    p.xi_factor = fpconv::f32_normal(c.pp_half_r2 * beta_d);
+    p.qf = fpconv::f32_normal(q);
+    if constexpr (FINE) {
+        p.betaF = ff_from(beta_d);
+        p.xfF = ff_from(c.pp_half_r2 * beta_d);
+        p.qF = ff_from(q);
+        p.aq2F = ff_mul(FF{c.pp_AZ13sq_h, c.pp_AZ13sq_l}, ff_mul(p.qF, p.qF));
+    }
+}
+
+// Node j without its weight; eg takes its error, infinite where FP64 has to
+// decide a branch or a clamp.
+template <bool FINE>
+NOA_HD float pprod32_node(const Pprod32<FINE> &p, int j, const noa_dcs_consts &c, float &eg_out) {
+    const float tmin = p.tmin.h, tmin_lo = p.tmin.l;
+    const float beta = p.beta, xi_factor = p.xi_factor, qf = p.qf;
     const float AZ13 = c.pp_AZ13_f, cL = c.pp_cL_f, cLe = c.pp_cLe_f;
     const float rAZ13 = c.pp_r_AZ13_f, Z13_15 = c.pp_15_Z13_f, inv_r2 = c.pp_inv_r2_f;
     const float b2 = 2.f * beta, b15 = 1.5f * beta, b3 = 3.f * beta, b4 = 4.f * beta;
-
-    // float-float inputs of the screening log (FINE only)
-    FF tminF{}, betaF{}, xfF{}, qF{}, cLF{}, cLeF{}, aq2F{};
-    if (FINE) {
-        tminF = tminF0;
-        betaF = ff_from(beta_d);
-        xfF = ff_from(c.pp_half_r2 * beta_d);
-        qF = ff_from(q);
-        cLF = ff_from(c.pp_cL);
-        cLeF = ff_from(c.pp_cLe);
-        aq2F = ff_mul(ff_from(c.pp_AZ13 * c.pp_AZ13), ff_mul(qF, qF));
-    }
-
-    KSum I;
-    float err = 0.f;
     bool edge = !(fabsf(tmin) > 1e-6f);
-    NOA_UNROLL_NODES
-    for (int j = 0; j < 8; j++) {
-        float eps, rho;
-        f_exp_split_ff(kF8XH[j], kF8XL[j], tmin, tmin_lo, eps, rho);
-        rho = -rho;
-        const float rho2 = rho * rho;
-        const float rho21 = eps * (2.f - eps);
-        const float xi = xi_factor * rho21;
-        const float xi_i = f_rcp_n(xi);
-        const float opxi = 1.f + xi;
-        const float inv_opxi = f_rcp_n(opxi);
-        // branch thresholds of the reference (1e3, 1e-3) must be taken as it takes them
-        edge |= fabsf(xi - 1e3f) <= 2e-4f || fabsf(xi - 1e-3f) <= 2e-10f;
+    float eps, rho;
+    f_exp_split_ff(kF8XH[j], kF8XL[j], tmin, tmin_lo, eps, rho);
+    rho = -rho;
+    const float rho2 = rho * rho;
+    const float rho21 = eps * (2.f - eps);
+    const float xi = xi_factor * rho21;
+    const float xi_i = f_rcp_n(xi);
+    const float opxi = 1.f + xi;
+    const float inv_opxi = f_rcp_n(opxi);
+    // branch thresholds of the reference (1e3, 1e-3) must be taken as it takes them
+    edge |= fabsf(xi - 1e3f) <= 2e-4f || fabsf(xi - 1e-3f) <= 2e-10f;
 
-        // One H and one log1p a node serve both screening functions: Be takes
-        // log(1 + 1/xi) and Bmu log(1 + xi), one of them at u = min(xi, 1/xi),
-        // from H, and the other at 1/u.  As branches of their own, the lanes of
-        // a warp on either side of xi = 1 made it run two of each.
-        const bool above = xi >= 1.f;
-        const float u = above ? xi_i : xi;
-        const float Gs = u * poly_H(u);                     // log1p(u)/u - 1
-        const float Ls = u * (1.f + Gs);                    // log1p(u)
-        const float Ll = log1pf(above ? xi : xi_i);         // log1p(1/u)
-        const float Gl = fmaf(Ll, u, -1.f);                 // u log1p(1/u) - 1
+    // One H and one log1p a node serve both screening functions: Be takes
+    // log(1 + 1/xi) and Bmu log(1 + xi), one of them at u = min(xi, 1/xi),
+    // from H, and the other at 1/u.  As branches of their own, the lanes of
+    // a warp on either side of xi = 1 made it run two of each.
+    const bool above = xi >= 1.f;
+    const float u = above ? xi_i : xi;
+    const float Gs = u * poly_H(u);                     // log1p(u)/u - 1
+    const float Ls = u * (1.f + Gs);                    // log1p(u)
+    const float Ll = log1pf(above ? xi : xi_i);         // log1p(1/u)
+    const float Gl = fmaf(Ll, u, -1.f);                 // u log1p(1/u) - 1
 
-        float Be, eBe;
-        if (xi >= 1E+03f) {
-            Be = 0.5f * xi_i * ((3.f - rho2) + b2 * (1.f + rho2));
-            eBe = 2.f * U32 * Be;
-        } else {
-            const float A = (2.f + rho2) * (1.f + beta);
-            const float L = above ? Ls : Ll;  // log(1 + 1/xi)
-            const float G = above ? Gs : Gl;  // xi L - 1
-            const float t1 = A * L, t2 = (3.f + rho2) * G, t3 = (rho21 - beta) * inv_opxi;
-            Be = t1 + t2 + t3;
-            eBe = 2.f * U32 * (fabsf(t1) + fabsf(t2) + fabsf(t3) + fabsf(beta) * inv_opxi);
-        }
-        const float Ye = f_div_n(5.f - rho2 + b4 * (1.f + rho2), 2.f * (1.f + b3) * logf(3.f + xi_i) - rho2 -
-                                                                  b2 * (2.f - rho2));
-        const float xe = opxi * (1.f + Ye);
-        const float cLi = cL * f_rcp_n(rho21);
-        float Le;
-        if (FINE) {
-            // Le = log(AZ13 q sqrt(xe) / D1) - log(D2) / 2 (dcs.hh:199-202) as one
-            // float-float log of AZ13^2 q^2 xe / (D1^2 D2)
-            const FF epsF = ff_exp(ff_mul(FF{kF8XH[j], kF8XL[j]}, tminF));
-            const FF rhoF = ff_add(1.f, ff_neg(epsF));
-            const FF rho2F = ff_mul(rhoF, rhoF);
-            const FF r21F = ff_mul(epsF, ff_add(2.f, ff_neg(epsF)));
-            const FF xiF = ff_mul(xfF, r21F);
-            const FF L3 = ff_log(ff_add(3.f, ff_div(FF{1.f, 0.f}, xiF)));
-            const FF num = ff_add(ff_add(5.f, ff_neg(rho2F)), ff_mul(ff_mul(4.f, betaF), ff_add(1.f, rho2F)));
-            const FF den = ff_add(ff_add(ff_mul(ff_mul(2.f, ff_add(1.f, ff_mul(3.f, betaF))), L3), ff_neg(rho2F)),
-                                  ff_neg(ff_mul(ff_mul(2.f, betaF), ff_add(2.f, ff_neg(rho2F)))));
-            const FF xeF = ff_mul(ff_add(1.f, xiF), ff_add(1.f, ff_div(num, den)));
-            const FF d1 = ff_add(qF, ff_mul(ff_div(cLF, r21F), xeF));
-            const FF lg = ff_log(ff_div(ff_mul(aq2F, xeF), ff_mul(ff_mul(d1, d1), ff_add(1.f, ff_mul(cLeF, xeF)))));
-            Le = 0.5f * (lg.h + lg.l);
-        } else {
-            const float r1 = AZ13 * qf * f_rcp_n(qf + cLi * xe);
-            const float r2 = xe * f_rcp_n(1.f + cLe * xe);
-            Le = 0.5f * logf(r1 * r1 * r2);
-        }
-        const float Phi_e = f_clamp0(Be * Le);
-
-        float Bmu, eBmu;
-        if (xi <= 1E-03f) {
-            Bmu = 0.5f * xi * (5.f - rho2 + beta * (3.f + rho2));
-            eBmu = 2.f * U32 * Bmu;
-        } else {
-            const float L1 = xi > 1.f ? Ll : Ls;  // log(1 + xi)
-            const float G2 = xi > 1.f ? Gl : Gs;  // L1 / xi - 1
-            const float s1 = (1.f + rho2) * (1.f + b15) * L1, s2 = (1.f + b2) * rho21 * G2,
-                        s3 = xi * (rho21 - beta) * inv_opxi;
-            Bmu = s1 - s2 + s3;
-            eBmu = 2.f * U32 * (fabsf(s1) + fabsf(s2) + fabsf(s3) + xi * fabsf(beta) * inv_opxi);
-        }
-        const float Ymu = f_div_n(4.f + rho2 + b3 * (1.f + rho2),
-                                (1.f + rho2) * (1.5f + b2) * logf(3.f + xi) + 1.f - 1.5f * rho2);
-        const float xmu = opxi * (1.f + Ymu);
-        const float Lmu = logf(rAZ13 * qf * f_rcp_n(Z13_15 * (qf + cLi * xmu)));
-        const float Phi_mu = f_clamp0(Bmu * Lmu);
-        const float g = -(Phi_e + Phi_mu * inv_r2) * eps * tmin;
-        I.add(g * kF8W[j]);
-        // error of this node: the logs to a few u absolute (Le 3 u, or 0.5 u
-        // relative when FINE; Lmu 4 u: its argument carries the float error of
-        // xmu), the B terms as tracked, the rest ~3 u relative
-        const float eg = fabsf(eps * tmin) *
-                         ((Phi_e > 0.f ? fabsf(Be) * (FINE ? fabsf(Le) : 3.f) * U32 + fabsf(Le) * eBe : 0.f) +
-                          (Phi_mu > 0.f ? (fabsf(Bmu) * 4.f * U32 + fabsf(Lmu) * eBmu) * inv_r2 : 0.f)) +
-                         fabsf(g) * 3.f * U32;
-        err += eg * kF8W[j];
-        // a screening log near zero decides the clamp; let FP64 decide it
-        edge |= (fabsf(Le) < 64.f * U32) || (fabsf(Lmu) < 64.f * U32);
+    float Be, eBe;
+    if (xi >= 1E+03f) {
+        Be = 0.5f * xi_i * ((3.f - rho2) + b2 * (1.f + rho2));
+        eBe = 2.f * U32 * Be;
+    } else {
+        const float A = (2.f + rho2) * (1.f + beta);
+        const float L = above ? Ls : Ll;  // log(1 + 1/xi)
+        const float G = above ? Gs : Gl;  // xi L - 1
+        const float t1 = A * L, t2 = (3.f + rho2) * G, t3 = (rho21 - beta) * inv_opxi;
+        Be = t1 + t2 + t3;
+        eBe = 2.f * U32 * (fabsf(t1) + fabsf(t2) + fabsf(t3) + fabsf(beta) * inv_opxi);
     }
+    const float Ye = f_div_n(5.f - rho2 + b4 * (1.f + rho2), 2.f * (1.f + b3) * logf(3.f + xi_i) - rho2 -
+                                                              b2 * (2.f - rho2));
+    const float xe = opxi * (1.f + Ye);
+    const float cLi = cL * f_rcp_n(rho21);
+    float Le;
+    if constexpr (FINE) {
+        // Le = log(AZ13 q sqrt(xe) / D1) - log(D2) / 2 (dcs.hh:199-202) as one
+        // float-float log of AZ13^2 q^2 xe / (D1^2 D2)
+        const FF epsF = ff_exp(ff_mul(FF{kF8XH[j], kF8XL[j]}, p.tmin));
+        const FF rhoF = ff_add(1.f, ff_neg(epsF));
+        const FF rho2F = ff_mul(rhoF, rhoF);
+        const FF r21F = ff_mul(epsF, ff_add(2.f, ff_neg(epsF)));
+        const FF xiF = ff_mul(p.xfF, r21F);
+        const FF L3 = ff_log(ff_add(3.f, ff_div(FF{1.f, 0.f}, xiF)));
+        const FF num = ff_add(ff_add(5.f, ff_neg(rho2F)), ff_mul(ff_mul(4.f, p.betaF), ff_add(1.f, rho2F)));
+        const FF den = ff_add(ff_add(ff_mul(ff_mul(2.f, ff_add(1.f, ff_mul(3.f, p.betaF))), L3), ff_neg(rho2F)),
+                              ff_neg(ff_mul(ff_mul(2.f, p.betaF), ff_add(2.f, ff_neg(rho2F)))));
+        const FF xeF = ff_mul(ff_add(1.f, xiF), ff_add(1.f, ff_div(num, den)));
+        const FF d1 = ff_add(p.qF, ff_mul(ff_div(FF{cL, c.pp_cL_l}, r21F), xeF));
+        const FF d2 = ff_add(1.f, ff_mul(FF{cLe, c.pp_cLe_l}, xeF));
+        const FF lg = ff_log(ff_div(ff_mul(p.aq2F, xeF), ff_mul(ff_mul(d1, d1), d2)));
+        Le = 0.5f * (lg.h + lg.l);
+    } else {
+        const float r1 = AZ13 * qf * f_rcp_n(qf + cLi * xe);
+        const float r2 = xe * f_rcp_n(1.f + cLe * xe);
+        Le = 0.5f * logf(r1 * r1 * r2);
+    }
+    const float Phi_e = f_clamp0(Be * Le);
 
+    float Bmu, eBmu;
+    if (xi <= 1E-03f) {
+        Bmu = 0.5f * xi * (5.f - rho2 + beta * (3.f + rho2));
+        eBmu = 2.f * U32 * Bmu;
+    } else {
+        const float L1 = xi > 1.f ? Ll : Ls;  // log(1 + xi)
+        const float G2 = xi > 1.f ? Gl : Gs;  // L1 / xi - 1
+        const float s1 = (1.f + rho2) * (1.f + b15) * L1, s2 = (1.f + b2) * rho21 * G2,
+                    s3 = xi * (rho21 - beta) * inv_opxi;
+        Bmu = s1 - s2 + s3;
+        eBmu = 2.f * U32 * (fabsf(s1) + fabsf(s2) + fabsf(s3) + xi * fabsf(beta) * inv_opxi);
+    }
+    const float Ymu = f_div_n(4.f + rho2 + b3 * (1.f + rho2),
+                            (1.f + rho2) * (1.5f + b2) * logf(3.f + xi) + 1.f - 1.5f * rho2);
+    const float xmu = opxi * (1.f + Ymu);
+    const float Lmu = logf(rAZ13 * qf * f_rcp_n(Z13_15 * (qf + cLi * xmu)));
+    const float Phi_mu = f_clamp0(Bmu * Lmu);
+    const float g = -(Phi_e + Phi_mu * inv_r2) * eps * tmin;
+    // error of this node: the logs to a few u absolute (Le 3 u, or 0.5 u
+    // relative when FINE; Lmu 4 u: its argument carries the float error of
+    // xmu), the B terms as tracked, the rest ~3 u relative
+    const float eg = fabsf(eps * tmin) *
+                     ((Phi_e > 0.f ? fabsf(Be) * (FINE ? fabsf(Le) : 3.f) * U32 + fabsf(Le) * eBe : 0.f) +
+                      (Phi_mu > 0.f ? (fabsf(Bmu) * 4.f * U32 + fabsf(Lmu) * eBmu) * inv_r2 : 0.f)) +
+                     fabsf(g) * 3.f * U32;
+    // a screening log near zero decides the clamp; let FP64 decide it
+    edge |= (fabsf(Le) < 64.f * U32) || (fabsf(Lmu) < 64.f * U32);
+    eg_out = edge ? INFINITY : eg;
+    return g;
+}
+
+// The sum's scaling and the estimate of its relative error.
+NOA_HD double pprod32_finish(double K, double q, const KSum &I, float err, const noa_dcs_consts &c, float &est) {
+    const double mass = c.mass;
+    const double E = K + mass;
+    const double Emq = E - q;
+    bool edge = false;
     const double gamma = 1. + K * c.inv_mass;
     // zeta (dcs.hh:230-251) in float, with a bound on its float error; where
     // the cancellations in its numerator or denominator make that bound
@@ -469,6 +471,36 @@ NOA_HD double pprod_fp32c(double K, double q, const noa_dcs_consts &c, float &es
     est = edge ? INFINITY : 1.2f * err * f_rcp(fpconv::f32_normal(fabs(Id))) + zeta_err * f_rcp(c.Zd_f + zeta);
     const double dcs = c.pp_cZ * (c.Zd + fpconv::f64(zeta)) * Emq * Id * d_rcp(q * E);
     return (dcs < 0.) ? 0. : dcs * (mass + K) * c.scale_A;
+}
+
+template <bool CHECKED = true, bool FINE = false>
+NOA_HD double pprod_fp32c(double K, double q, const noa_dcs_consts &c, float &est) {
+    est = 0.f;
+    FF argmin;
+    if (CHECKED) {
+        if (q <= 4. * ME)
+            return 0.;
+        if (q >= K + c.pp_kmax_shift)
+            return 0.;
+        const double a = pprod_argmin_exact(K, q, c);
+        if ((a >= 1.) || (a <= 0.))
+            return 0.;
+        argmin = ff_from(a);
+    } else {
+        argmin = pprod_argmin_ff(K, q, c);
+    }
+    Pprod32<FINE> p;
+    pprod32_setup<FINE>(K, q, argmin, c, p);
+    KSum I;
+    float err = 0.f;
+    NOA_UNROLL_NODES
+    for (int j = 0; j < 8; j++) {
+        float eg;
+        const float g = pprod32_node<FINE>(p, j, c, eg);
+        I.add(g * kF8W[j]);
+        err += eg * kF8W[j];
+    }
+    return pprod32_finish(K, q, I, err, c, est);
 }
 
 // ---------------------------------------------------------------- photonuclear
