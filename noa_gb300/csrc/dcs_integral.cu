@@ -20,10 +20,11 @@
  * warp per K then sums its nodes in a fixed order, so the result does not
  * depend on scheduling.
  *
- * kpt and the CTA's width follow the number of energies: a table of 146
- * energies has one energy a CTA and 512 threads on it (a 9-node photonuclear
- * batch of 8 energies in 256 threads kept 19 of 152 SMs busy for 740 us); a
- * fine grid has 8 energies a CTA of 128 threads, five or six CTAs an SM.
+ * kpt and the CTA's width follow the number of energies (integral_width): a
+ * table of 146 energies has one energy a CTA and up to 1024 threads on it (a
+ * 9-node photonuclear batch of 8 energies in 256 threads kept 19 of 152 SMs
+ * busy for 740 us); a fine grid has 8 energies a CTA of 128 threads, five or
+ * six CTAs an SM.
  */
 #include "dcs_quad.cuh"
 
@@ -34,9 +35,14 @@ namespace noa_dcs {
 constexpr int I_PAIRS = 1536;  // pairs per tile (kpt * nodes <= I_PAIRS)
 constexpr int I_KMAX = 128;    // kinetic energies per tile at most
 
-constexpr int I_BATCH = 128;   // pairs per batch of the quadrature processes
-constexpr int I_NARROW = 128;  // CTA widths: many energies / at most one per SM
-constexpr int I_WIDE = 512;
+// CTA widths: many energies / at most two per SM / at most one.
+constexpr int I_NARROW = 128, I_MID = 256, I_WIDE = 1024;
+// Pairs per batch of the quadrature processes -- all nodes of an energy in the
+// wider CTAs (180 and 300 nodes are usual), as each batch waits once for its
+// pairs' setup and once for their end -- and the resident CTAs that the
+// kernels are compiled for.
+constexpr int i_batch(int threads) { return threads == I_WIDE ? 320 : (threads == I_MID ? 192 : 128); }
+constexpr int i_ctas(int threads) { return threads == I_WIDE ? 1 : (threads == I_MID ? 2 : 5); }
 
 __constant__ double kGL6X[6] = {0.03376524, 0.16939531, 0.38069041, 0.61930959, 0.83060469, 0.96623476};
 __constant__ double kGL6W[6] = {0.08566225, 0.18038079, 0.23395697, 0.23395697, 0.18038079, 0.08566225};
@@ -117,9 +123,10 @@ __device__ __forceinline__ double warp_node_sum(const double *v, int nodes) {
 }
 
 template <int PROC, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == I_NARROW ? 5 : 1)
+__global__ void __launch_bounds__(THREADS, i_ctas(THREADS))
     recoil_integral_kernel(const IntegralParams p, const noa_dcs_consts c) {
     extern __shared__ double vals[];          // weighted node values of the tile, [k][node]
+    constexpr int I_BATCH = i_batch(THREADS);
     __shared__ double qQ[I_BATCH + THREADS];  // queued recoil energies
     __shared__ int qS[I_BATCH + THREADS];     // their slots in vals
     __shared__ QuadSmem<PROC, I_BATCH> quad;
@@ -288,8 +295,9 @@ __device__ __forceinline__ void soft_node(double K, int i, const SoftParams &p, 
 }
 
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == I_NARROW ? 5 : 1)
+__global__ void __launch_bounds__(THREADS, i_ctas(THREADS))
     soft_scattering_kernel(const SoftParams p, const noa_dcs_consts c) {
+    constexpr int I_BATCH = i_batch(THREADS);
     __shared__ double vals[S_KMAX * S_NODES];
     __shared__ int qS[I_BATCH + THREADS];
     __shared__ QuadSmem<NOA_DCS_PROC_PHOTO, I_BATCH> quad;
@@ -386,6 +394,25 @@ int energies_per_tile(int64_t n, int64_t sms, int most) {
     return (int)(k < 1 ? 1 : (k > most ? most : k));
 }
 
+// The width for n energies of `nodes` nodes.  Up to one an SM a CTA has the SM
+// for itself: the (pair, node) rounds of the quadrature processes shrink up to
+// 1024 threads (pair production / photonuclear, 146 energies of 180 nodes:
+// 54.9 / 70.0 us at 128 threads, 34.0 / 46.4 at 256, 27.3 / 39.3 at 512, 26.8 /
+// 36.4 at 1024), while bremsstrahlung, ionisation and soft scattering, which
+// wait for one or two rounds of usual node counts, are as fast at 256 as above
+// (9.8, 10.1 and 26.0 us).  Up to two an SM both are resident at 256 (304
+// energies: 43.3 / 63.0 us against 60.5 / 80.9 at 128 and 51.3 / 69.6 at 1024);
+// a quadrature's batch of 192 leaves room for 4 KB of node values there.
+// Above, 128 threads leave room for five (456 energies: 14.5 us of
+// bremsstrahlung against 19.8 at 256).
+constexpr int I_MID_NODES = 512;
+int integral_width(bool quadrature, int nodes, int64_t n, int64_t sms) {
+    const bool few = nodes <= I_MID_NODES;
+    if (n <= sms)
+        return quadrature || !few ? I_WIDE : I_MID;
+    return n <= 2 * sms && (few || !quadrature) ? I_MID : I_NARROW;
+}
+
 template <int THREADS>
 cudaError_t launch_recoil(int process, const IntegralParams &p, const noa_dcs_consts &c, cudaStream_t stream) {
     const int64_t tiles = (p.n + p.kpt - 1) / p.kpt;
@@ -430,8 +457,14 @@ cudaError_t noa_dcs_launch_recoil_integral(int process, int moment, const double
     const int most = p.nodes >= I_PAIRS / 2 ? 1 : I_PAIRS / 2 / p.nodes;
     p.kpt = energies_per_tile(n, sms, most < I_KMAX ? most : I_KMAX);
     p.moment = moment;
-    return n <= sms ? launch_recoil<I_WIDE>(process, p, *c, stream)
-                    : launch_recoil<I_NARROW>(process, p, *c, stream);
+    switch (integral_width(is_quad(process), p.nodes, n, sms)) {
+    case I_WIDE:
+        return launch_recoil<I_WIDE>(process, p, *c, stream);
+    case I_MID:
+        return launch_recoil<I_MID>(process, p, *c, stream);
+    default:
+        return launch_recoil<I_NARROW>(process, p, *c, stream);
+    }
 }
 
 cudaError_t noa_dcs_launch_soft_scattering(const double *K, double *out, int64_t n, const noa_dcs_consts *c,
@@ -448,8 +481,8 @@ cudaError_t noa_dcs_launch_soft_scattering(const double *K, double *out, int64_t
     p.kpt = energies_per_tile(n, sms, S_KMAX);
     const int64_t tiles = (n + p.kpt - 1) / p.kpt;
     const int grid = (int)(tiles < (1 << 30) ? tiles : (1 << 30));
-    if (n <= sms)
-        soft_scattering_kernel<I_WIDE><<<grid, I_WIDE, 0, stream>>>(p, *c);
+    if (integral_width(false, S_NODES, n, sms) == I_MID)
+        soft_scattering_kernel<I_MID><<<grid, I_MID, 0, stream>>>(p, *c);
     else
         soft_scattering_kernel<I_NARROW><<<grid, I_NARROW, 0, stream>>>(p, *c);
     return cudaGetLastError();
