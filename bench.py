@@ -598,13 +598,14 @@ def load_traffic():
 
 def hw_view(process):
     """The hardware view of the roofline for one FP64 kernel: ncu's pipe
-    utilisations of a 1e7-pair launch (profiles/traffic.json), the FP64 pipe
-    being the bound."""
+    utilisations of a 1e7-pair launch (profiles/traffic.json).  frac is that of
+    the pipe that `bound` names; the two quadratures keep the issue slots and
+    the ALU pipe as busy (pipes), so that no single one bounds them."""
     pipes = load_traffic().get("pipes_fp64_1e7", {}).get(process)
     if not pipes:
         return None
     return {"bound": "fp64 pipe", "frac": pipes["fp64_pipe"], "pipes": pipes,
-            "source": "ncu --set full of one 1e7-pair launch (profiles/dcs_fp64_1e8.md)"}
+            "source": "ncu, one 1e7-pair launch (profiles/dcs_fp64_1e8.md)"}
 
 
 def run_ours(args):
@@ -758,8 +759,8 @@ def run_ours(args):
                                     "this run",
                      "numerator": f"{FLOP_EQ_PER_EVAL[dom]} flop-eq/eval x {n} evals per launch",
                      "convention": "flop-eq counted on the oracle, each libm log/exp/pow = 20; the kernels "
-                                   "compute log/exp/reciprocal mostly on the integer and FP32 pipes (1/2/0 FP64 "
-                                   "instructions), so frac can exceed 1; hw_view is the hardware roofline",
+                                   "compute log/exp/reciprocal and most products between them on the integer and "
+                                   "FP32 pipes, so frac can exceed 1; hw_view is the hardware roofline",
                      "hw_view": hw_view(dom)},
         "per_process": per_process,
         "variants": variants,

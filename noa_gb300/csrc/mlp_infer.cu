@@ -1,5 +1,5 @@
 /*
- * Learned DCS surrogate, inference (noa_dcs_mlp_infer): four kernels on the
+ * Learned DCS surrogate, inference (noa_dcs_mlp_infer): three kernels on the
  * caller's stream.
  *
  *  1. classify: per pair, the kinematic bounds decided as the FP64 kernels
