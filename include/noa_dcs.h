@@ -203,7 +203,7 @@ const char *noa_dcs_batch_last_error(void);
  * on the GPU (different streams, or different host threads) race and must be
  * serialised by the caller.  Set-up on the first call on each device: the
  * array's device address is looked up with that device current, and for
- * FP32C pair production (54 KB of shared memory) the kernel's shared-memory
+ * FP32C pair production (83 KB of shared memory) the kernel's shared-memory
  * limit is raised; later calls make no runtime set-up call.  Tile
  * shape is fixed (256 threads x 4 pairs, 2 CTAs per SM).  Buffers as for the
  * plan. */

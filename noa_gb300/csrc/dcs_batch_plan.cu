@@ -463,8 +463,8 @@ extern "C" int noa_dcs_cuda_vmap_batched_noalloc(int process, int precision, int
         noa_dcs_fill_consts(&p.params.consts[s], elements[s].A, elements[s].I, elements[s].Z, mass);
     }
     // Fixed tile shape (the plan default): 256 threads x 4 pairs, 2 CTAs per
-    // SM.  Its queues take 43 KB of shared memory, 54 KB for FP32C pair
-    // production (a third queue); above 48 KB the launch raises the kernel's
+    // SM.  Its queues take 43 KB of shared memory, 83 KB for FP32C pair
+    // production (a third queue and its float-float step's nodes); above 48 KB the launch raises the kernel's
     // limit once per device, on its first call there.
     p.threads = 256;
     p.items = 4;

@@ -28,6 +28,7 @@
 #pragma once
 
 #include "dcs_fp32c.cuh"
+#include "dcs_fp32c_batch.cuh"
 #include "dcs_quad.cuh"
 
 #include <atomic>
@@ -84,7 +85,8 @@ __host__ __device__ constexpr bool batch_third_queue(int proc, int prec) {
 // pairs); for FP32C the redo queue (2*THREADS), and for its pair production
 // the third queue (2*THREADS) of the pairs its float-float redo step still
 // rejects; for the quadrature processes the batch of quad_batch (FP64) or
-// quad_redo (FP32C).
+// quad_redo (FP32C), in the same place as that of pair production's
+// float-float step.
 template <int THREADS>
 struct BatchSmem {
     static constexpr size_t pair_bytes = 2 * sizeof(double) + sizeof(int64_t);
@@ -92,11 +94,16 @@ struct BatchSmem {
         return pair_bytes * THREADS *
                (items + 1 + (prec != NOA_DCS_FP64 ? 2 : 0) + (batch_third_queue(proc, prec) ? 2 : 0));
     }
+    static __host__ __device__ constexpr size_t fine_or_redo() {
+        return sizeof(Pprod32Smem<THREADS>) > sizeof(QuadSmem<NOA_DCS_PROC_PPROD, QUAD_REDO>)
+                   ? sizeof(Pprod32Smem<THREADS>)
+                   : sizeof(QuadSmem<NOA_DCS_PROC_PPROD, QUAD_REDO>);
+    }
     static __host__ __device__ constexpr size_t bytes(int items, int proc, int prec) {
         return queues(items, proc, prec) +
                (proc == NOA_DCS_PROC_PPROD
                     ? (prec == NOA_DCS_FP64 ? sizeof(QuadSmem<NOA_DCS_PROC_PPROD, THREADS>)
-                                            : sizeof(QuadSmem<NOA_DCS_PROC_PPROD, QUAD_REDO>))
+                                            : fine_or_redo())
                     : 0) +
                (proc == NOA_DCS_PROC_PHOTO
                     ? (prec == NOA_DCS_FP64 ? sizeof(QuadSmem<NOA_DCS_PROC_PHOTO, THREADS>)
@@ -124,12 +131,15 @@ __device__ __forceinline__ void batch_push(bool push, double k, double q, int64_
     }
 }
 
-// Pair production, FP32C: evaluates redo-queue entry e (if valid) with the
-// float-float screening log; pairs whose estimate still exceeds tol go to the
-// third queue.
-__device__ __forceinline__ bool batch_fine_step(double *rK, double *rQ, int64_t *rI, double *xK, double *xQ,
-                                                int64_t *xI, int *xn, int e, bool valid, double *out,
-                                                const noa_dcs_consts &c, float tol) {
+// Pair production, FP32C: evaluates `take` redo-queue entries from `at` with the
+// float-float screening log, one (pair, node) a thread; pairs whose estimate
+// still exceeds tol go to the third queue (true for this thread's).
+template <int THREADS>
+__device__ __forceinline__ bool batch_fine_step(Pprod32Smem<THREADS> &s, double *rK, double *rQ, int64_t *rI,
+                                                double *xK, double *xQ, int64_t *xI, int *xn, int at, int take,
+                                                double *out, const noa_dcs_consts &c, float tol) {
+    const int e = at + threadIdx.x;
+    const bool valid = (int)threadIdx.x < take;
     bool redo = false;
     double k = 0., q = 0.;
     int64_t i = 0;
@@ -137,8 +147,10 @@ __device__ __forceinline__ bool batch_fine_step(double *rK, double *rQ, int64_t 
         k = rK[e];
         q = rQ[e];
         i = rI[e];
-        float est;
-        const double v = pprod_fp32c<false, true>(k, q, c, est);
+    }
+    float est;
+    const double v = pprod32_batch<true>(s, take, k, q, c, est);
+    if (valid) {
         redo = !(est <= tol);
         if (!redo)
             out[i] = v;
@@ -258,8 +270,8 @@ __global__ void __launch_bounds__(THREADS) dcs_batched_kernel(const __grid_const
                         if (threadIdx.x == 0)
                             s_rn = rn;
                         if constexpr (third) {
-                            rejected = batch_fine_step(rK, rQ, rI, xK, xQ, xI, &s_xn, rn + threadIdx.x,
-                                                       (int)threadIdx.x < take, p.out, cc, p.tol);
+                            rejected = batch_fine_step(*reinterpret_cast<Pprod32Smem<THREADS> *>(&quad), rK, rQ, rI,
+                                                       xK, xQ, xI, &s_xn, rn, take, p.out, cc, p.tol);
                             xn += __syncthreads_count(rejected);
                             while (xn >= QUAD_REDO || (flush && qn == 0 && rn == 0 && xn > 0)) {
                                 const int some = xn < QUAD_REDO ? xn : QUAD_REDO;

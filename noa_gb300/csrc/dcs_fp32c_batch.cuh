@@ -22,7 +22,9 @@ struct Pprod32Smem {
 // thread a pair, the 22 or so redo pairs that a CTA has left at the end of a
 // call kept it waiting for eight float-float nodes in a row: 1000 / 60013 /
 // 250007 pairs of iron 26.7 / 39.8 / 53.4 us, now 16.8 / 29.8 / 43.8 (1e7 pairs
-// unchanged).  The float form gains less (14.3 / 28.3 / 44.4 us) and loses 6%
+// unchanged); the batched engine with ten elements, which ends a step at each
+// element, at 1000 / 1e5 / 1e6 / 1e7 pairs 42.8 / 47.0 / 211 / 1191 -> 34.7 /
+// 38.5 / 183 / 1159.  The float form gains less (14.3 / 28.3 / 44.4 us) and loses 6%
 // at 1e7 pairs to the round trip through shared memory, so it keeps one thread
 // a pair.  Called by every thread; the caller synchronises before the next
 // call.
