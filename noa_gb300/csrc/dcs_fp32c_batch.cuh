@@ -28,15 +28,16 @@ struct Pprod32Smem {
 // at 1e7 pairs to the round trip through shared memory, so it keeps one thread
 // a pair.  Called by every thread; the caller synchronises before the next
 // call.
-template <bool FINE, int THREADS>
-__device__ __forceinline__ double pprod32_batch(Pprod32Smem<THREADS> &s, int take, double K, double q,
-                                                const noa_dcs_consts &c, float &est) {
+// consts(e) are the constants of pair e's element.
+template <bool FINE, int THREADS, typename Consts>
+__device__ __forceinline__ double pprod32_batch_mixed(Pprod32Smem<THREADS> &s, int take, double K, double q,
+                                                      Consts consts, float &est) {
     constexpr int WORDS = sizeof(Pprod32<FINE>) / sizeof(float);
     const int t = threadIdx.x;
     Pprod32<FINE> p;
     float *w = reinterpret_cast<float *>(&p);
     if (t < take) {
-        pprod32_setup<FINE>(K, q, pprod_argmin_ff(K, q, c), c, p);
+        pprod32_setup<FINE>(K, q, pprod_argmin_ff(K, q, consts(t)), consts(t), p);
 #pragma unroll
         for (int i = 0; i < WORDS; i++)
             s.pair[i][t] = w[i];
@@ -49,7 +50,7 @@ __device__ __forceinline__ double pprod32_batch(Pprod32Smem<THREADS> &s, int tak
         for (int i = 0; i < WORDS; i++)
             w[i] = s.pair[i][e];
         float eg;
-        s.g[j][e] = pprod32_node<FINE>(p, j, c, eg);
+        s.g[j][e] = pprod32_node<FINE>(p, j, consts(e), eg);
         s.e[j][e] = eg;
     }
     __syncthreads();
@@ -63,7 +64,14 @@ __device__ __forceinline__ double pprod32_batch(Pprod32Smem<THREADS> &s, int tak
         I.add(s.g[j][t] * kF8W[j]);
         err += s.e[j][t] * kF8W[j];
     }
-    return pprod32_finish(K, q, I, err, c, est);
+    return pprod32_finish(K, q, I, err, consts(t), est);
+}
+
+// All pairs of one element.
+template <bool FINE, int THREADS>
+__device__ __forceinline__ double pprod32_batch(Pprod32Smem<THREADS> &s, int take, double K, double q,
+                                                const noa_dcs_consts &c, float &est) {
+    return pprod32_batch_mixed<FINE>(s, take, K, q, [&](int) -> const noa_dcs_consts & { return c; }, est);
 }
 
 } // namespace noa_dcs

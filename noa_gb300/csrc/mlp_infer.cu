@@ -36,6 +36,7 @@
  * flight one more bounded wait, frees its TMEM and returns.
  */
 #include "dcs_fp32c.cuh"
+#include "dcs_fp32c_batch.cuh"
 #include "dcs_fp64.cuh"
 #include "dcs_launch.h"
 #include "dcs_quad.cuh"
@@ -301,6 +302,13 @@ static __device__ __noinline__ void quad_redo_listed(noa_dcs::QuadSmem<PROC, noa
 // kernel a form without barriers), photonuclear 231 / 233 / 238.
 __host__ __device__ constexpr int fb_threads(int proc) { return proc == NOA_DCS_PAIR_PRODUCTION ? 512 : 256; }
 constexpr int FB_WARPS = 32;  // per SM
+// Pair production's float-float step, one (pair, node) a thread: all-fallback
+// calls of 4e4 / 4e5 queries 130 / 165 -> 114 / 150 us against one thread a pair
+// (4e6 and 1e7 within 1%).
+template <int PROC>
+struct FineSmem {};
+template <>
+struct FineSmem<NOA_DCS_PAIR_PRODUCTION> : noa_dcs::Pprod32Smem<fb_threads(NOA_DCS_PAIR_PRODUCTION)> {};
 template <int PROC>
 __global__ void __launch_bounds__(fb_threads(PROC), FB_WARPS * 32 / fb_threads(PROC))
     fallback_kernel(const __grid_constant__ InferParams p) {
@@ -314,6 +322,7 @@ __global__ void __launch_bounds__(fb_threads(PROC), FB_WARPS * 32 / fb_threads(P
     __shared__ int32_t rq[redo_batch + FB_THREADS], xq[fine ? QUAD_REDO + FB_THREADS : 1];
     __shared__ uint8_t rs[redo_batch + FB_THREADS], xs[fine ? QUAD_REDO + FB_THREADS : 1];
     __shared__ noa_dcs::QuadSmem<PROC, QUAD_REDO> quad;
+    __shared__ FineSmem<PROC> nodes;
     __shared__ int rn_next, xn_next;
     if (threadIdx.x == 0) {
         rn_next = 0;
@@ -358,11 +367,17 @@ __global__ void __launch_bounds__(fb_threads(PROC), FB_WARPS * 32 / fb_threads(P
                 bool again = false;
                 int32_t j = 0;
                 uint8_t sj = 0;
+                double K = 0., q = 0.;
                 if ((int)threadIdx.x < take) {
                     j = rq[rn + threadIdx.x];
                     sj = rs[rn + threadIdx.x];
-                    float est;
-                    const double v = noa_dcs::pprod_fp32c<false, true>(p.K[j], p.q[j], p.consts[sj], est);
+                    K = p.K[j];
+                    q = p.q[j];
+                }
+                float est;
+                const double v = noa_dcs::pprod32_batch_mixed<true>(
+                    nodes, take, K, q, [&](int e) -> const noa_dcs_consts & { return p.consts[rs[rn + e]]; }, est);
+                if ((int)threadIdx.x < take) {
                     again = !(est <= p.tol);
                     if (!again)
                         p.out[j] = v;
