@@ -154,55 +154,82 @@ __global__ void __launch_bounds__(C_THREADS) coulomb_data_kernel(const double *_
     }
 }
 
-// dcs.hh:624-677
-__device__ __forceinline__ void transport_coefficients(double *coefs, const double *ps, double fspin, double mu) {
-    const double nuclear_screening = (ps[1] < ps[2]) ? ps[1] : ps[2];
-    if (mu < 1E-08 * nuclear_screening) {
-        const double L = log(1. + qdiv(mu, ps[0]));
-        const double r = qdiv(mu, mu + ps[0]);
-        const double k = ps[0] * (1. + ps[0]);
-        coefs[0] = k * (qdiv(r, ps[0]) - fspin * (L - r));
-        const double I2 = mu - ps[0] * (r - 2. * L);
-        coefs[1] = 2. * k * (L - r - fspin * I2);
-        return;
-    }
-    const double mu2 = 0.5 * mu * mu;
-    double c0 = 0., c1 = 0.;
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        double r = qdiv(mu, mu + ps[i]);
-        double L = log(1. + qdiv(mu, ps[i]));
-        double mu1 = mu;
-        const double I0 = qdiv(r, ps[i]);
-        const double J0 = L;
-        const double I1 = L - r;
-        r *= ps[i];
-        L *= ps[i];
-        const double J1 = mu1 - L;
-        const double I2 = mu1 - 2. * L + r;
-        L *= ps[i];
-        mu1 *= ps[i];
-        const double J2 = mu2 + L - mu1;
-        c0 += ps[3 + i] * (J0 - fspin * J1) + ps[6 + i] * (I0 - fspin * I1);
-        c1 += ps[3 + i] * (J1 - fspin * J2) + ps[6 + i] * (I1 - fspin * I2);
-    }
-    const double k = ps[0] * (1. + ps[0]) * ps[1] * ps[1] * ps[2] * ps[2];
-    coefs[0] = c0 * k;
-    coefs[1] = c1 * (2. * k);
+// Pole i's share of the coefficients, dcs.hh:639-672: s = screen[i], a and b its
+// factors.
+__device__ __forceinline__ void transport_term(double s, double a, double b, double fspin, double mu, double mu2,
+                                               double &t0, double &t1) {
+    double r = qdiv(mu, mu + s);
+    double L = log(1. + qdiv(mu, s));
+    double mu1 = mu;
+    const double I0 = qdiv(r, s);
+    const double J0 = L;
+    const double I1 = L - r;
+    r *= s;
+    L *= s;
+    const double J1 = mu1 - L;
+    const double I2 = mu1 - 2. * L + r;
+    L *= s;
+    mu1 *= s;
+    const double J2 = mu2 + L - mu1;
+    t0 = a * (J0 - fspin * J1) + b * (I0 - fspin * I1);
+    t1 = a * (J1 - fspin * J2) + b * (I1 - fspin * I2);
 }
 
+// dcs.hh:624-677, an energy by W lanes (1: all poles in one thread, 4: a lane a
+// pole, added in the reference's order by shuffles).
+template <int W>
 __global__ void __launch_bounds__(C_THREADS) coulomb_transport_kernel(const double *__restrict__ screen,
                                                                 const double *__restrict__ fspin,
-                                                                const double *__restrict__ mu, int64_t n_mu,
+                                                                const double *__restrict__ mu_, int64_t n_mu,
                                                                 int64_t n, double *__restrict__ coefs) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double ps[NSF], c[2];
+    constexpr int PER = C_THREADS / W;
+    const int lane = threadIdx.x % W, first = threadIdx.x - lane, pole = lane < 3 ? lane : 2;
+    for (int64_t base = blockIdx.x * (int64_t)PER; base < n; base += (int64_t)gridDim.x * PER) {  // warp-uniform
+        const int64_t at = base + threadIdx.x / W, i = at < n ? at : n - 1;
+        const double *s = screen + NSF * i;
+        const double s0 = s[0], s1 = s[1], s2 = s[2], spin = fspin[i], mu = mu_[n_mu == 1 ? 0 : i];
+        const double nuclear_screening = (s1 < s2) ? s1 : s2;
+        const bool tiny = mu < 1E-08 * nuclear_screening;
+        double out0 = 0., out1 = 0.;
+        // with W > 1 decided for the warp: its lanes exchange terms
+        if (W == 1 ? !tiny : __any_sync(0xFFFFFFFFu, !tiny)) {
+            const double mu2 = 0.5 * mu * mu;
+            double t0[3], t1[3];
+            if constexpr (W == 1) {
 #pragma unroll
-        for (int j = 0; j < NSF; j++)
-            ps[j] = screen[NSF * i + j];
-        transport_coefficients(c, ps, fspin[i], mu[n_mu == 1 ? 0 : i]);
-        coefs[2 * i] = c[0];
-        coefs[2 * i + 1] = c[1];
+                for (int j = 0; j < 3; j++)
+                    transport_term(s[j], s[3 + j], s[6 + j], spin, mu, mu2, t0[j], t1[j]);
+            } else {
+                double a, b;
+                transport_term(s[pole], s[3 + pole], s[6 + pole], spin, mu, mu2, a, b);
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    t0[j] = __shfl_sync(0xFFFFFFFFu, a, first + j);
+                    t1[j] = __shfl_sync(0xFFFFFFFFu, b, first + j);
+                }
+            }
+            double c0 = 0., c1 = 0.;
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                c0 += t0[j];
+                c1 += t1[j];
+            }
+            const double kk = s0 * (1. + s0) * s1 * s1 * s2 * s2;
+            out0 = c0 * kk;
+            out1 = c1 * (2. * kk);
+        }
+        if (tiny) {
+            const double L = log(1. + qdiv(mu, s0));
+            const double r = qdiv(mu, mu + s0);
+            const double k = s0 * (1. + s0);
+            out0 = k * (qdiv(r, s0) - spin * (L - r));
+            const double I2 = mu - s0 * (r - 2. * L);
+            out1 = 2. * k * (L - r - spin * I2);
+        }
+        if (at < n && lane == 0) {
+            coefs[2 * i] = out0;
+            coefs[2 * i + 1] = out1;
+        }
     }
 }
 
@@ -480,12 +507,24 @@ cudaError_t noa_dcs_launch_coulomb_data(const double *K, int64_t n, const noa_co
     return cudaGetLastError();
 }
 
+// Energies per SM up to which a pole has a lane of its own: one warp of whole
+// energies an SM waits 9.8 us for 1660 dependent instructions, four lanes an
+// energy 4.5 us up to one warp (1000 energies 4.7 against 9.8, 5003 energies 6.1
+// against 9.8), while with more the FP64 pipe fills and the idle fourth lane
+// costs (12000 energies 9.6 / 9.9, 20000 15.8 / 12.8, 1e5 67 / 45).
+constexpr int64_t TRANSPORT_LANES = 64;
+
 cudaError_t noa_dcs_launch_coulomb_transport(const double *screen, const double *fspin, const double *mu,
                                              int64_t n_mu, int64_t n, double *coefs, cudaStream_t stream) {
     if (n <= 0)
         return cudaSuccess;
-    coulomb_transport_kernel<<<grid_for(n, C_THREADS, sm_count()), C_THREADS, 0, stream>>>(screen, fspin, mu, n_mu, n,
-                                                                                           coefs);
+    const int sms = sm_count();
+    if (n <= TRANSPORT_LANES * (int64_t)sms)
+        coulomb_transport_kernel<4><<<grid_for(n, C_THREADS / 4, sms), C_THREADS, 0, stream>>>(screen, fspin, mu, n_mu,
+                                                                                              n, coefs);
+    else
+        coulomb_transport_kernel<1><<<grid_for(n, C_THREADS, sms), C_THREADS, 0, stream>>>(screen, fspin, mu, n_mu, n,
+                                                                                          coefs);
     return cudaGetLastError();
 }
 
