@@ -43,6 +43,9 @@ constexpr int I_NARROW = 128, I_MID = 256, I_WIDE = 1024;
 // kernels are compiled for.
 constexpr int i_batch(int threads) { return threads == I_WIDE ? 320 : (threads == I_MID ? 192 : 128); }
 constexpr int i_ctas(int threads) { return threads == I_WIDE ? 1 : (threads == I_MID ? 2 : 5); }
+// A queue drained below `batch` after every step holds up to batch - 1 entries
+// when the next step's `threads` arrive.
+constexpr int queue_capacity(int batch, int threads) { return batch - 1 + threads; }
 
 __constant__ double kGL6X[6] = {0.03376524, 0.16939531, 0.38069041, 0.61930959, 0.83060469, 0.96623476};
 __constant__ double kGL6W[6] = {0.08566225, 0.18038079, 0.23395697, 0.23395697, 0.18038079, 0.08566225};
@@ -125,10 +128,12 @@ __device__ __forceinline__ double warp_node_sum(const double *v, int nodes) {
 template <int PROC, int THREADS>
 __global__ void __launch_bounds__(THREADS, i_ctas(THREADS))
     recoil_integral_kernel(const IntegralParams p, const noa_dcs_consts c) {
-    extern __shared__ double vals[];          // weighted node values of the tile, [k][node]
+    extern __shared__ double vals[];  // weighted node values of the tile, [k][node]
     constexpr int I_BATCH = i_batch(THREADS);
-    __shared__ double qQ[I_BATCH + THREADS];  // queued recoil energies
-    __shared__ int qS[I_BATCH + THREADS];     // their slots in vals
+    constexpr int batch = is_quad(PROC) ? I_BATCH : THREADS;
+    constexpr int QCAP = queue_capacity(batch, THREADS);
+    __shared__ double qQ[QCAP];  // queued recoil energies
+    __shared__ int qS[QCAP];     // their slots in vals
     __shared__ QuadSmem<PROC, I_BATCH> quad;
     __shared__ double sK[I_KMAX], sLb[I_KMAX], sH[I_KMAX];
     __shared__ int warp_tot[THREADS / 32];
@@ -136,8 +141,6 @@ __global__ void __launch_bounds__(THREADS, i_ctas(THREADS))
     const int pairs = p.kpt * p.nodes;
     const int64_t tiles = (p.n + p.kpt - 1) / p.kpt;
     const double ion_thr = c.io_k_rad;  // 0.5 (m - me)^2 / me, dcs.hh:962-963
-    constexpr int batch = is_quad(PROC) ? I_BATCH : THREADS;
-    static_assert(batch <= I_BATCH + THREADS, "queue capacity");
 
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t k0 = tile * p.kpt;
@@ -299,7 +302,7 @@ __global__ void __launch_bounds__(THREADS, i_ctas(THREADS))
     soft_scattering_kernel(const SoftParams p, const noa_dcs_consts c) {
     constexpr int I_BATCH = i_batch(THREADS);
     __shared__ double vals[S_KMAX * S_NODES];
-    __shared__ int qS[I_BATCH + THREADS];
+    __shared__ int qS[queue_capacity(I_BATCH, THREADS)];
     __shared__ QuadSmem<NOA_DCS_PROC_PHOTO, I_BATCH> quad;
     __shared__ double sK[S_KMAX];
     __shared__ int warp_tot[THREADS / 32];
