@@ -20,9 +20,9 @@
  * These are scalar, branchy, per-K computations (a few logs, a series of
  * 10 + Z terms, up to 100 root iterations), bound by the FP64 pipe when there
  * are enough energies and by latency when there are not: CTAs of one warp
- * spread the energies over the SMs, divisions are the correctly rounded
- * quotient in 3 FP64 instructions, and the hard-scattering search gives an
- * energy up to 32 lanes (hard_scattering_kernel).  Records are the
+ * spread the energies over the SMs, divisions take 3 FP64 instructions
+ * (lean64::qdiv), and the hard-scattering search gives an energy up to 32 lanes
+ * (hard_scattering_kernel).  Records are the
  * reference's: fCM [n][2], screen [n][9].
  */
 #include "dcs_launch.h"
@@ -39,21 +39,8 @@ constexpr double KIN_CUTOFF = 1E-9;              // physics.hh:78
 constexpr double EHS_PATH_MAX = 1E+9;            // physics.hh:79
 constexpr double EHS_OVER_MSC = 1E-4;            // physics.hh:80
 
-// a / b, correctly rounded: Markstein's correction of a * rcp(b) by its exact
-// residual (P. Markstein, IBM J. Res. Dev. 34(1), 1990), 3 FP64 instructions
-// instead of 8.5.  For |a| and |b| in [2^-400, 2^400); everything else takes
-// the hardware's division sequence.
-__device__ __forceinline__ bool qdiv_range(double a) {
-    return ((unsigned)__double2hiint(a) & 0x7FFFFFFFu) - 0x26F00000u < 0x32000000u;
-}
-__device__ __forceinline__ double qdiv_fast(double a, double b) {
-    const double y = lean64::lean_rcp(b);
-    const double q = a * y;
-    return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-__device__ __forceinline__ double qdiv(double a, double b) {
-    return qdiv_range(a) && qdiv_range(b) ? qdiv_fast(a, b) : a / b;
-}
+using lean64::qdiv;
+using lean64::qdiv_fast;
 
 // std::min's rule (b < a ? b : a), which differs from fmin for NaN.
 __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }

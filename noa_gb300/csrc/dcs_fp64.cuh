@@ -42,7 +42,6 @@
 namespace noa_dcs {
 
 using lean64::bits_ge;
-using lean64::lean_div;
 using lean64::lean_exp;
 using lean64::lean_log;
 using lean64::lean_rcp;
@@ -91,7 +90,7 @@ __device__ __forceinline__ double clamp0(double v) {
 static __device__ __noinline__ double ol_log(double x) { return lean_log(x); }
 static __device__ __noinline__ double ol_exp(double x) { return lean_exp(x); }
 static __device__ __noinline__ double ol_rcp(double x) { return lean_rcp(x); }
-static __device__ __noinline__ double ol_div(double a, double b) { return lean_div(a, b); }
+static __device__ __noinline__ double ol_qdiv(double a, double b) { return lean64::qdiv(a, b); }
 static __device__ __noinline__ long long ol_log_fx(double x) { return lean64::lean_log_fx(x); }
 static __device__ __noinline__ long long ol_log3p_fx(double x) { return lean64::lean_log3p_fx(x); }
 static __device__ __noinline__ long long ol_log_of_fx(long long v) { return lean64::log_of_fx(v); }

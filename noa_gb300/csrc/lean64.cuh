@@ -496,6 +496,21 @@ LEAN64_FN double round_by_one(double x) {
 
 LEAN64_FN double lean_div(double a, double b) { return a * lean_rcp(b); }
 
+// a / b rounded to nearest, unless it lies within about 2^-52 ulp of a tie:
+// Markstein's correction of a rcp(b) by its exact residual (P. Markstein, IBM J.
+// Res. Dev. 34(1), 1990; his theorem asks for a correctly rounded reciprocal,
+// lean_rcp's is 0.504 ulp), 3 FP64 instructions instead of 8.5.  For |a| and |b| in
+// [2^-400, 2^400); everything else takes the hardware's division sequence.
+LEAN64_FN bool qdiv_range(double a) {
+    return ((unsigned)((unsigned long long)detail::d2ll(a) >> 32) & 0x7FFFFFFFu) - 0x26F00000u < 0x32000000u;
+}
+LEAN64_FN double qdiv_fast(double a, double b) {
+    const double y = lean_rcp(b);
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+LEAN64_FN double qdiv(double a, double b) { return qdiv_range(a) && qdiv_range(b) ? qdiv_fast(a, b) : a / b; }
+
 __device__ __forceinline__ double lean_sqrt(double x) {
     const float xf = fpconv::f32(x);
     if (!(xf >= 2e-38f && xf <= 1e38f))
