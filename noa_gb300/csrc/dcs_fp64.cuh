@@ -320,7 +320,7 @@ __device__ __forceinline__ void pprod_setup(double K, double q, const noa_dcs_co
 
 // Clamp of the reference's `if (Phi < 0.) Phi = 0.;` for -Phi; keeps NaN.
 __device__ __forceinline__ double clamp0_neg(double v) {
-    return (unsigned long long)(__double_as_longlong(v) - 1) < 0x7FF0000000000000ULL ? 0. : v;
+    return (unsigned long long)__double_as_longlong(v) - 1ull < 0x7FF0000000000000ULL ? 0. : v;
 }
 
 // Node j: -(1 - rho) (Phi_e + Phi_mu / r^2), 19 FP64 instructions (about 75
@@ -536,8 +536,8 @@ __device__ __forceinline__ void photo_setup(double K, double q, const noa_dcs_co
     p.pc = fits ? lean64::to_fx(pc, 57) : __double_as_longlong(pc);
     p.k2 = fits ? lean64::to_fx(k2, 57) : __double_as_longlong(k2);
     p.hdf = lean64::to_fx(p.hd, 58);
-    p.lP = -ol_log_fx(fma(2.0 * PH_M, q, 49.457));
-    p.lR = -ol_log_fx(fma(2.0 * PH_M, q, 0.15052));
+    p.lP = (long long)(0ull - (unsigned long long)ol_log_fx(fma(2.0 * PH_M, q, 49.457)));
+    p.lR = (long long)(0ull - (unsigned long long)ol_log_fx(fma(2.0 * PH_M, q, 0.15052)));
 }
 
 // Node j: (F2A / (A / 2)) Q2 dds of dcs.hh:289-354, 26 FP64 instructions
@@ -589,7 +589,7 @@ __device__ __forceinline__ double photo_node(const PhotoPair &p, int j, const no
     F2 = fma(lean64::from_fx(cR), ol_exp_fx(fx_mul(aR, ol_log_fx(Q2 + mR2) + p.lR) + fx_mul(bR, l1x) + f), F2);
     // 2 - 1.85 x + 2.45 x^2 - 2.35 x^3 + x^4, in units of 2^-61
     const long long xf = (long long)lean64::unit_to_fx62(x);
-    const auto times_x = [xf](long long a) { return lean64::detail::mulhi_s64(xf, a) << 2; };
+    const auto times_x = [xf](long long a) { return lean64::detail::mulhi_s64(xf, a) * 4; };
     const long long poly =
         fx_const(2., 61) + times_x(fx_const(-1.85, 61) +
                                    times_x(fx_const(2.45, 61) + times_x((xf >> 1) - fx_const(2.35, 61))));

@@ -222,6 +222,14 @@ LEAN64_FN long long log_bin(long long R, long long L) {
     return R + (long long)((unsigned long long)L + (unsigned long long)b1 * 0x400000ull + b2);
 }
 
+// exp: k ln2 / 128 in units of 2^-63, modulo 2^64 (unsigned, as its first part and
+// the sum wrap).
+LEAN64_FN unsigned long long k_ln2n(int k) {
+    return (unsigned long long)((long long)k * LEAN64_K_M) +
+           ((unsigned long long)((unsigned)k * (unsigned)LEAN64_K_H) << 32) +
+           (unsigned long long)(long long)(int)mulhi_s(k, LEAN64_K_L);
+}
+
 // exp: T_j (1 + expm1 r) in units of 2^-61, in [2^61, 2^62), for k = 128 k' + j
 // and r = R 2^-63, |r| < 2^-8.4; q = k' or, where T_0 (1 + expm1 r) < 1, k' - 1.
 LEAN64_FN unsigned long long exp_bin(int k, long long r, int &q) {
@@ -321,12 +329,9 @@ LEAN64_FN double lean_exp(double x) {
     const unsigned long long M = (((unsigned long long)b) & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
     const int n = (int)(a >> 20) - 1012;  // -1012 .. 20
     const unsigned long long X = n >= 0 ? M << n : M >> (n < -63 ? 63 : -n);
-    const long long sx = (long long)(int)hi >> 63;
-    const long long r = (((long long)X ^ sx) - sx) -
-                        ((long long)k * LEAN64_K_M + (long long)((unsigned long long)(long long)(k * LEAN64_K_H) << 32) +
-                         (int)mulhi_s(k, LEAN64_K_L));
+    const unsigned long long sx = (unsigned long long)((long long)(int)hi >> 63);
     int q;
-    const unsigned long long m = (exp_bin(k, r, q) + 0x100ull) >> 9;  // leading bit at 52
+    const unsigned long long m = (exp_bin(k, (long long)((X ^ sx) - sx - k_ln2n(k)), q) + 0x100ull) >> 9;  // leading bit at 52
     return ll2d((long long)(((unsigned long long)(q + 1022) << 52) + m));
 }
 
@@ -372,7 +377,8 @@ LEAN64_FN long long fx_mul(long long a, long long b, int F = 57) {
     return (long long)(((unsigned long long)detail::mulhi_s64(a, b) << (64 - F)) | (lo >> F));
 }
 
-// log x, x positive, normal and finite; to about 2^-57 absolute.
+// log x, x positive, normal and finite and |log x| < 64 (else a number modulo
+// 128, which no caller uses); |e| / 2 + 2 units for x = 2^e m.
 LEAN64_FN long long lean_log_fx(double x) {
     using namespace detail;
     const long long b = d2ll(x);
@@ -380,7 +386,8 @@ LEAN64_FN long long lean_log_fx(double x) {
     const int e = (int)(hi + ((512u - LEAN64_LOG_SPLIT) << 11) - 0x3FF00000u) >> 20;
     const longlong2 ent = log_entry((hi >> 11) & 0x1FFu);
     const unsigned long long M = ((unsigned long long)((hi & 0x000FFFFFu) | 0x00100000u) << 32) | (unsigned)b;
-    return (log_bin((long long)(M * (unsigned)ent.x), ent.y) >> 7) + (long long)e * LEAN64_LN2_57;
+    return (long long)((unsigned long long)(log_bin((long long)(M * (unsigned)ent.x), ent.y) >> 7) +
+                       (unsigned long long)(long long)e * LEAN64_LN2_57);
 }
 
 // log(N 2^E), N with its leading bit at 63 (taken as its top 53 bits and the
@@ -417,10 +424,7 @@ LEAN64_FN long long log_of_fx(long long v) {
 LEAN64_FN unsigned long long exp_fx_bin(long long x, int &q) {
     using namespace detail;
     const int k = (int)(((long long)(int)(x >> 32) * LEAN64_INV_LN2N_22 + (1ll << 46)) >> 47);
-    const long long r = (long long)((unsigned long long)x << 6) -
-                        ((long long)k * LEAN64_K_M + (long long)((unsigned long long)(long long)(k * LEAN64_K_H) << 32) +
-                         (int)mulhi_s(k, LEAN64_K_L));
-    return exp_bin(k, r, q);
+    return exp_bin(k, (long long)(((unsigned long long)x << 6) - k_ln2n(k)), q);
 }
 LEAN64_FN double lean_exp_fx(long long x) {
     int q;
