@@ -72,8 +72,9 @@ int occupancy(const noa_dcs_batch_plan *p, int threads, int items) {
                                         : noa_dcs_batched_occupancy32(p->process, threads, smem);
 }
 
-// Fills the tile prefix sums for the current tile shape; the first
-// sample_per_segment pairs of each segment only, if > 0.  The tile spreads
+// Fills the tile prefix sums for the current tile shape; of the first
+// sample_per_segment pairs of each segment only, if > 0, in the tiles of the whole
+// call (so that the autotuner times the tile that will run).  The tile spreads
 // the pairs over all CTAs in equal steps, with room for a partial tile per
 // segment (a few tiles more than CTAs cost a whole further step), at most the
 // shape's items x threads pairs, down to a warp: a short call left most CTAs
@@ -84,13 +85,7 @@ int occupancy(const noa_dcs_batch_plan *p, int threads, int items) {
 // (photonuclear 72 us against 64).
 void set_tiles(noa_dcs_batch_plan *p, int64_t sample_per_segment = 0) {
     const int64_t *begin = p->params.seg_begin;
-    int64_t count[NOA_DCS_MAX_SEGMENTS], total = 0;
-    for (int s = 0; s < p->params.n_seg; s++) {
-        count[s] = begin[s + 1] - begin[s];
-        if (sample_per_segment > 0 && count[s] > sample_per_segment)
-            count[s] = sample_per_segment;
-        total += count[s];
-    }
+    const int64_t total = begin[p->params.n_seg];
     const int64_t most = (int64_t)p->items * p->threads;
     const int64_t ctas = (int64_t)p->sms * p->ctas_per_sm;
     const int64_t steps = (total + p->params.n_seg * most + ctas * most - 1) / (ctas * most);
@@ -101,8 +96,12 @@ void set_tiles(noa_dcs_batch_plan *p, int64_t sample_per_segment = 0) {
     p->params.items = p->items;
     p->params.tile = (int)tile;
     p->params.tile_begin[0] = 0;
-    for (int s = 0; s < p->params.n_seg; s++)
-        p->params.tile_begin[s + 1] = p->params.tile_begin[s] + (count[s] + tile - 1) / tile;
+    for (int s = 0; s < p->params.n_seg; s++) {
+        int64_t count = begin[s + 1] - begin[s];
+        if (sample_per_segment > 0 && count > sample_per_segment)
+            count = sample_per_segment;
+        p->params.tile_begin[s + 1] = p->params.tile_begin[s] + (count + tile - 1) / tile;
+    }
 }
 
 int launch(noa_dcs_batch_plan *p, double *out, const double *K, const double *q, cudaStream_t s) {
