@@ -202,11 +202,12 @@ const char *noa_dcs_batch_last_error(void);
  * before the launch.  All calls share that array: calls whose work overlaps
  * on the GPU (different streams, or different host threads) race and must be
  * serialised by the caller.  Set-up on the first call on each device: the
- * array's device address is looked up with that device current, and for
- * FP32C pair production (83 KB of shared memory) the kernel's shared-memory
- * limit is raised; later calls make no runtime set-up call.  Tile
- * shape is fixed (256 threads x 4 pairs, 2 CTAs per SM).  Buffers as for the
- * plan. */
+ * array's device address is looked up with that device current, and, on the
+ * first call of each of the three kernels that take more than 48 KB of shared
+ * memory (FP64 pair production 76 KB, FP64 photonuclear 70 KB, FP32C pair
+ * production 83 KB), that kernel's limit is raised; later calls make no runtime
+ * set-up call.  Tile shape is fixed (256 threads x 4 pairs, 2 CTAs per SM).
+ * Buffers as for the plan. */
 int noa_dcs_cuda_vmap_batched_noalloc(int process, int precision, int n_segments, const noa_dcs_element *elements,
                                       const int64_t *counts, double mass, double *result, const double *K,
                                       const double *q, void *stream);

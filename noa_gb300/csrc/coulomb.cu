@@ -1,5 +1,5 @@
 /*
- * Elastic (Coulomb) scattering per kinetic energy, FP64, one thread per K:
+ * Elastic (Coulomb) scattering per kinetic energy, FP64:
  *
  *   coulomb_data       dcs.hh:499-622  CM Lorentz factors, spin factor,
  *                                      screening parameters + pole factors,
@@ -21,8 +21,8 @@
  * 10 + Z terms, up to 100 root iterations), bound by the FP64 pipe when there
  * are enough energies and by latency when there are not: CTAs of one warp
  * spread the energies over the SMs, divisions take 3 FP64 instructions
- * (lean64::qdiv), and the hard-scattering search gives an energy up to 32 lanes
- * (hard_scattering_kernel).  Records are the
+ * (lean64::qdiv), the transport coefficients give a pole a lane where energies are
+ * few, and the hard-scattering search an energy up to 32 (hard_scattering_kernel).  Records are the
  * reference's: fCM [n][2], screen [n][9].
  */
 #include "dcs_launch.h"

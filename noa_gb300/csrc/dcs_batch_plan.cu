@@ -462,9 +462,11 @@ extern "C" int noa_dcs_cuda_vmap_batched_noalloc(int process, int precision, int
         noa_dcs_fill_consts(&p.params.consts[s], elements[s].A, elements[s].I, elements[s].Z, mass);
     }
     // Fixed tile shape (the plan default): 256 threads x 4 pairs, 2 CTAs per
-    // SM.  Its queues take 43 KB of shared memory, 83 KB for FP32C pair
-    // production (a third queue and its float-float step's nodes); above 48 KB the launch raises the kernel's
-    // limit once per device, on its first call there.
+    // SM.  The work queue takes 30 KB of shared memory, FP32C's redo queue 12 KB
+    // more; with the nodes of a batch FP64 pair production takes 76 KB, FP64
+    // photonuclear 70 KB and FP32C pair production (a third queue, its float-float
+    // step's nodes) 83 KB.  Above 48 KB the launch raises the kernel's limit once
+    // per device, on its first call there.
     p.threads = 256;
     p.items = 4;
     p.ctas_per_sm = 2;

@@ -82,20 +82,6 @@ NOA_HD double d_log(double x) {
     return log(x);
 #endif
 }
-NOA_HD double d_exp(double x) {
-#if defined(__CUDA_ARCH__)
-    return lean64::lean_exp(x);
-#else
-    return exp(x);
-#endif
-}
-NOA_HD double d_sqrt(double x) {
-#if defined(__CUDA_ARCH__)
-    return lean64::lean_sqrt(x);
-#else
-    return sqrt(x);
-#endif
-}
 NOA_HD double d_rcp(double x) {
 #if defined(__CUDA_ARCH__)
     return lean64::lean_rcp(x);

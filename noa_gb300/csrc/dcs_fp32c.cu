@@ -4,8 +4,8 @@
  * Pair production and photonuclear use the compacting kernel of the FP64 path
  * (dcs_fp64.cu) with a second queue:
  *
- *   1. a CTA classifies a 1024-pair tile with the exact kinematic bounds,
- *      writes the zeros, and appends the open pairs to the shared-memory work
+ *   1. a CTA classifies a tile of 32 to 1024 pairs with the exact kinematic
+ *      bounds, writes the zeros, and appends the open pairs to the shared-memory work
  *      queue;
  *   2. whenever the work queue holds 256 pairs, each thread pops one and
  *      evaluates it in FP32 (dcs_fp32c.cuh), which also returns an estimate

@@ -28,7 +28,7 @@
  * of what cancels), or infinity where a branch or clamp of the reference sits
  * within rounding distance.  When est exceeds the caller's tolerance the
  * kernel evaluates that pair in FP64 instead (pair production: first again
- * in FP32 with its screening log in FF, pprod_fp32c<false, true>).
+ * in FP32 with its screening log in FF, Pprod32<true>).
  *
  * Written for host and device (NOA_HD) so that the same source can be
  * checked against the CPU oracle.
@@ -127,17 +127,8 @@ struct KSum {
     NOA_HD double value() const { return fpconv::f64(s) + fpconv::f64(c); }
 };
 
-// exp(uh + ul) and -expm1(uh + ul) for a double argument split into floats.
-NOA_HD void f_exp_split(double u, float &e, float &em1) {
-    const float uh = fpconv::f32(u);
-    const float ul = fpconv::f32(u - fpconv::f64(uh));
-    const float eh = expf(uh);
-    e = fmaf(eh, ul, eh);
-    em1 = fmaf(eh, ul, expm1f(uh));
-}
-
-// The same for u = x t with x = xh + xl and t = th + tl float-float pairs,
-// entirely in FP32: x t is formed as a float-float product (the FMA gives
+// exp(u) and expm1(u) for u = x t with x = xh + xl and t = th + tl float-float
+// pairs, entirely in FP32: x t is formed as a float-float product (the FMA gives
 // xh th exactly), so exp sees u to ~2^-48 without an FP64 instruction.
 NOA_HD void f_exp_split_ff(float xh, float xl, float th, float tl, float &e, float &em1) {
     const float ph = xh * th;

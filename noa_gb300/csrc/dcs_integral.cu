@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(THREADS, i_ctas(THREADS))
  * mu-integrated angular weight of dcs.hh:911-934.  Same tile / queue scheme
  * as the recoil integrals: closed photonuclear nodes contribute
  * 0 * ratio * nu (0, or NaN where the weight is not finite, as in the
- * reference), open ones are evaluated 256 at a time.
+ * reference), open ones are evaluated in batches of 128 or 192.
  */
 constexpr int S_NODES = 102;             // 6 * ceil(100 / 6)
 constexpr int S_KMAX = 8;                // kinetic energies per tile at most
@@ -409,7 +409,7 @@ int energies_per_tile(int64_t n, int64_t sms, int most) {
 // 54.9 / 70.0 us at 128 threads, 34.0 / 46.4 at 256, 27.3 / 39.3 at 512, 26.8 /
 // 36.4 at 1024), while bremsstrahlung, ionisation and soft scattering, which
 // wait for one or two rounds of usual node counts, are as fast at 256 as above
-// (9.8, 10.1 and 26.0 us).  Up to two an SM both are resident at 256 (304
+// (9.8, 10.1 and 26.3 us).  Up to two an SM both are resident at 256 (304
 // energies: 43.3 / 63.0 us against 60.5 / 80.9 at 128 and 51.3 / 69.6 at 1024);
 // a quadrature's batch of 192 leaves room for 4 KB of node values there.
 // Above, 128 threads leave room for five (456 energies: 14.5 us of

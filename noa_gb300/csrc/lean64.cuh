@@ -18,7 +18,7 @@
  * instead of shifts) or as the two 32-bit words of a fixed-point number,
  * never by normalising.  Four processes x 3e7 pairs: 42.2 ms with the same
  * methods at 1 / 2 / 0 FP64 instructions and normalised conversions (about
- * twice the ALU instructions), 35.3 ms as they are:
+ * twice the ALU instructions), 35.3 ms with these in the same bodies:
  *
  *   lean_log   0 FP64 ops.  Tang's table method (P. T. P. Tang, ACM TOMS
  *              16(4), 1990): x = 2^e m, c_t ~ 1/m with 11 fractional bits from

@@ -51,23 +51,15 @@ struct Norm {
     float out_scale;  // r = out_shift + y / out_scale
 };
 
-// SiLU and its derivative.  On the GPU through the MUFU exponential and an
-// approximate division (relative error ~2^-21), in training and inference
-// alike; z / (1 + inf) gives the correct limit 0.
+// SiLU.  On the GPU through the MUFU exponential and an approximate division
+// (relative error ~2^-21), in training and inference alike; z / (1 + inf) gives
+// the correct limit 0.
 __host__ __device__ __forceinline__ float silu(float z) {
 #if defined(__CUDA_ARCH__)
     return __fdividef(z, 1.f + __expf(-z));
 #else
     return z / (1.f + expf(-z));
 #endif
-}
-__host__ __device__ __forceinline__ float dsilu(float z) {
-#if defined(__CUDA_ARCH__)
-    const float s = __fdividef(1.f, 1.f + __expf(-z));
-#else
-    const float s = 1.f / (1.f + expf(-z));
-#endif
-    return s * (1.f + z * (1.f - s));
 }
 
 // Baseline of log DCS and the open / closed decision, in FP64 with the exact
